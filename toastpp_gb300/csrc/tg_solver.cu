@@ -323,7 +323,12 @@ struct Engine {
     V* vec(int i, size_t nk) { return (V*)w[i].ensure(nk * sizeof(V)); }
     int ntiles() const { return (int)cdiv_u(mesh->d.n, ROW_TILE); }
     double* parts(int k, int np) { return (double*)part.ensure((size_t)k * np * ntiles() * sizeof(double)); }
-    unsigned rowblk(int k) const { return (unsigned)std::min(256, std::max(32, (k + 31) / 32 * 32)); }
+    // threads of a tile kernel's block: one per (column, row group) item of the
+    // tile, so that the tile's rows are read in one round.  With one thread per
+    // column a 32-column block walked its 8 row groups one after the other
+    // (12.5k nodes, 32 complex FP32 columns: update pass 42 us, 32-column
+    // requests 1.07x to 1.30x as fast with this split; sums unchanged).
+    unsigned rowblk(int k) const { return (unsigned)std::min(256, std::max(32, (k * TILE_RG + 31) / 32 * 32)); }
 
     // SpMM variants: 0 halo-staged, 1 vector words, 2 warp per row, 3 narrow
     bool spmm_ok(int var, int k) const
