@@ -153,7 +153,8 @@ int tg_solver_set(tg_solver s, double tol, int maxit);
    (default 12) and the
    elimination ordering of the inner IC(0) preconditioner: 1 (default) a
    colour-major ordering of a greedy colouring, whose colour classes are the
-   levels of the triangular sweeps, or 0 the natural ordering of the reference.
+   levels of the triangular sweeps, or 0 the natural ordering of the reference
+   (which also keeps the sweeps where the default would run on chip).
    The FP64 path always factors in the natural ordering.  Takes effect at the
    next tg_solver_reset. */
 int tg_solver_set_refinement(tg_solver s, double inner_tol, int max_outer, int inner_ordering);
@@ -163,8 +164,12 @@ int tg_solver_set_refinement(tg_solver s, double inner_tol, int max_outer, int i
       by the FP64 residual b - A x whenever it has fallen by inner_tol
       (reliable updates);
    2 (default): as 1 with an FP32 COCG process for complex systems (the
-      conjugate-orthogonal CG of the complex symmetric F: one SpMM and one
-      IC(0) apply per iteration); real systems use 1.
+      conjugate-orthogonal CG of the complex symmetric F).  While the vectors
+      fit on the chip, an ICH-preconditioned solve in the default ordering runs
+      as one kernel on thread-block clusters, with CG for real systems and a
+      factorised sparse approximate inverse on F's own pattern in place of the
+      IC(0) sweeps; CG requests run the same way.  Larger blocks take one SpMM
+      and one IC(0) apply per COCG iteration, real systems as 1.
    The FP64 result meets tol in every mode.  At most 4 * max_outer residual
    replacements per right-hand side. */
 /* mixed precision only: the componentwise backward-error bound of every

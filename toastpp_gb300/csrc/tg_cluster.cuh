@@ -1,0 +1,58 @@
+// tg_cluster.cuh -- the interface of the resident solve (tg_resident.cu): one
+// kernel in which thread-block clusters run a conjugate-gradient process on
+// their own right-hand sides, and the kernel that forms its preconditioner.
+#pragma once
+#include "tg_kernels.cuh"
+
+namespace tg {
+
+constexpr int CL_NT = 800;      // threads per CTA at most (80 registers each)
+constexpr int CL_MAXCG = 4;     // columns per cluster at most
+constexpr int CL_MAXCS = 16;    // CTAs per cluster at most
+constexpr int CL_NV = 3;        // quantities per column in one reduction at most
+constexpr int FSAI_MAXM = 32;   // entries of a row of G at most
+
+// a matrix in slices of 32 rows, entry by entry: entry e of row r at
+// ptr[r / 32] + 32 e + r % 32, its column as the slot of the CTA's gather
+// buffers; padding: the row's own slot and the value 0
+template <class V>
+struct Sell {
+    const int* ptr;
+    const unsigned short* col;
+    const V* val;
+};
+
+template <class V64, class V32>
+struct ResArgs {
+    int n, k, cs;
+    int slots, own;             // rows of a gather buffer (own rows and halo) and own rows, the largest of the CTAs
+    int msm, mofs_val, mofs_col, mofs_ptr, mofs_push;  // msm: the matrices go to shared memory, at these byte offsets
+    Sell<V32> A, G, T;          // system matrix, approximate inverse and its transpose
+    const int* pofs;            // per CTA: its halo copies in push,
+    const uint2* push;          //   {own slot, rank << 16 | slot there}
+    V32* x;                     // FP32 correction, [cluster][node][CG]
+    V64 *X, *R;                 // solution and true residual, node-major, k columns
+    const V64* B;
+    void* Xff;                  // solution of the columns being updated, as float-float, node-major
+    const int *rowptr, *colidx; // layout CSR of the system matrix, for the residuals:
+    const V64* A64;             //   FP64 values,
+    const void* Aff;            //   float-float values,
+    const float* absA;          //   magnitudes
+    ColState* co;               // per column: tol on entry, results on exit
+    float trig;                 // residual drop that triggers a correction
+    double cwtol;               // componentwise bound (0: none)
+    int maxit, max_upd, zero_guess;
+    int all64;                  // every residual product in FP64
+};
+
+// the kernel for lv columns a cluster (1, 2; real systems also 4)
+template <class V64, class V32>
+void (*resident_kernel(int lv))(ResArgs<V64, V32>);
+
+// G of the approximate inverse from A's values in CSR order, a warp per row
+constexpr int FSAI_WARPS = 4;
+template <class V>
+void (*fsai_kernel_of())(int n, const int* rowptr, const int* colidx, const int* diagpos, const V* A, const int* gptr,
+                         const int* gcol, const int* gcnt, V* gval);
+
+}  // namespace tg

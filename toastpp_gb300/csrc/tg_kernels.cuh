@@ -1010,6 +1010,8 @@ __global__ void reduce_finalize_kernel(int k, int ntiles, const double* __restri
         S.its++;
         if (S.err <= S.tol * S.bnorm) { S.active = 0; S.status = 0; break; }
         if (S.its >= S.maxit) { S.active = 0; S.status = 1; }
+        // a process that grows has lost its directions: it restarts
+        else if (!(S.err <= 100.0 * S.bnorm)) { S.active = 0; S.status = 2; }
         break;
     case PH_COCG_BETA: {
         if (S.active != 1) break;
@@ -1392,8 +1394,8 @@ static __global__ void count_active_kernel(int k, const ColState* __restrict__ c
 // added to the FP64 solution, the true residual b - A x is formed in FP64 and
 // replaces the FP32 residual, and the same Krylov process continues.
 // ---------------------------------------------------------------------------
-// out[0] outer columns active, out[1] inner columns iterating, out[2] waiting
-// for an update (outer active, inner stopped)
+// out[0] outer columns active, out[1] waiting columns with five updates or
+// more behind them, out[2] waiting for an update (outer active, inner stopped)
 static __global__ void rel_flags_kernel(int k, const ColState* __restrict__ co, const ColState* __restrict__ ci,
                                         int* out)
 {
@@ -1404,7 +1406,7 @@ static __global__ void rel_flags_kernel(int k, const ColState* __restrict__ co, 
     for (int c = threadIdx.x; c < k; c += blockDim.x) {
         const bool oa = co[c].active == 1, ia = ci[c].active == 1;
         a += oa;
-        b += ia;
+        b += oa && !ia && ci[c].nupd >= 5;
         f += oa && !ia;
     }
     atomicAdd(&s[0], a);
@@ -1538,7 +1540,8 @@ __global__ void rel_accumulate_kernel(int n, int k, const ColState* __restrict__
     if (t >= (size_t)n * k) return;
     int c = (int)(t % k);
     if (!ci[c].rel) return;
-    x[t] = vadd(x[t], vscale(vcast<V64, V32>(x32[t]), ci[c].scale));
+    // (the correction of a process that grew is dropped)
+    if (ci[c].err <= ci[c].bnorm) x[t] = vadd(x[t], vscale(vcast<V64, V32>(x32[t]), ci[c].scale));
     x32[t] = vzero<V32>();
 }
 
@@ -1556,11 +1559,12 @@ static __global__ void rel_outer_kernel(int k, ColState* __restrict__ co, ColSta
     if (O.active != 1 || !I.rel) return;
     if (col_converged(O, c, cwtol, cmax)) { O.active = 0; O.status = 0; I.rel = 0; return; }
     if (limit || ++I.nupd >= max_upd) { O.active = 0; O.status = 1; I.rel = 0; return; }
-    // a true residual far above the recursive one means the process no longer
+    // a true residual above the recursive one means the process no longer
     // follows the FP64 system (at the rounding floor of the FP64 residual the
     // true residual stops falling while the recursion goes on): resuming it
     // with the old directions stagnates, so it restarts from the true residual
-    if (O.err > 8.0 * I.err * I.scale) I.rel = 2;
+    // (off that floor the two agree to 1e-3)
+    if (O.err > 1.25 * I.err * I.scale) I.rel = 2;
     // rescale the process to the new residual (exact: powers of two)
     I.scale_prev = I.scale;
     I.scale = pow2_floor(O.err);

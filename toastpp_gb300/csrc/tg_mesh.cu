@@ -217,6 +217,53 @@ static void halo_lists(MeshHost& m)
     }
 }
 
+// rows of (column, source index) as slices
+static void sell_slices(const std::vector<std::vector<std::pair<int, int>>>& rows, SellHost& s)
+{
+    const int n = (int)rows.size(), ns = (n + 31) / 32;
+    s.ptr.assign(ns + 1, 0);
+    for (int t = 0; t < ns; t++) {
+        size_t w = 0;
+        for (int r = t * 32; r < std::min(n, t * 32 + 32); r++) w = std::max(w, rows[r].size());
+        s.ptr[t + 1] = s.ptr[t] + 32 * (int)w;
+    }
+    s.col.assign(s.ptr[ns], 0);
+    s.src.assign(s.ptr[ns], -1);
+    for (int t = 0; t < ns; t++)
+        for (int r = t * 32; r < t * 32 + 32; r++) {
+            const int w = (s.ptr[t + 1] - s.ptr[t]) / 32, own = std::min(r, n - 1);
+            for (int e = 0; e < w; e++) {
+                const int o = s.ptr[t] + 32 * e + (r & 31);
+                const bool in = r < n && e < (int)rows[r].size();
+                s.col[o] = in ? rows[r][e].first : own;
+                s.src[o] = in ? rows[r][e].second : -1;
+            }
+        }
+}
+
+static void sell_patterns(MeshHost& m)
+{
+    const int n = m.n;
+    std::vector<std::vector<std::pair<int, int>>> rows(n), trows(n);
+    for (int r = 0; r < n; r++)
+        for (int e = m.lrowptr[r]; e < m.lrowptr[r + 1]; e++) rows[r].push_back({m.lcolidx[e], e});
+    sell_slices(rows, m.sa);
+    m.gcnt.assign(n, 0);
+    for (int r = 0; r < n; r++) {
+        rows[r].clear();
+        for (int e = m.lrowptr[r]; e < m.lrowptr[r + 1]; e++)
+            if (m.lcolidx[e] <= r) rows[r].push_back({m.lcolidx[e], -1});
+        std::sort(rows[r].begin(), rows[r].end());
+        m.gcnt[r] = (int)rows[r].size();
+        m.gmax = std::max(m.gmax, m.gcnt[r]);
+    }
+    sell_slices(rows, m.sg);
+    for (int r = 0; r < n; r++)
+        for (int e = 0; e < m.gcnt[r]; e++)
+            trows[rows[r][e].first].push_back({r, m.sg.ptr[r / 32] + 32 * e + (r & 31)});
+    sell_slices(trows, m.st);
+}
+
 static void layout_order(MeshHost& m)
 {
     int n = m.n, dim = m.dim;
@@ -587,14 +634,86 @@ Mesh::~Mesh()
 {
     void* ptrs[] = {d.rec, d.el, d.rowptr, d.colidx, d.diagpos, d.perm, d.iperm, d.jrowptr, d.jcolidx, d.asm_ptr,
                     d.asm_list, d.nel_ptr, d.nel_list, d.nel_pos, d.bndnode, d.halo_ptr, d.halo_col, d.lcol,
-                    d.intbff};
+                    d.intbff, d.sa.ptr, d.sa.col, d.sa.src, d.sg.ptr, d.sg.col, d.sg.src, d.st.ptr, d.st.col,
+                    d.st.src, d.gcnt};
     for (void* p : ptrs) if (p) cudaFree(p);
+    for (auto& p : parts)
+        if (p.second) {
+            void* q[] = {p.second->ca, p.second->cg, p.second->ct, p.second->pofs, p.second->push};
+            for (void* x : q) if (x) cudaFree(x);
+        }
     for (auto& g : d.ic) {
         void* q[] = {g.key, g.Lrowptr, g.Lcolidx, g.Lapos, g.Lkey, g.Ucolptr, g.Urow, g.Umap, g.fwd_lev_rows,
                      g.bwd_lev_rows, g.fwd_ell_col, g.fwd_ell_src, g.bwd_ell_col, g.bwd_ell_src, g.fwd_lev_ptr,
                      g.bwd_lev_ptr, g.fwd_ell_w, g.bwd_ell_w, g.fwd_ell_off, g.bwd_ell_off};
         for (void* p : q) if (p) cudaFree(p);
     }
+}
+
+const PartDev* Mesh::part(int cs)
+{
+    std::lock_guard<std::mutex> lk(part_mu);
+    auto it = parts.find(cs);
+    if (it != parts.end()) return it->second.get();
+    const int n = h.n, ns = (n + 31) / 32;
+    auto P = std::make_unique<PartDev>();
+    P->cs = cs;
+    P->slots = P->own = P->len = P->nsl = 0;
+    std::vector<unsigned short> ca(h.sa.col.size()), cg(h.sg.col.size()), ct(h.st.col.size());
+    std::vector<std::vector<uint2>> places(cs);
+    auto owner = [&](int row) {
+        int r = (int)((long long)(row / 32) * cs / ns);
+        while ((int)((long long)ns * (r + 1) / cs) <= row / 32) r++;
+        while ((int)((long long)ns * r / cs) > row / 32) r--;
+        return r;
+    };
+    std::vector<int> slot(n, -1), halo;
+    for (int r = 0; r < cs; r++) {
+        const int s0 = (int)((long long)ns * r / cs), s1 = (int)((long long)ns * (r + 1) / cs);
+        const int r0 = s0 * 32, r1 = std::min(n, s1 * 32), own = std::max(0, r1 - r0);
+        halo.clear();
+        for (int i = r0; i < r1; i++)
+            for (int e = h.lrowptr[i]; e < h.lrowptr[i + 1]; e++) {
+                const int c = h.lcolidx[e];
+                if ((c < r0 || c >= r1) && slot[c] < 0) { slot[c] = 0; halo.push_back(c); }
+            }
+        std::sort(halo.begin(), halo.end());
+        P->slots = std::max(P->slots, own + (int)halo.size());
+        P->own = std::max(P->own, own);
+        P->nsl = std::max(P->nsl, s1 - s0);
+        P->len = std::max(P->len, h.sa.ptr[s1] - h.sa.ptr[s0] + h.sg.ptr[s1] - h.sg.ptr[s0] + h.st.ptr[s1] - h.st.ptr[s0]);
+        if (own + halo.size() > 65535) { parts[cs] = nullptr; return nullptr; }
+        for (int i = r0; i < r1; i++) slot[i] = i - r0;
+        for (size_t t = 0; t < halo.size(); t++) {
+            slot[halo[t]] = own + (int)t;
+            const int o = owner(halo[t]), o0 = (int)((long long)ns * o / cs) * 32;
+            places[o].push_back(uint2{(unsigned)(halo[t] - o0), (unsigned)r << 16 | (unsigned)(own + t)});
+        }
+        auto local = [&](const SellHost& s, std::vector<unsigned short>& c) {
+            for (int o = s.ptr[s0]; o < s.ptr[s1]; o++) c[o] = (unsigned short)slot[s.col[o]];
+        };
+        local(h.sa, ca);
+        local(h.sg, cg);
+        local(h.st, ct);
+        for (int i = r0; i < r1; i++) slot[i] = -1;
+        for (int c : halo) slot[c] = -1;
+    }
+    std::vector<uint2> push;
+    std::vector<int> pofs(cs + 1, 0);
+    P->npush = 0;
+    for (int r = 0; r < cs; r++) {
+        push.insert(push.end(), places[r].begin(), places[r].end());
+        pofs[r + 1] = (int)push.size();
+        P->npush = std::max(P->npush, (int)places[r].size());
+    }
+    P->ca = upload(ca);
+    P->cg = upload(cg);
+    P->ct = upload(ct);
+    P->pofs = upload(pofs);
+    P->push = upload(push);
+    const PartDev* p = P.get();
+    parts[cs] = std::move(P);
+    return p;
 }
 
 Mesh* mesh_build(int dim, int n, const double* coords, int ne, const int* el)
@@ -616,6 +735,7 @@ Mesh* mesh_build(int dim, int n, const double* coords, int ne, const int* el)
         if (m.diagpos[i] < 0) { delete M; throw Error{1, "node not referenced by any element"}; }
     layout_order(m);
     halo_lists(m);
+    sell_patterns(m);
     {
         std::vector<int> natkey(n);
         for (int i = 0; i < n; i++) natkey[i] = i;
@@ -649,6 +769,16 @@ Mesh* mesh_build(int dim, int n, const double* coords, int ne, const int* el)
     d.nel_list = upload(m.nel_list);
     d.nel_pos = upload(m.nel_pos);
     d.bndnode = upload(m.bndnode);
+    auto sell = [&](const SellHost& s, SellDev& g) {
+        g.ptr = upload(s.ptr);
+        g.col = upload(s.col);
+        g.src = upload(s.src);
+        g.len = (int)s.col.size();
+    };
+    sell(m.sa, d.sa);
+    sell(m.sg, d.sg);
+    sell(m.st, d.st);
+    d.gcnt = upload(m.gcnt);
     for (int t = 0; t < 2; t++) {
         const ICHost& c = m.ic[t];
         ICDev& g = d.ic[t];

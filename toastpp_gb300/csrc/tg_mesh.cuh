@@ -3,6 +3,9 @@
 // Built once per mesh on the host (the equivalent of Mesh::Setup), uploaded
 // once; every per-request step runs on the GPU.
 #pragma once
+#include <map>
+#include <memory>
+#include <mutex>
 #include <vector>
 #include "tg_common.cuh"
 
@@ -39,6 +42,18 @@ struct ICDev {
     int *fwd_lev_ptr, *bwd_lev_ptr, *fwd_ell_w, *bwd_ell_w, *fwd_ell_off, *bwd_ell_off;
 };
 
+// A sparsity pattern in slices of 32 rows: entry e of row r at ptr[r / 32] +
+// 32 e + r % 32 (col), the value's index in its source array (src); padding:
+// the row's own column, src -1.
+struct SellHost {
+    std::vector<int> ptr, col, src;
+};
+
+struct SellDev {
+    int *ptr, *col, *src;
+    int len;
+};
+
 struct MeshHost {
     int dim = 0, n = 0, ne = 0, nn = 0;
     std::vector<double> coords;       // n*dim
@@ -64,6 +79,13 @@ struct MeshHost {
     // the FP32 inner preconditioner of the mixed path
     ICHost ic[2];
     int ncolors = 0;
+    // the layout CSR in slices (src: CSR entries), and the pattern of the
+    // approximate inverse's factor G (tg_resident.cu): row r holds its
+    // neighbours of smaller layout position, ascending, then r (gcnt[r]
+    // entries, at most gmax); T is G transposed (src: entries of G's slices)
+    SellHost sa, sg, st;
+    std::vector<int> gcnt;
+    int gmax = 0;
     // assembly gather map: for F entry k, contributions (el*16 + i*4 + j) in element order
     std::vector<int> asm_ptr, asm_list;
     // node -> (element*4 + local index), element order
@@ -87,12 +109,32 @@ struct MeshDev {
     unsigned char* bndnode;
     double* intbff;            // ne*nn*nn boundary integrals BndIntFF (element basis, source vectors)
     ICDev ic[2];
+    SellDev sa, sg, st;
+    int* gcnt;
+};
+
+// The rows split into cs contiguous ranges (of whole slices), one per CTA of a
+// cluster: the slice columns as slots of the CTA's buffers (own rows, then its
+// halo, the other rows its rows refer to, ascending), and the copies of its
+// rows in other halos, {own slot, rank << 16 | slot there}, from pofs[rank].
+struct PartDev {
+    int cs, slots, own;                    // slots and own rows: the largest of the CTAs
+    int len, nsl;                          // entries of the three matrices and slices: the same
+    unsigned short *ca, *cg, *ct;          // columns of A, G and G^T
+    int npush;                             // halo copies of a CTA: the largest of the CTAs
+    int* pofs;
+    uint2* push;
 };
 
 struct Mesh {
     MeshHost h;
     MeshDev d{};
     int device = 0;
+    // the split for clusters of cs CTAs, built at its first use; null when a
+    // CTA's slots pass 16 bits
+    const PartDev* part(int cs);
+    std::mutex part_mu;
+    std::map<int, std::unique_ptr<PartDev>> parts;
     long long uid = 0;  // unique per mesh built in this process
     ~Mesh();
 };

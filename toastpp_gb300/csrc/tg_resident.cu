@@ -1,0 +1,742 @@
+// tg_resident.cu -- the mixed path's solve as one kernel: each thread-block
+// cluster runs a conjugate-gradient process on its own right-hand sides from
+// the first residual to the last FP64 correction.
+//
+// Why.  As separate launches an iteration was one SpMM, 2 x (levels) launches
+// of the triangular sweeps, five vector and reduction kernels, and every
+// fourth one a host read; each of them took 2 to 10 us whatever its size, so
+// solves were bound by launches and level latency (3.2k-node request: 92
+// iterations of 70 us; 30k-node request: 290 us an iteration of which about
+// 60 were memory time).  Right-hand sides never exchange data, so a cluster
+// that owns a few columns needs only its own barrier (a fraction of a
+// microsecond), the dot products meet in distributed shared memory, and the
+// host is not asked until the solve has ended.
+//
+// Preconditioner.  A triangular sweep has one dependent step per level (22 in
+// 3D with a colour ordering).  In its place stands a factorised sparse
+// approximate inverse (Kolotilina and Yeremin 1993): G lower triangular on
+// A's own pattern with G A G^T close to 1, row i of G from the small system
+// A(S, S) y = e_last over the row's pattern S, scaled to unit diagonal of
+// G A G^T.  Applying it is two sparse products without any dependence.  On
+// these systems it takes 1.12 to 1.15 times the iterations of IC(0) in the
+// colour ordering.  G works for the complex symmetric systems unchanged, with
+// the bilinear product throughout.
+//
+// On-chip state.  A cluster of cs CTAs splits the rows (the mesh's Morton
+// layout) into cs contiguous ranges.  Each CTA keeps its rows of p, r and
+// t = G r in shared memory, with a copy of the rows of other CTAs that its
+// matrix rows refer to (its halo); whoever computes such a row stores it into
+// the halos too, through distributed shared memory.  So every gather of the
+// three products is a shared-memory read; only matrix values (10 bytes an
+// entry with 16-bit local columns) and x stream from L2, and where the matrices
+// fit too they are copied in once.  With the vectors in global memory the same
+// process was bound by the rate of L1 lookups: 50 us an iteration on the
+// 12.5k-node disc with 64 columns, 35 with them on chip, and 22 against 11 on
+// the 3.2k-node disc with 32.
+//
+// Measured, whole requests before and after: 217 nodes, 8 columns 2.88 -> 0.49
+// ms; 3.2k nodes CW, 32 columns 8.41 -> 1.00 ms; data gradient on 12.5k nodes
+// (two solves of 32 columns) 157 -> 8.2 ms, of which most was columns whose
+// residuals the float-float product could not resolve (below).
+//
+// Thread mapping: a thread per row, with the cluster's LV columns as one word
+// of 4 to 16 bytes.  (Sharing a row between lanes, for more columns a cluster,
+// was never faster.)
+#include "tg_cluster.cuh"
+#include "tg_jac.cuh"
+
+namespace tg {
+
+template <int LV, class V>
+struct alignas(LV * sizeof(V)) VecN {
+    V v[LV];
+};
+
+__device__ __forceinline__ int cl_rank()
+{
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int)r;
+}
+
+// all threads of the cluster (cs = 1: of the CTA); writes before it are seen
+// by every thread after it
+__device__ __forceinline__ void cl_sync(int cs)
+{
+    if (cs == 1) {
+        __syncthreads();
+    } else {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+}
+
+// the shared::cluster address of this CTA's shared variable p in CTA `rank`
+__device__ __forceinline__ unsigned cl_map(const void* p, int rank)
+{
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cl_store(unsigned a, float2 v)
+{
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void cl_store(unsigned a, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+template <int B>
+__device__ __forceinline__ void cl_store_bytes(unsigned a, const void* v)
+{
+    const float* f = (const float*)v;
+    if constexpr (B == 4) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(f[0]) : "memory");
+    else if constexpr (B == 8) cl_store(a, make_float2(f[0], f[1]));
+    else asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]) : "memory");
+}
+
+// a compensated FP32 sum (TwoSum): about 2^-46 relative, without FP64 adds
+struct FSum {
+    float h = 0.f, l = 0.f;
+    __device__ __forceinline__ void add(float x)
+    {
+        const float s = __fadd_rn(h, x), b = __fsub_rn(s, h);
+        l += __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(x, b));
+        h = s;
+    }
+    __device__ __forceinline__ void add(const FSum& o)
+    {
+        l += o.l;
+        add(o.h);
+    }
+};
+
+// FP32 scalar arithmetic of the recursions: a / b (Smith's scaling for complex
+// values), and the square root with non-negative real part
+__device__ __forceinline__ float sdiv(float a, float b) { return a / b; }
+__device__ __forceinline__ cf sdiv(cf a, cf b)
+{
+    if (fabsf(b.x) >= fabsf(b.y)) {
+        const float r = b.y / b.x, d = 1.0f / (b.x + b.y * r);
+        return cf{(a.x + a.y * r) * d, (a.y - a.x * r) * d};
+    }
+    const float r = b.x / b.y, d = 1.0f / (b.x * r + b.y);
+    return cf{(a.x * r + a.y) * d, (a.y * r - a.x) * d};
+}
+template <class V> __device__ __forceinline__ V smake(float r, float i);
+template <> __device__ __forceinline__ float smake<float>(float r, float) { return r; }
+template <> __device__ __forceinline__ cf smake<cf>(float r, float i) { return cf{r, i}; }
+__device__ __forceinline__ float ssqrt(float a) { return sqrtf(a); }
+__device__ __forceinline__ cf ssqrt(cf z)
+{
+    const float r = hypotf(z.x, z.y);
+    if (r == 0.f) return cf{0.f, 0.f};
+    if (z.x >= 0.f) {
+        const float t = sqrtf(0.5f * (r + z.x));
+        return cf{t, z.y / (2.f * t)};
+    }
+    const float t = sqrtf(0.5f * (r - z.x));
+    return cf{fabsf(z.y) / (2.f * t), z.y < 0.f ? -t : t};
+}
+__device__ __forceinline__ bool sfinite(float a) { return isfinite(a); }
+__device__ __forceinline__ bool sfinite(cf a) { return isfinite(a.x) && isfinite(a.y); }
+__device__ __forceinline__ bool szero(float a) { return a == 0.f; }
+__device__ __forceinline__ bool szero(cf a) { return a.x == 0.f && a.y == 0.f; }
+
+// ---------------------------------------------------------------------------
+// G of the approximate inverse: a warp per row.  The row's pattern S (m
+// entries, ascending, the row itself last) is in the slice layout; the warp
+// gathers A(S, S) into shared memory, factors it L D L^T in place (lane =
+// row), and back-substitutes L^T y = e_m; the row is y / sqrt(d_m).  A row
+// whose pivots are not finite keeps its scaled diagonal alone.
+// ---------------------------------------------------------------------------
+template <class V>
+__global__ void __launch_bounds__(32 * FSAI_WARPS) fsai_kernel(int n, const int* __restrict__ rowptr,
+                                                              const int* __restrict__ colidx,
+                                                              const int* __restrict__ diagpos,
+                                                              const V* __restrict__ A, const int* __restrict__ gptr,
+                                                              const int* __restrict__ gcol,
+                                                              const int* __restrict__ gcnt, V* __restrict__ gval)
+{
+    __shared__ V sm[FSAI_WARPS][FSAI_MAXM][FSAI_MAXM + 1];
+    __shared__ int ss[FSAI_WARPS][FSAI_MAXM];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * FSAI_WARPS + w;
+    if (i >= n) return;
+    V(*M)[FSAI_MAXM + 1] = sm[w];
+    int* S = ss[w];
+    const int m = gcnt[i], base = gptr[i >> 5] + (i & 31);
+    if (lane < m) S[lane] = gcol[base + 32 * lane];
+    for (int a = 0; a < m; a++)
+        if (lane < m) M[a][lane] = vzero<V>();
+    __syncwarp();
+    for (int a = 0; a < m; a++) {
+        const int ra = S[a];
+        for (int p = rowptr[ra] + lane; p < rowptr[ra + 1]; p += 32) {
+            const int c = colidx[p];
+            for (int b = 0; b <= a; b++)
+                if (S[b] == c) M[a][b] = A[p];
+        }
+    }
+    __syncwarp();
+    bool ok = true;
+    for (int j = 0; j < m; j++) {
+        const V d = M[j][j];
+        ok &= sfinite(d) && !szero(d) && re(d) > 0.f;
+        if (!ok) break;  // the same value in every lane
+        V l = vzero<V>();
+        if (lane > j && lane < m) {
+            l = sdiv(M[lane][j], d);
+            for (int c = j + 1; c <= lane; c++) M[lane][c] = vfms(M[lane][c], l, M[c][j]);
+        }
+        __syncwarp();
+        if (lane > j && lane < m) M[lane][j] = l;
+        __syncwarp();
+    }
+    V y = vzero<V>();
+    if (ok) {
+        // lane j holds y_j
+        y = lane == m - 1 ? vmake<V>(1.0, 0.0) : vzero<V>();
+        for (int r = m - 1; r > 0; r--) {
+            const V yr = shfl(y, r);
+            if (lane < r) y = vfms(y, M[r][lane], yr);
+        }
+        const V s = sdiv(vmake<V>(1.0, 0.0), ssqrt(M[m - 1][m - 1]));
+        y = vmul(y, s);
+        ok = __all_sync(0xffffffffu, lane >= m || sfinite(y));
+    }
+    if (!ok) y = lane == m - 1 ? sdiv(vmake<V>(1.0, 0.0), ssqrt(A[diagpos[i]])) : vzero<V>();
+    if (lane < m) gval[base + 32 * lane] = y;
+    // padding entries of the slice
+    const int wd = (gptr[(i >> 5) + 1] - gptr[i >> 5]) >> 5;
+    for (int e = m + lane; e < wd; e += 32) gval[base + 32 * e] = vzero<V>();
+}
+
+// ---------------------------------------------------------------------------
+// The resident solve.
+// ---------------------------------------------------------------------------
+// per-column state of the process, in every CTA's shared memory
+template <class V>
+struct ResCols {
+    V alpha[CL_MAXCG], beta[CL_MAXCG], zr[CL_MAXCG];
+    float bn[CL_MAXCG], err[CL_MAXCG], fs[CL_MAXCG], thr[CL_MAXCG];
+    double bnorm[CL_MAXCG], oerr[CL_MAXCG], scale[CL_MAXCG], berr[CL_MAXCG];
+    int outer[CL_MAXCG], on[CL_MAXCG], rel[CL_MAXCG], its[CL_MAXCG], st[CL_MAXCG], ost[CL_MAXCG], nupd[CL_MAXCG];
+};
+
+template <class V64, class V, int LV>
+__global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a)
+{
+    constexpr bool CPLX = vt<V>::cplx;
+    const int NT = blockDim.x, NW = NT >> 5;
+    using VN = VecN<LV, V>;
+    constexpr int U = 8;   // entries of a matrix row in flight
+    constexpr int RX = 2;  // rows in flight of the x update
+    __shared__ ResCols<V> S;
+    __shared__ __align__(16) float2 s_w[CL_NT / 32][CL_MAXCG * CL_NV];
+    __shared__ float2 s_red[2][CL_MAXCS][CL_MAXCG * CL_NV];
+    __shared__ double s_nrm[CL_MAXCS][CL_MAXCG * 2];
+    extern __shared__ __align__(16) unsigned char cl_sm[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int CG = LV;
+    const int cs = a.cs, rank = cs > 1 ? cl_rank() : 0;
+    const int grp = blockIdx.x / cs, cg0 = grp * CG;       // this cluster's first column
+    const int nc = min(CG, a.k - cg0);                     // columns of the cluster
+    const int n = a.n, k = a.k, ns = (n + 31) >> 5;
+    const int R0 = (int)((long long)ns * rank / cs) * 32, R1 = min(n, (int)((long long)ns * (rank + 1) / cs) * 32);
+    const int rb = R0 + tid, rs = NT;                      // a thread per row
+    // gather buffers of p, r and t (q in between), and z of the own rows
+    V* bp = reinterpret_cast<V*>(cl_sm);
+    V* br = bp + (size_t)a.slots * CG;
+    V* bt = br + (size_t)a.slots * CG;
+    V* bz = bt + (size_t)a.slots * CG;
+    V* x = a.x + (size_t)grp * n * CG;
+    // the slice pointers of this CTA's rows, and the matrices where they fit, go
+    // to shared memory behind the vectors
+    Sell<V> M[3] = {a.A, a.G, a.T};
+    {
+        const int s0 = R0 >> 5, s1 = (R1 + 31) >> 5;
+        V* vp = reinterpret_cast<V*>(cl_sm + a.mofs_val);
+        unsigned short* cp = reinterpret_cast<unsigned short*>(cl_sm + a.mofs_col);
+        int* pp = reinterpret_cast<int*>(cl_sm + a.mofs_ptr);
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            const int b = M[m].ptr[s0], len = M[m].ptr[s1] - b;
+            for (int o = tid; o <= s1 - s0; o += NT) pp[o] = M[m].ptr[s0 + o];
+            if (a.msm) {
+                for (int o = tid; o < len; o += NT) { vp[o] = M[m].val[b + o]; cp[o] = M[m].col[b + o]; }
+                M[m].val = vp - b;
+                M[m].col = cp - b;
+                vp += len;
+                cp += len;
+            }
+            M[m].ptr = pp - s0;
+            pp += s1 - s0 + 1;
+        }
+    }
+    int rbuf = 0;
+    auto at = [&](V* v, int i) -> VN& { return *reinterpret_cast<VN*>(v + (i - R0) * CG); };
+    auto gx = [&](int i) -> VN& { return *reinterpret_cast<VN*>(x + (size_t)i * CG); };
+    // this CTA's rows of a gather buffer into the other CTAs' halos, then the
+    // cluster's barrier
+    uint2* const push = reinterpret_cast<uint2*>(cl_sm + a.mofs_push);
+    const int npush = cs > 1 ? a.pofs[rank + 1] - a.pofs[rank] : 0;
+    auto share = [&](V* v) {
+        if (cs > 1) {
+            __syncthreads();
+            for (int t = tid; t < npush; t += NT) {
+                const uint2 e = push[t];
+                const VN y = *reinterpret_cast<const VN*>(v + e.x * CG);
+                cl_store_bytes<sizeof(VN)>(cl_map(v + (e.y & 0xffffu) * CG, (int)(e.y >> 16)), &y);
+            }
+        }
+        cl_sync(cs);
+    };
+    // Sums (mx: the last quantity is a maximum) of nv quantities per column
+    // over the cluster, in a fixed order; red(c, i) reads the result.  All
+    // writes before it are visible after it.
+    auto reduce = [&](FSum (&v)[LV][CL_NV], int nv, bool mx) {
+        for (int o = 16; o; o >>= 1)
+#pragma unroll
+            for (int j = 0; j < LV; j++)
+#pragma unroll
+                for (int i = 0; i < CL_NV; i++)
+                    if (i < nv) {
+                        FSum t;
+                        t.h = __shfl_xor_sync(0xffffffffu, v[j][i].h, o);
+                        t.l = __shfl_xor_sync(0xffffffffu, v[j][i].l, o);
+                        if (mx && i == nv - 1) v[j][i].h = fmaxf(v[j][i].h, t.h);
+                        else v[j][i].add(t);
+                    }
+        if (lane == 0)
+#pragma unroll
+            for (int j = 0; j < LV; j++)
+#pragma unroll
+                for (int i = 0; i < CL_NV; i++)
+                    if (i < nv) s_w[warp][j * CL_NV + i] = make_float2(v[j][i].h, v[j][i].l);
+        __syncthreads();
+        for (int t = warp; t < CG * CL_NV; t += NW) {
+            const int i = t % CL_NV;
+            if (i >= nv) continue;
+            FSum s;
+            if (lane < NW) { const float2 w = s_w[lane][t]; s.h = w.x; s.l = w.y; }
+            for (int o = 16; o; o >>= 1) {
+                FSum u;
+                u.h = __shfl_xor_sync(0xffffffffu, s.h, o);
+                u.l = __shfl_xor_sync(0xffffffffu, s.l, o);
+                if (mx && i == nv - 1) s.h = fmaxf(s.h, u.h);
+                else s.add(u);
+            }
+            if (cs == 1) { if (lane == 0) s_red[rbuf][0][t] = make_float2(s.h, s.l); }
+            else if (lane < cs) cl_store(cl_map(&s_red[rbuf][rank][t], lane), make_float2(s.h, s.l));
+        }
+        cl_sync(cs);
+        rbuf ^= 1;
+    };
+    auto red = [&](int c, int i, bool mx) {
+        FSum s;
+        for (int d = 0; d < cs; d++) {
+            const float2 t = s_red[rbuf ^ 1][d][c * CL_NV + i];
+            if (mx) s.h = fmaxf(s.h, t.x);
+            else { FSum u; u.h = t.x; u.l = t.y; s.add(u); }
+        }
+        return s.h + s.l;
+    };
+    for (int t = tid; t < npush; t += NT) push[t] = a.push[a.pofs[rank] + t];
+    // every CTA of the cluster runs before any stores into another's shared memory
+    cl_sync(cs);
+    // ---- start: r = b (zero guess) or the residual in R; norms in FP64
+    {
+        double v[LV][2];
+#pragma unroll
+        for (int j = 0; j < LV; j++) v[j][0] = v[j][1] = 0.0;
+        for (int i = rb; i < R1; i += rs)
+#pragma unroll
+            for (int j = 0; j < LV; j++)
+                if (j < nc) {
+                    const size_t o = (size_t)i * k + cg0 + j;
+                    v[j][0] += nrm2(a.B[o]);
+                    if (!a.zero_guess) v[j][1] += nrm2(a.R[o]);
+                }
+        double* w = reinterpret_cast<double*>(s_w);  // [NW][2 CG]
+        for (int o = 16; o; o >>= 1)
+#pragma unroll
+            for (int j = 0; j < LV; j++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) v[j][i] += __shfl_xor_sync(0xffffffffu, v[j][i], o);
+        if (lane == 0)
+#pragma unroll
+            for (int j = 0; j < LV; j++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) w[warp * 2 * CG + j * 2 + i] = v[j][i];
+        __syncthreads();
+        if (tid < 2 * CG) {
+            double s = 0.0;
+            for (int u = 0; u < NW; u++) s += w[u * 2 * CG + tid];
+            if (cs == 1) s_nrm[0][tid] = s;
+            else
+                for (int d = 0; d < cs; d++) cl_store(cl_map(&s_nrm[rank][tid], d), s);
+        }
+        cl_sync(cs);
+    }
+    if (tid < CG) {
+        const int c = tid;
+        double b2 = 0.0, r2 = 0.0;
+        for (int d = 0; d < cs; d++) { b2 += s_nrm[d][2 * c]; r2 += s_nrm[d][2 * c + 1]; }
+        const double tol = c < nc ? a.co[cg0 + c].tol : 0.0, bn = sqrt(b2), er = a.zero_guess ? bn : sqrt(r2);
+        int on = c < nc && bn > 0.0;
+        S.berr[c] = 1.0;
+        S.bnorm[c] = bn;
+        S.oerr[c] = er;
+        // with a componentwise bound only an exact initial guess stops here
+        if (on && er <= tol * bn && (a.cwtol <= 0.0 || er == 0.0)) { on = 0; S.berr[c] = 0.0; }
+        S.outer[c] = S.on[c] = on;
+        S.scale[c] = pow2_floor(er);
+        S.bn[c] = S.err[c] = (float)(er / S.scale[c]);
+        S.rel[c] = S.its[c] = S.st[c] = S.ost[c] = S.nupd[c] = 0;
+        S.alpha[c] = S.beta[c] = S.zr[c] = vzero<V>();
+    }
+    __syncthreads();
+    for (int i = rb; i < R1; i += rs) {
+        VN rv, zero;
+#pragma unroll
+        for (int j = 0; j < LV; j++) {
+            zero.v[j] = rv.v[j] = vzero<V>();
+            if (j < nc && S.outer[j]) {
+                const size_t o = (size_t)i * k + cg0 + j;
+                rv.v[j] = vcast<V, V64>(vscale(a.zero_guess ? a.B[o] : a.R[o], 1.0 / S.scale[j]));
+            }
+        }
+        at(br, i) = rv;
+        gx(i) = zero;
+        at(bp, i) = zero;
+    }
+    share(br);
+    // The process as a sequence of products, so that each piece of code stands
+    // once (a turn is short enough for instruction fetches to count):
+    //   1  t = G r
+    //   2  z = G^T t, rho = r.z, then the scalars of the step that left r, the
+    //      corrections when they are due, and p = z + beta p
+    //   0  q = A p, alpha, then x += alpha p, r -= alpha q
+    // mode: what r is, 0 the start, 1 an iteration's, 2 a corrected residual.
+    int mode = 0, it = 0, ph = 1;
+    bool run = true;
+    FSum v[LV][CL_NV];
+    for (;;) {
+        const V* src = ph == 0 ? bp : ph == 1 ? br : bt;
+        V* dst = ph == 2 ? bz : bt;
+        const V* dw = ph == 0 ? bp : br;
+        const Sell<V> Mx = ph == 0 ? M[0] : ph == 1 ? M[1] : M[2];
+        if (run)
+            for (int i = rb; i < R1; i += rs) {
+                const int b = Mx.ptr[i >> 5], w = (Mx.ptr[(i >> 5) + 1] - b) >> 5;
+                const unsigned short* col = Mx.col + b + (i & 31);
+                const V* val = Mx.val + b + (i & 31);
+                VN acc;
+#pragma unroll
+                for (int j = 0; j < LV; j++) acc.v[j] = vzero<V>();
+#pragma unroll 1
+                for (int e = 0; e < w; e += U) {
+                    int c[U];
+                    V av[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (e + u < w) { c[u] = col[32 * (e + u)]; av[u] = val[32 * (e + u)]; }
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (e + u < w) {
+                            const VN g = *reinterpret_cast<const VN*>(src + c[u] * CG);
+#pragma unroll
+                            for (int j = 0; j < LV; j++) acc.v[j] = vfma(acc.v[j], av[u], g.v[j]);
+                        }
+                }
+                at(dst, i) = acc;
+                if (ph != 1) {
+                    const VN wv = *reinterpret_cast<const VN*>(dw + (i - R0) * CG);
+#pragma unroll
+                    for (int j = 0; j < LV; j++) {
+                        const V t = vmul(wv.v[j], acc.v[j]);
+                        v[j][0].add(re(t));
+                        if (CPLX) v[j][1].add(im(t));
+                    }
+                }
+            }
+        if (ph == 1) {
+            share(bt);
+            ph = 2;
+            continue;
+        }
+        reduce(v, 3, false);
+        if (ph == 0) {
+            if (tid < CG && S.on[tid]) {
+                const V al = sdiv(S.zr[tid], smake<V>(red(tid, 0, false), CPLX ? red(tid, 1, false) : 0.f));
+                S.alpha[tid] = al;
+                if (!sfinite(al)) { S.on[tid] = 0; S.st[tid] = 2; }
+            }
+            __syncthreads();
+            bool on[LV], any = false;
+            V sc[LV];
+#pragma unroll
+            for (int j = 0; j < LV; j++) {
+                on[j] = S.on[j]; any |= on[j]; sc[j] = S.alpha[j];
+#pragma unroll
+                for (int i = 0; i < CL_NV; i++) v[j][i] = FSum();
+            }
+            if (any)
+                for (int i = rb; i < R1; i += RX * rs) {
+                    VN xv[RX];
+#pragma unroll
+                    for (int u = 0; u < RX; u++)
+                        if (i + u * rs < R1) xv[u] = gx(i + u * rs);
+#pragma unroll
+                    for (int u = 0; u < RX; u++) {
+                        const int o = i + u * rs;
+                        if (o >= R1) continue;
+                        VN rv = at(br, o);
+                        const VN pv = at(bp, o), qv = at(bt, o);
+#pragma unroll
+                        for (int j = 0; j < LV; j++)
+                            if (on[j]) {
+                                xv[u].v[j] = vfma(xv[u].v[j], sc[j], pv.v[j]);
+                                rv.v[j] = vfms(rv.v[j], sc[j], qv.v[j]);
+                                v[j][2].add(nrm2(rv.v[j]));
+                            }
+                        gx(o) = xv[u];
+                        at(br, o) = rv;
+                    }
+                }
+            share(br);
+            mode = 1;
+            run = any;
+            ph = 1;
+            continue;
+        }
+        if (tid < CG) {
+            const int c = tid;
+            const V rz = smake<V>(red(c, 0, false), CPLX ? red(c, 1, false) : 0.f);
+            bool go = S.on[c];
+            if (mode == 1 && go) {
+                S.err[c] = sqrtf(red(c, 2, false));
+                S.its[c]++;
+                go = false;
+                if (S.err[c] <= a.trig * S.bn[c]) { S.on[c] = 0; S.st[c] = 0; }
+                else if (S.its[c] >= a.maxit) { S.on[c] = 0; S.st[c] = 1; }
+                // a process that grows has lost its directions: it restarts
+                else if (!(S.err[c] <= 100.f * S.bn[c])) { S.on[c] = 0; S.st[c] = 2; }
+                else go = true;
+            }
+            if (mode == 2) go = S.rel[c] != 0;
+            if (go) {
+                const V be = mode == 0 || S.rel[c] == 2 ? vzero<V>() : sdiv(rz, S.zr[c]);
+                S.beta[c] = be;
+                S.zr[c] = rz;
+                S.rel[c] = 0;
+                if (szero(rz) || !sfinite(rz) || !sfinite(be)) { S.on[c] = 0; S.st[c] = 2; }
+            }
+        }
+        __syncthreads();
+        if (mode == 1) {
+        it++;
+        int nact = 0, nwait = 0;
+        for (int c = 0; c < CG; c++) { nact += S.outer[c]; nwait += S.outer[c] && !S.on[c]; }
+        const bool limit = it >= a.maxit;
+        if (nact == 0) break;
+        // corrections: every fourth iteration, or when no column iterates
+        if ((nwait && ((it & 3) == 0 || nwait == nact)) || limit) {
+        __syncthreads();
+        if (tid < CG) {
+            const int c = tid;
+            // 1: the trigger was reached, the process goes on; 2: it restarts
+            S.rel[c] = S.outer[c] ? (S.on[c] ? (limit ? 1 : 0) : (S.st[c] == 0 ? 1 : 2)) : 0;
+            // rows whose float-float residual may be off by more than a
+            // thousandth of the residual that the recursion expects are formed
+            // in FP64 (float-float carries about 2^-46 of |A||x|)
+            S.thr[c] = a.all64 ? -1.f : (float)((double)S.err[c] * 1e-3 * 70368744177664.0);
+        }
+        __syncthreads();
+        bool rel[LV], anyr = false;
+#pragma unroll
+        for (int j = 0; j < LV; j++) { rel[j] = S.rel[j]; anyr |= rel[j]; }
+        if (anyr)
+            for (int i = rb; i < R1; i += rs) {
+                VN xv = gx(i);
+#pragma unroll
+                for (int j = 0; j < LV; j++)
+                    if (rel[j]) {
+                        const size_t o = (size_t)i * k + cg0 + j;
+                        // (the correction of a process that grew is dropped)
+                        const V64 s = S.err[j] <= S.bn[j] ? vadd(a.X[o], vscale(vcast<V64, V>(xv.v[j]), S.scale[j])) : a.X[o];
+                        a.X[o] = s;
+                        const float2 h = ff_split(re(s)), l = ff_split(im(s));
+                        if constexpr (CPLX) ((float4*)a.Xff)[o] = make_float4(h.x, h.y, l.x, l.y);
+                        else ((float2*)a.Xff)[o] = h;
+                        xv.v[j] = vzero<V>();
+                    }
+                gx(i) = xv;
+            }
+        cl_sync(cs);
+        // the true residual b - A x, its norm and the componentwise backward error
+        {
+            FSum w[LV][CL_NV];
+            if (anyr)
+                for (int i = rb; i < R1; i += rs) {
+                    const int e0 = a.rowptr[i], e1 = a.rowptr[i + 1];
+#pragma unroll
+                    for (int j = 0; j < LV; j++) {
+                        if (!rel[j]) continue;
+                        const int c = cg0 + j;
+                        float d = 0.f;
+                        V64 ax;
+                        f2x h = 0ull, l = 0ull;
+#pragma unroll 2
+                        for (int e = e0; e < e1; e++) {
+                            const size_t o = (size_t)a.colidx[e] * k + c;
+                            if constexpr (CPLX) {
+                                const float4 f = ((const float4*)a.Aff)[e], xf = ((const float4*)a.Xff)[o];
+                                ff2_mac(h, l, f2_bcast(f.x), f2_bcast(f.y), f2_pack(xf.x, xf.z), f2_pack(xf.y, xf.w));
+                                ff2_mac(h, l, f2_pack(-f.z, f.z), f2_pack(-f.w, f.w), f2_pack(xf.z, xf.x),
+                                        f2_pack(xf.w, xf.y));
+                                d = fmaf(a.absA[e], fmaxf(fabsf(xf.x), fabsf(xf.z)), d);
+                            } else {
+                                const float2 f = ((const float2*)a.Aff)[e], xf = ((const float2*)a.Xff)[o];
+                                ff2_mac(h, l, f2_bcast(f.x), f2_bcast(f.y), f2_bcast(xf.x), f2_bcast(xf.y));
+                                d = fmaf(a.absA[e], fabsf(xf.x), d);
+                            }
+                        }
+                        const size_t o = (size_t)i * k + c;
+                        const V64 b = a.B[o];
+                        d += mag1f(b);
+                        if (d > S.thr[j] * (float)S.scale[j]) {
+                            ax = vzero<V64>();
+                            for (int e = e0; e < e1; e++) ax = vfma(ax, a.A64[e], a.X[(size_t)a.colidx[e] * k + c]);
+                        } else {
+                            const float2 hh = f2_unpack(h), ll = f2_unpack(l);
+                            if constexpr (CPLX) ax = V64{oz_to_double(hh.x, ll.x, 0), oz_to_double(hh.y, ll.y, 0)};
+                            else ax = oz_to_double(hh.x, ll.x, 0);
+                        }
+                        const V64 rv = vsub(b, ax);
+                        a.R[o] = rv;
+                        const float m = mag1f(rv), qd = m == 0.f ? 0.f : (d > 0.f ? m / d : INFINITY);
+                        // a NaN must not pass the test
+                        w[j][1].h = qd <= w[j][1].h ? w[j][1].h : (qd == qd ? qd : INFINITY);
+                        w[j][0].add(nrm2(vcast<V, V64>(vscale(rv, 1.0 / S.scale[j]))));
+                    }
+                }
+            reduce(w, 2, true);
+        }
+        if (tid < CG && S.rel[tid]) {
+            const int c = tid;
+            const double er = sqrt((double)red(c, 0, false)) * S.scale[c], tol = a.co[cg0 + c].tol;
+            S.oerr[c] = er;
+            if (a.cwtol > 0.0) S.berr[c] = red(c, 1, true);
+            if (er <= tol * S.bnorm[c] && (a.cwtol <= 0.0 || S.berr[c] <= a.cwtol)) {
+                S.outer[c] = S.on[c] = S.rel[c] = 0;
+                S.ost[c] = 0;
+            } else if (limit || ++S.nupd[c] >= a.max_upd || !isfinite(er)) {
+                S.outer[c] = S.on[c] = S.rel[c] = 0;
+                S.ost[c] = 1;
+            } else {
+                // a true residual above the recursive one: the process no longer
+                // follows the FP64 system and restarts from it.  (Off the rounding
+                // floor the two agree to 1e-3; with the line at 8 a column at 7.4
+                // kept its old directions and diverged on the 919-node disc.)
+                if (er > 1.25 * S.err[c] * S.scale[c]) S.rel[c] = 2;
+                const double old = S.scale[c];
+                S.scale[c] = pow2_floor(er);
+                const float f = (float)(old / S.scale[c]);
+                S.fs[c] = f;
+                S.bn[c] = (float)(er / S.scale[c]);
+                S.zr[c] = vscale(S.zr[c], f * f);
+                S.on[c] = 1;
+                S.st[c] = 0;
+            }
+        }
+        __syncthreads();
+        if (limit) break;
+        anyr = false;
+#pragma unroll
+        for (int j = 0; j < LV; j++) { rel[j] = S.rel[j]; anyr |= rel[j]; }
+        int nrel = 0;
+        for (int c = 0; c < CG; c++) nrel += S.rel[c] != 0;
+        if (nrel) {
+            // the columns go on from the true residual: r and p in the new scale
+            if (anyr)
+                for (int i = rb; i < R1; i += rs) {
+                    VN rv = at(br, i), pv = at(bp, i);
+#pragma unroll
+                    for (int j = 0; j < LV; j++)
+                        if (rel[j]) {
+                            const int c = j;
+                            rv.v[j] = vcast<V, V64>(vscale(a.R[(size_t)i * k + cg0 + c], 1.0 / S.scale[c]));
+                            pv.v[j] = S.rel[c] == 2 ? vzero<V>() : vscale(pv.v[j], S.fs[c]);
+                        }
+                    at(br, i) = rv;
+                    at(bp, i) = pv;
+                }
+            share(br);
+            mode = 2;
+            run = anyr;
+            ph = 1;
+#pragma unroll
+            for (int j = 0; j < LV; j++)
+#pragma unroll
+                for (int i = 0; i < CL_NV; i++) v[j][i] = FSum();
+            continue;
+        }
+        }
+        }
+        bool on[LV], any = false;
+        V sc[LV];
+#pragma unroll
+        for (int j = 0; j < LV; j++) {
+            on[j] = S.on[j]; any |= on[j]; sc[j] = S.beta[j];
+#pragma unroll
+            for (int i = 0; i < CL_NV; i++) v[j][i] = FSum();
+        }
+        if (any)
+            for (int i = rb; i < R1; i += rs) {
+                VN pv = at(bp, i);
+                const VN zv = at(bz, i);
+#pragma unroll
+                for (int j = 0; j < LV; j++)
+                    if (on[j]) pv.v[j] = vfma(zv.v[j], sc[j], pv.v[j]);
+                at(bp, i) = pv;
+            }
+        share(bp);
+        run = any;
+        ph = 0;
+    }
+    // results; no CTA leaves while another may still write its shared memory
+    __syncthreads();
+    if (rank == 0 && tid < nc) {
+        ColState& O = a.co[cg0 + tid];
+        O.bnorm = S.bnorm[tid];
+        O.err = S.oerr[tid];
+        O.berr = S.berr[tid];
+        O.its = S.its[tid];
+        O.status = S.outer[tid] ? 1 : S.ost[tid];
+        O.active = 0;
+    }
+    cl_sync(cs);
+}
+
+template <class V64, class V32>
+void (*resident_kernel(int lv))(ResArgs<V64, V32>)
+{
+    if constexpr (sizeof(V32) == 4)
+        if (lv == 4) return resident_cg_kernel<V64, V32, 4>;
+    return lv == 2 ? resident_cg_kernel<V64, V32, 2> : resident_cg_kernel<V64, V32, 1>;
+}
+template void (*resident_kernel<double, float>(int))(ResArgs<double, float>);
+template void (*resident_kernel<cd, cf>(int))(ResArgs<cd, cf>);
+
+template <class V>
+void (*fsai_kernel_of())(int, const int*, const int*, const int*, const V*, const int*, const int*, const int*, V*)
+{
+    return fsai_kernel<V>;
+}
+template void (*fsai_kernel_of<float>())(int, const int*, const int*, const int*, const float*, const int*, const int*,
+                                         const int*, float*);
+template void (*fsai_kernel_of<cf>())(int, const int*, const int*, const int*, const cf*, const int*, const int*,
+                                      const int*, cf*);
+
+}  // namespace tg

@@ -16,6 +16,7 @@
 
 #include "../../include/toastgpu.h"
 #include "tg_jac.cuh"
+#include "tg_cluster.cuh"
 #include "tg_gmres.cuh"
 #include "tg_grid.cuh"
 
@@ -78,6 +79,33 @@ static inline void launch_pdl(void (*k)(KArgs...), dim3 g, dim3 b, size_t sm, cu
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    TG_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...));
+    g_nlaunch.fetch_add(1, std::memory_order_relaxed);
+}
+
+// ng clusters of cs CTAs (cs = 1: plain CTAs) of nt threads
+static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, unsigned ng, int cs, int nt, size_t sm,
+                           cudaStream_t st)
+{
+    cfg.gridDim = dim3(ng * (unsigned)cs);
+    cfg.blockDim = dim3((unsigned)nt);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cs > 1 ? 1 : 0;
+}
+
+template <class... KArgs, class... Args>
+static inline void launch_cluster(void (*k)(KArgs...), unsigned ng, int cs, int nt, size_t sm, cudaStream_t st,
+                                  Args&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cluster_config(cfg, at, ng, cs, nt, sm, st);
     TG_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...));
     g_nlaunch.fetch_add(1, std::memory_order_relaxed);
 }
@@ -1828,6 +1856,17 @@ struct LinkCache {
     bool qm_on_dev = false, pair_on_dev = false;
 };
 
+// The shape of a resident solve: lv columns a cluster of cs CTAs (0: none) of
+// nt threads; sm bytes of shared memory with the parts at mofs_*, msm: the
+// matrices among them
+struct ClShape {
+    int lv = 1, cs = 0, nt = CL_NT;
+    size_t sm = 0;
+    const PartDev* part = nullptr;
+    bool msm = false;
+    int mofs_val = 0, mofs_col = 0, mofs_ptr = 0, mofs_push = 0;
+};
+
 struct tg_solver_s {
     Mesh* mesh = nullptr;
     int cplx = 0, method = 1, precon = 2, precision = 0, maxit = 0;
@@ -1847,6 +1886,10 @@ struct tg_solver_s {
     cudaEvent_t jev[2] = {nullptr, nullptr}, jready = nullptr;
     int jflip = 0;
     bool reset_done = false;
+    bool ic_done = false;      // the factor of the current matrix is in place
+    bool res_ready = false;    // and the resident solve's matrices
+    std::map<int, ClShape> shapes;  // by number of columns
+    DBuf sa32, sg32, st32, xff, xkeep;  // resident solve: sliced matrices, split solution, kept guess
     DBuf val64, val32, L64, L32, dinv64, dinv32, idiag64, idiag32, params;
     DBuf ef64, eb64, ef32, eb32;  // factor values in the level ELL layouts
     Engine<double> er64;
@@ -1964,6 +2007,77 @@ static void setup_engine(tg_solver s, Engine<V64>& e64)
 // FP32 inner solves of the mixed path (unless the natural one is requested)
 static int ic_order(tg_solver s) { return (s->precision == TG_PREC_MIXED && s->inner_colour) ? 1 : 0; }
 
+// IC(0) in the mesh's ordering o, or the direct solver's complete factor, of
+// the matrix of the last reset
+template <class V64, class V32>
+static void factor_ic(tg_solver s)
+{
+    const MeshDev& m = s->mesh->d;
+    const V64* A = s->val64.as<V64>();
+    const bool direct = s->method == TG_SOLVER_DIRECT;
+    const bool mixed = s->precision == TG_PREC_MIXED && !direct;
+    // IC(0) in the mesh's ordering o, or the direct solver's complete
+    // factor: the same level-scheduled factorisation on either pattern
+    const int o = direct ? -1 : ic_order(s);
+    const ICDev& ic = direct ? s->dd : m.ic[o];
+    const ICHost& ch = direct ? *s->dh : s->mesh->h.ic[o];
+    V64* L = (V64*)s->L64.ensure((size_t)std::max(ic.nnzL, 1) * sizeof(V64));
+    V64* dinv = (V64*)s->dinv64.ensure((size_t)m.n * sizeof(V64));
+    std::vector<const void*> key = {A, L, dinv, s->mesh, (const void*)(size_t)(o + 1), (const void*)&ic};
+    s->graphs.run(s->stream, key, [&] {
+        const std::vector<int>& fp = ch.fwd_lev_ptr;
+        for (size_t l = 0; l + 1 < fp.size(); l++) {
+            int nr = fp[l + 1] - fp[l];
+            launch(ic_factor_level<V64>, cdiv_u((size_t)nr * 32, 256), 256, 0, s->stream, m, ic,
+                   ic.fwd_lev_rows + fp[l], nr, A, L, dinv);
+        }
+    });
+    V64* ef = (V64*)s->ef64.ensure((size_t)std::max(ic.nell_fwd, 1) * sizeof(V64));
+    V64* eb = (V64*)s->eb64.ensure((size_t)std::max(ic.nell_bwd, 1) * sizeof(V64));
+    launch(ell_gather_kernel<V64>, cdiv_u(std::max(ic.nell_fwd, 1), 256), 256, 0, s->stream, ic.nell_fwd,
+           ic.fwd_ell_src, L, ef);
+    launch(ell_gather_kernel<V64>, cdiv_u(std::max(ic.nell_bwd, 1), 256), 256, 0, s->stream, ic.nell_bwd,
+           ic.bwd_ell_src, L, eb);
+    if (mixed) {
+        launch(cast_kernel<V32, V64>, cdiv_u(std::max(ic.nell_fwd, 1), 256), 256, 0, s->stream,
+               (size_t)ic.nell_fwd, ef, (V32*)s->ef32.ensure((size_t)std::max(ic.nell_fwd, 1) * sizeof(V32)));
+        launch(cast_kernel<V32, V64>, cdiv_u(std::max(ic.nell_bwd, 1), 256), 256, 0, s->stream,
+               (size_t)ic.nell_bwd, eb, (V32*)s->eb32.ensure((size_t)std::max(ic.nell_bwd, 1) * sizeof(V32)));
+        launch(cast_kernel<V32, V64>, cdiv_u(std::max(ic.nnzL, 1), 256), 256, 0, s->stream, (size_t)ic.nnzL, L,
+               (V32*)s->L32.ensure((size_t)std::max(ic.nnzL, 1) * sizeof(V32)));
+        launch(cast_kernel<V32, V64>, cdiv_u(m.n, 256), 256, 0, s->stream, (size_t)m.n, dinv,
+               (V32*)s->dinv32.ensure(m.n * sizeof(V32)));
+    }
+    s->ic_done = true;
+}
+
+// the resident solve's matrices of the last reset: A in slices, G, and G^T
+template <class V32>
+static void build_resident(tg_solver s)
+{
+    const MeshDev& m = s->mesh->d;
+    const V32* A32 = s->val32.as<V32>();
+    V32* sa = (V32*)s->sa32.ensure((size_t)m.sa.len * sizeof(V32));
+    V32* sg = (V32*)s->sg32.ensure((size_t)m.sg.len * sizeof(V32));
+    V32* st = (V32*)s->st32.ensure((size_t)m.st.len * sizeof(V32));
+    launch(ell_gather_kernel<V32>, cdiv_u(m.sa.len, 256), 256, 0, s->stream, m.sa.len, m.sa.src, A32, sa);
+    launch(fsai_kernel_of<V32>(), cdiv_u(m.n, FSAI_WARPS), 32 * FSAI_WARPS, 0, s->stream, m.n, m.rowptr, m.colidx,
+           m.diagpos, A32, m.sg.ptr, m.sg.col, m.gcnt, sg);
+    launch(ell_gather_kernel<V32>, cdiv_u(m.st.len, 256), 256, 0, s->stream, m.st.len, m.st.src, sg, st);
+    s->res_ready = true;
+}
+
+// The default mixed path (ICH, colour ordering) of a CG request, or of a
+// BiCGSTAB request in its default mode, runs as one resident kernel
+// (tg_resident.cu); a mesh with a node of more than 31 neighbours before it in
+// the layout does not fit its preconditioner's row solver.
+static bool resident_ok(tg_solver s)
+{
+    return s->precision == TG_PREC_MIXED && s->precon == TG_PRECON_ICH && s->inner_colour &&
+           (s->method == TG_SOLVER_CG || (s->method == TG_SOLVER_BICGSTAB && s->reliable == 2)) &&
+           s->mesh->h.gmax <= FSAI_MAXM;
+}
+
 template <class V64, class V32>
 static void do_reset(tg_solver s, const double* cmua, const double* ckap, const double* c2a, double omega, int mem,
                      int elbasis = 0)
@@ -1990,40 +2104,10 @@ static void do_reset(tg_solver s, const double* cmua, const double* ckap, const 
     launch(diag_inv_kernel<V64>, cdiv_u(m.n, 256), 256, 0, s->stream, m.n, m.diagpos, A, idg);
     const bool direct = s->method == TG_SOLVER_DIRECT;
     const bool mixed = s->precision == TG_PREC_MIXED && !direct;
-    if (pre == TG_PRECON_ICH || direct) {
-        // IC(0) in the mesh's ordering o, or the direct solver's complete
-        // factor: the same level-scheduled factorisation on either pattern
-        const int o = direct ? -1 : ic_order(s);
-        const ICDev& ic = direct ? s->dd : m.ic[o];
-        const ICHost& ch = direct ? *s->dh : s->mesh->h.ic[o];
-        V64* L = (V64*)s->L64.ensure((size_t)std::max(ic.nnzL, 1) * sizeof(V64));
-        V64* dinv = (V64*)s->dinv64.ensure((size_t)m.n * sizeof(V64));
-        std::vector<const void*> key = {A, L, dinv, s->mesh, (const void*)(size_t)(o + 1), (const void*)&ic};
-        s->graphs.run(s->stream, key, [&] {
-            const std::vector<int>& fp = ch.fwd_lev_ptr;
-            for (size_t l = 0; l + 1 < fp.size(); l++) {
-                int nr = fp[l + 1] - fp[l];
-                launch(ic_factor_level<V64>, cdiv_u((size_t)nr * 32, 256), 256, 0, s->stream, m, ic,
-                       ic.fwd_lev_rows + fp[l], nr, A, L, dinv);
-            }
-        });
-        V64* ef = (V64*)s->ef64.ensure((size_t)std::max(ic.nell_fwd, 1) * sizeof(V64));
-        V64* eb = (V64*)s->eb64.ensure((size_t)std::max(ic.nell_bwd, 1) * sizeof(V64));
-        launch(ell_gather_kernel<V64>, cdiv_u(std::max(ic.nell_fwd, 1), 256), 256, 0, s->stream, ic.nell_fwd,
-               ic.fwd_ell_src, L, ef);
-        launch(ell_gather_kernel<V64>, cdiv_u(std::max(ic.nell_bwd, 1), 256), 256, 0, s->stream, ic.nell_bwd,
-               ic.bwd_ell_src, L, eb);
-        if (mixed) {
-            launch(cast_kernel<V32, V64>, cdiv_u(std::max(ic.nell_fwd, 1), 256), 256, 0, s->stream,
-                   (size_t)ic.nell_fwd, ef, (V32*)s->ef32.ensure((size_t)std::max(ic.nell_fwd, 1) * sizeof(V32)));
-            launch(cast_kernel<V32, V64>, cdiv_u(std::max(ic.nell_bwd, 1), 256), 256, 0, s->stream,
-                   (size_t)ic.nell_bwd, eb, (V32*)s->eb32.ensure((size_t)std::max(ic.nell_bwd, 1) * sizeof(V32)));
-            launch(cast_kernel<V32, V64>, cdiv_u(std::max(ic.nnzL, 1), 256), 256, 0, s->stream, (size_t)ic.nnzL, L,
-                   (V32*)s->L32.ensure((size_t)std::max(ic.nnzL, 1) * sizeof(V32)));
-            launch(cast_kernel<V32, V64>, cdiv_u(m.n, 256), 256, 0, s->stream, (size_t)m.n, dinv,
-                   (V32*)s->dinv32.ensure(m.n * sizeof(V32)));
-        }
-    }
+    s->ic_done = s->res_ready = false;
+    // (a resident solve's matrices, or the factor where its columns do not fit,
+    // follow at the solve)
+    if ((pre == TG_PRECON_ICH || direct) && !resident_ok(s)) factor_ic<V64, V32>(s);
     if (mixed) {
         launch(abs_values_kernel<V64>, cdiv_u(m.nnz, 256), 256, 0, s->stream, m.nnz, A,
                (float*)s->absA.ensure((size_t)m.nnz * sizeof(float)));
@@ -2220,7 +2304,12 @@ static void solve_reliable(tg_solver s, int k, const V64* B, V64* X, ColState* c
                     V64* Ac = (V64*)s->rel_ac.ensure(nkf * sizeof(V64));
                     // (float-float carries about 2^-46 of |A||x|: stopping tests finer
                     // than 1e-13 take the FP64 product)
-                    const bool ff = kf <= 256 && s->tol >= 1e-13 && (s->cw_tol == 0 || s->cw_tol >= 1e-13);
+                    // A column that has taken five updates stands at the rounding
+                    // floor near its source, where the float-float noise is more
+                    // than its far entries' test allows: an FP64 product then (such
+                    // columns stalled for a thousand iterations and ended without
+                    // reaching the bound)
+                    const bool ff = kf <= 256 && hc[1] == 0 && s->tol >= 1e-13 && (s->cw_tol == 0 || s->cw_tol >= 1e-13);
                     if (ff) {
                         residual_product_ff<V64>(s, k, kf, idx, X, Xc, Ac);
                     } else {
@@ -2253,6 +2342,144 @@ static void solve_reliable(tg_solver s, int k, const V64* B, V64* X, ColState* c
     launch(rel_finish_kernel, ek, 128, 0, s->stream, k, co, ci);
 }
 
+constexpr size_t CL_SMEM = 212 * 1024;
+
+// How k columns go to clusters: the lv columns of a cluster, its CTAs and
+// threads, by the estimated time of an iteration times the waves of clusters.
+// The estimate (clock cycles) is a fixed part of barriers and reductions, and
+// per round of a CTA's rows a latency and a shared-memory part; it was fitted
+// to sweeps of every shape on discs of 217 to 12.5k nodes and cylinders of
+// 4.6k and 30.8k nodes with 5 to 160 columns, where its choice is within 8 %
+// of the best one.  cs = 0: no shape fits the shared memory, or the columns
+// are so many that the batched kernels, which read the matrices once for all
+// of them, are faster: the crossing is at 20 MB of vector on the 30.8k-node
+// cylinder (80 complex columns: 21.0 against 21.5 ms; 20: 7.4 against 14.6;
+// 160: 42 against 31).
+template <class V64, class V32>
+static ClShape resident_shape(tg_solver s, int k)
+{
+    Mesh* mesh = s->mesh;
+    const int n = mesh->d.n;
+    ClShape best;
+    if ((size_t)n * k * sizeof(V32) > ((size_t)20 << 20)) return best;
+    const double f = std::max(1.0, (double)mesh->d.nnz / n / 7.0);  // matrix entries against a 2D mesh's
+    double tbest = 1e300;
+    for (int cs = 1; cs <= CL_MAXCS; cs *= 2) {
+        if (cs > 1 && n / cs < 150) break;
+        if (n / cs > 8000) continue;
+        const PartDev* part = mesh->part(cs);
+        if (!part) continue;
+        const PartDev& P = *part;
+        for (int lv = 1; lv * sizeof(V32) <= 16 && (lv == 1 || lv < 2 * k); lv *= 2) {
+            ClShape c;
+            c.lv = lv;
+            c.cs = cs;
+            c.part = part;
+            // shared memory: vectors, halo copies, slice pointers, and the matrices where they fit
+            const size_t mh = ((size_t)(3 * P.slots + P.own) * lv * sizeof(V32) + 15) / 16 * 16;
+            const size_t mp = mh + (size_t)P.npush * 8, mv = (mp + (size_t)3 * (P.nsl + 1) * 4 + 15) / 16 * 16;
+            const size_t mc = mv + (size_t)P.len * sizeof(V32), end = mc + (size_t)P.len * 2;
+            c.mofs_push = (int)mh;
+            c.mofs_ptr = (int)mp;
+            c.mofs_val = (int)mv;
+            c.mofs_col = (int)mc;
+            c.msm = end <= CL_SMEM;
+            c.sm = c.msm ? end : mv;
+            if (c.sm > CL_SMEM) continue;
+            // as many threads as spread the rows evenly over the rounds
+            const int rounds = (P.own + CL_NT - 1) / CL_NT;
+            c.nt = std::max(64, (P.own + rounds * 32 - 1) / (rounds * 32) * 32);
+            auto kern = resident_kernel<V64, V32>(lv);
+            allow_smem((const void*)kern);
+            int at_once = 0;
+            if (cs > 1) {
+                cudaLaunchConfig_t cfg = {};
+                cudaLaunchAttribute at[1];
+                cluster_config(cfg, at, (k + lv - 1) / lv, cs, c.nt, c.sm, s->stream);
+                if (cs > 8) TG_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+                if (cudaOccupancyMaxActiveClusters(&at_once, (const void*)kern, &cfg) != cudaSuccess) {
+                    cudaGetLastError();
+                    continue;
+                }
+            } else {
+                int nsm = 0;
+                TG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&at_once, kern, c.nt, c.sm));
+                TG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, mesh->device));
+                at_once *= nsm;
+            }
+            if (at_once < 1) continue;
+            const int waves = ((k + lv - 1) / lv + at_once - 1) / at_once;
+            const double fix = 9e3 + (cs > 1 ? 800.0 * std::log2((double)cs) * std::log2((double)cs) : 0.0);
+            const double word = lv * sizeof(V32) == 4 ? 0.8 : lv * sizeof(V32) == 8 ? 1.0 : 1.5;
+            const double round = (c.msm ? 1.4e3 : 2.5e3) + 3.2e3 * c.nt / CL_NT * word;
+            const double t = waves * (fix + rounds * round * f);
+            if (t < tbest) { tbest = t; best = c; }
+        }
+    }
+    return best;
+}
+
+// Columns that ended without reaching their bounds for another reason than
+// the iteration limit
+static __global__ void resident_failed_kernel(int k, const ColState* __restrict__ co, int* __restrict__ out)
+{
+    __shared__ int f;
+    if (threadIdx.x == 0) f = 0;
+    __syncthreads();
+    for (int c = threadIdx.x; c < k; c += blockDim.x)
+        if (co[c].status != 0 && co[c].its < co[c].maxit) atomicOr(&f, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) *out = f;
+}
+
+// the shape for k columns, chosen at their first solve
+template <class V64, class V32>
+static const ClShape& shape_of(tg_solver s, int k)
+{
+    auto it = s->shapes.find(k);
+    if (it == s->shapes.end()) {
+        if (s->shapes.size() >= 64) s->shapes.clear();
+        it = s->shapes.emplace(k, resident_shape<V64, V32>(s, k)).first;
+    }
+    return it->second;
+}
+
+// The resident solve of k columns (R: the residual of a nonzero guess);
+// false: some column failed, X is to be restored and solved otherwise
+template <class V64, class V32>
+static bool solve_resident(tg_solver s, int k, const V64* B, V64* X, ColState* co, V64* R, int maxit, bool zero_guess)
+{
+    const MeshDev& m = s->mesh->d;
+    const ClShape& sh = shape_of<V64, V32>(s, k);
+    const unsigned ng = cdiv_u(k, sh.lv);
+    ResArgs<V64, V32> a;
+    a.n = m.n; a.k = k; a.cs = sh.cs; a.slots = sh.part->slots; a.own = sh.part->own;
+    a.msm = sh.msm; a.mofs_val = sh.mofs_val; a.mofs_col = sh.mofs_col; a.mofs_ptr = sh.mofs_ptr;
+    a.A = {m.sa.ptr, sh.part->ca, s->sa32.as<V32>()};
+    a.G = {m.sg.ptr, sh.part->cg, s->sg32.as<V32>()};
+    a.T = {m.st.ptr, sh.part->ct, s->st32.as<V32>()};
+    a.pofs = sh.part->pofs; a.push = sh.part->push; a.mofs_push = sh.mofs_push;
+    a.x = (V32*)s->X32.ensure((size_t)ng * m.n * sh.lv * sizeof(V32));
+    a.X = X; a.R = R; a.B = B;
+    a.Xff = s->xff.ensure((size_t)m.n * k * sizeof(V64));
+    a.rowptr = m.rowptr; a.colidx = m.colidx;
+    a.A64 = s->val64.as<V64>(); a.Aff = s->valff.p; a.absA = s->absA.as<float>();
+    a.co = co;
+    a.trig = (float)s->inner_tol; a.cwtol = s->cw_tol; a.maxit = maxit; a.max_upd = 4 * std::max(1, s->max_outer);
+    a.zero_guess = zero_guess ? 1 : 0;
+    // float-float residuals carry about 2^-46 of |A||x|: finer tests than 1e-13 take FP64 ones
+    a.all64 = !(s->tol >= 1e-13 && (s->cw_tol == 0 || s->cw_tol >= 1e-13));
+    {
+        ProfScope ps(&s->prof, PC_VEC, s->stream);
+        launch_cluster(resident_kernel<V64, V32>(sh.lv), ng, sh.cs, sh.nt, sh.sm, s->stream, a);
+    }
+    int* df = (int*)s->rel_cnt.ensure(4 * sizeof(int));
+    launch(resident_failed_kernel, 1, 256, 0, s->stream, k, (const ColState*)co, df);
+    int failed = 0;
+    s->bnc.fetch(&failed, df, sizeof(int), s->stream);
+    return failed == 0;
+}
+
 template <class V64, class V32>
 static void solve_nm_body(tg_solver s, int k, const V64* B, V64* X, ColState* co, bool zero_guess);
 
@@ -2282,6 +2509,26 @@ static void solve_nm_body(tg_solver s, int k, const V64* B, V64* X, ColState* co
     if (s->precision == TG_PREC_FP64) {
         e64.solve(s->method, k, B, X, co, zero_guess);
         return;
+    }
+    if (resident_ok(s) && shape_of<V64, V32>(s, k).cs) {
+        if (!s->res_ready) build_resident<V32>(s);
+        V64* R = (V64*)s->tmp.ensure(nk * sizeof(V64));
+        if (!zero_guess) {
+            TG_CUDA(cudaMemcpyAsync(s->xkeep.ensure(nk * sizeof(V64)), X, nk * sizeof(V64), cudaMemcpyDeviceToDevice,
+                                    s->stream));
+            e64.spmm(k, X, R, nullptr, false, nullptr, nullptr, 0);
+            launch(resid_kernel<V64>, cdiv_u(nk, 256), 256, 0, s->stream, n, k, k, B, R, nullptr);
+        }
+        if (solve_resident<V64, V32>(s, k, B, X, co, R, maxit, zero_guess)) return;
+        // a breakdown, or a process that does not converge: the path below
+        // from the same start
+        if (zero_guess) TG_CUDA(cudaMemsetAsync(X, 0, nk * sizeof(V64), s->stream));
+        else TG_CUDA(cudaMemcpyAsync(X, s->xkeep.p, nk * sizeof(V64), cudaMemcpyDeviceToDevice, s->stream));
+        launch(init_cols_kernel, cdiv_u(k, 128), 128, 0, s->stream, k, co, s->tol, maxit);
+    }
+    if (s->precon == TG_PRECON_ICH && !s->ic_done) {
+        factor_ic<V64, V32>(s);
+        setup_engine(s, e64);
     }
     // FP64 iterative refinement around FP32 / complex-FP32 inner solves:
     // r = b - F x in FP64, solve F e = r in FP32 to a loose tolerance,
