@@ -57,8 +57,8 @@ extern "C" {
 #define TG_SOLVER_BICGSTAB 1
 #define TG_SOLVER_GMRES 2
 /* LSOLVER_DIRECT (fwdsolver.cc:89-123, 467-505: Cholesky for real systems,
-   SuperLU for complex ones): a complete F = L L^T factorisation in FP64 at
-   each reset (complex systems: complex-symmetric L L^T), in a nested-dissection
+   SuperLU for complex ones): a complete F = L D L^T factorisation in FP64
+   at each reset (complex systems: complex symmetric), in a nested-dissection
    ordering of the nodes; each solve is the two triangular sweeps.  The
    preconditioner and precision settings do not apply.  Per right-hand side
    the result reports 0 iterations and the true relative residual.  A mesh

@@ -213,10 +213,8 @@ __global__ void ic_factor_level(MeshDev m, ICDev ic, const int* __restrict__ row
             else if (ca > cb) b++;
             else { s = vfma(s, L[a], L[b]); a++; b++; }
         }
-        // a_ji = a_ij (symmetric pattern and values); a fill entry of a
-        // complete factor has no entry in A (Lapos -1)
-        const int ap = ic.Lapos[ic.Umap[u]];
-        V aij = ap >= 0 ? A[ap] : vzero<V>();
+        // a_ji = a_ij (symmetric pattern and values)
+        V aij = A[ic.Lapos[ic.Umap[u]]];
         L[ic.Umap[u]] = vdiv(vsub(aij, s), di);
     }
     if (lane == 0) dinv[i] = vrecip(di);

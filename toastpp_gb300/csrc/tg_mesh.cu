@@ -419,16 +419,17 @@ static void ic_finish(const MeshHost& m, ICHost& c)
 }
 
 // ---------------------------------------------------------------------------
-// Complete factor for the direct solver (LSOLVER_DIRECT): a fill-reducing
-// nested-dissection ordering and the symbolic Cholesky pattern, in the same
-// ICHost form as the IC(0) patterns so the same factor and sweep kernels run
-// on it (IC on a pattern closed under fill is the exact factorisation).
+// Fronts of the direct solver (LSOLVER_DIRECT): the tree of a nested-dissection
+// ordering, a front per leaf block and separator (tg_direct.cuh).
 // ---------------------------------------------------------------------------
 namespace {
 struct NDState {
     const MeshHost* m;
     std::vector<int> mark, sep;
     int stamp = 0;
+    // tree nodes in postorder: columns [c0, c1) of the ordering, children
+    struct Node { int c0, c1; std::vector<int> kids; };
+    std::vector<Node> nodes;
     double coord(int p, int d) const { return m->coords[(size_t)m->iperm[p] * m->dim + d]; }
 };
 
@@ -436,14 +437,18 @@ struct NDState {
 // then the separator (upper-half nodes adjacent to the lower half); the
 // halves split at the median of the longest extent; sets of at most 32
 // nodes keep their layout (spatial) order
-void nd_order(NDState& S, std::vector<int>& idx, int lo, int hi, std::vector<int>& out)
+// returns the subtree's node, -1 when it has no columns
+int nd_order(NDState& S, std::vector<int>& idx, int lo, int hi, std::vector<int>& out)
 {
     const MeshHost& m = *S.m;
     const int cnt = hi - lo;
+    if (cnt == 0) return -1;
     if (cnt <= 32) {
         std::sort(idx.begin() + lo, idx.begin() + hi);
+        const int c0 = (int)out.size();
         out.insert(out.end(), idx.begin() + lo, idx.begin() + hi);
-        return;
+        S.nodes.push_back({c0, (int)out.size(), {}});
+        return (int)S.nodes.size() - 1;
     }
     double ext = -1.0;
     int ax = 0;
@@ -474,77 +479,108 @@ void nd_order(NDState& S, std::vector<int>& idx, int lo, int hi, std::vector<int
     }
     std::vector<int> sep(S.sep.begin() + s0, S.sep.end());
     S.sep.resize(s0);
-    nd_order(S, idx, lo, mid, out);
-    nd_order(S, idx, mid, w, out);
+    std::vector<int> kids;
+    for (int t : {nd_order(S, idx, lo, mid, out), nd_order(S, idx, mid, w, out)})
+        if (t >= 0) kids.push_back(t);
     std::sort(sep.begin(), sep.end());
+    const int c0 = (int)out.size();
     out.insert(out.end(), sep.begin(), sep.end());
+    S.nodes.push_back({c0, (int)out.size(), kids});
+    return (int)S.nodes.size() - 1;
 }
 }  // namespace
 
-void direct_pattern(const MeshHost& m, ICHost& c, long long max_nnz)
+void direct_pattern(const MeshHost& m, DirectHost& c, long long max_nnz)
 {
     const int n = m.n;
     NDState S;
     S.m = &m;
     S.mark.assign(n, 0);
-    std::vector<int> idx(n), order;
+    std::vector<int> idx(n), order, rank(n);
     for (int p = 0; p < n; p++) idx[p] = p;
     order.reserve(n);
     nd_order(S, idx, 0, n, order);
-    c.key.assign(n, 0);
-    for (int r = 0; r < n; r++) c.key[order[r]] = r;
-    // symbolic factorisation in rank space: column j holds the ranks i > j of
-    // its neighbours and of its elimination-tree children's columns
-    std::vector<std::vector<int>> col(n);
-    std::vector<std::vector<int>> kids(n);
-    std::vector<int> seen(n, -1);
-    long long total = 0;
-    for (int j = 0; j < n; j++) {
-        const int p = order[j];
-        std::vector<int>& cj = col[j];
-        seen[j] = j;
-        for (int e = m.lrowptr[p]; e < m.lrowptr[p + 1]; e++) {
-            const int i = c.key[m.lcolidx[e]];
-            if (i > j && seen[i] != j) { seen[i] = j; cj.push_back(i); }
-        }
-        for (int ch : kids[j]) {
-            for (int i : col[ch])
+    for (int r = 0; r < n; r++) rank[order[r]] = r;
+    // the sparse factor's entries, column by column (column j: the ranks i > j
+    // of its neighbours and of its elimination-tree children's columns)
+    {
+        std::vector<std::vector<int>> col(n), kids(n);
+        std::vector<int> seen(n, -1);
+        long long total = 0;
+        for (int j = 0; j < n; j++) {
+            const int p = order[j];
+            std::vector<int>& cj = col[j];
+            seen[j] = j;
+            for (int e = m.lrowptr[p]; e < m.lrowptr[p + 1]; e++) {
+                const int i = rank[m.lcolidx[e]];
                 if (i > j && seen[i] != j) { seen[i] = j; cj.push_back(i); }
+            }
+            for (int ch : kids[j]) {
+                for (int i : col[ch])
+                    if (i > j && seen[i] != j) { seen[i] = j; cj.push_back(i); }
+                std::vector<int>().swap(col[ch]);
+            }
+            if (!cj.empty()) kids[*std::min_element(cj.begin(), cj.end())].push_back(j);
+            total += (long long)cj.size();
+            TG_CHECK(total <= max_nnz, TG_ERR_UNSUPPORTED, "direct solver: the factor's fill exceeds its limit");
         }
-        std::sort(cj.begin(), cj.end());
-        if (!cj.empty()) kids[cj[0]].push_back(j);
-        total += (long long)cj.size();
-        TG_CHECK(total <= max_nnz, TG_ERR_UNSUPPORTED, "direct solver: the factor's fill exceeds its limit");
     }
-    // rows of L by layout row, entries in ascending rank (the transpose of
-    // the columns, which come in ascending rank)
-    std::vector<int> rcnt(n + 1, 0);
-    for (int j = 0; j < n; j++)
-        for (int i : col[j]) rcnt[order[i] + 1]++;
-    c.Lrowptr.assign(n + 1, 0);
-    for (int p = 0; p < n; p++) c.Lrowptr[p + 1] = c.Lrowptr[p] + rcnt[p + 1];
-    const size_t nl = (size_t)c.Lrowptr[n];
-    c.Lcolidx.assign(nl, 0);
-    c.Lkey.assign(nl, 0);
-    c.Lapos.assign(nl, -1);
-    std::vector<int> fill(c.Lrowptr.begin(), c.Lrowptr.end() - 1);
-    for (int j = 0; j < n; j++) {
-        for (int i : col[j]) {
-            const int pr = order[i];
-            const int q = fill[pr]++;
-            c.Lcolidx[q] = order[j];
-            c.Lkey[q] = j;
+    // fronts in postorder: the rows of a front are the later ranks that its
+    // columns or its children's rows reach
+    const int nf = (int)S.nodes.size();
+    c = DirectHost();
+    c.fronts.resize(nf);
+    std::vector<std::vector<int>> border(nf);
+    std::vector<int> seen(n, -1), place(n, -1), height(nf, 0);
+    for (int t = 0; t < nf; t++) {
+        const NDState::Node& d = S.nodes[t];
+        DFront& f = c.fronts[t];
+        f.c0 = d.c0;
+        f.nc = d.c1 - d.c0;
+        std::vector<int>& br = border[t];
+        for (int j = d.c0; j < d.c1; j++)
+            for (int e = m.lrowptr[order[j]]; e < m.lrowptr[order[j] + 1]; e++) {
+                const int i = rank[m.lcolidx[e]];
+                if (i >= d.c1 && seen[i] != t) { seen[i] = t; br.push_back(i); }
+            }
+        for (int q : d.kids) {
+            height[t] = std::max(height[t], height[q] + 1);
+            for (int i : border[q])
+                if (i >= d.c1 && seen[i] != t) { seen[i] = t; br.push_back(i); }
         }
-        std::vector<int>().swap(col[j]);
+        std::sort(br.begin(), br.end());
+        f.nr = (int)br.size();
+        f.off = c.nval;
+        c.nval += (long long)(f.nc + f.nr) * (f.nc + f.nr);
+        f.w0 = (int)c.rows.size();
+        for (int j = d.c0; j < d.c1; j++) { place[j] = j - d.c0; c.rows.push_back(order[j]); }
+        for (int i = 0; i < f.nr; i++) { place[br[i]] = f.nc + i; c.rows.push_back(order[br[i]]); }
+        f.a0 = (int)c.entries.size();
+        for (int j = d.c0; j < d.c1; j++)
+            for (int e = m.lrowptr[order[j]]; e < m.lrowptr[order[j] + 1]; e++) {
+                const int i = rank[m.lcolidx[e]];
+                if (i >= j) c.entries.push_back({place[i], j - d.c0, e});
+            }
+        f.na = (int)c.entries.size() - f.a0;
+        f.kid0 = (int)c.kids.size();
+        f.nkid = (int)d.kids.size();
+        for (int q : d.kids) {
+            c.kids.push_back(q);
+            DFront& k = c.fronts[q];
+            k.rel0 = (int)c.rel.size();
+            for (int i : border[q]) c.rel.push_back(place[i]);
+            std::vector<int>().swap(border[q]);
+        }
+        f.rel0 = 0;
     }
-    // Lapos: the entry of A at (row, column), or -1 for a fill entry
-    std::vector<int> where(n, -1);
-    for (int p = 0; p < n; p++) {
-        for (int e = m.lrowptr[p]; e < m.lrowptr[p + 1]; e++) where[m.lcolidx[e]] = e;
-        for (int q = c.Lrowptr[p]; q < c.Lrowptr[p + 1]; q++) c.Lapos[q] = where[c.Lcolidx[q]];
-        for (int e = m.lrowptr[p]; e < m.lrowptr[p + 1]; e++) where[m.lcolidx[e]] = -1;
-    }
-    ic_finish(m, c);
+    int nl = 0;
+    for (int h : height) nl = std::max(nl, h + 1);
+    c.level.assign(nl + 1, 0);
+    for (int h : height) c.level[h + 1]++;
+    for (int l = 0; l < nl; l++) c.level[l + 1] += c.level[l];
+    c.ids.assign(nf, 0);
+    std::vector<int> fill(c.level.begin(), c.level.end() - 1);
+    for (int t = 0; t < nf; t++) c.ids[fill[height[t]]++] = t;
 }
 
 // greedy colouring in natural order; key = colour-major rank (colour, natural index)

@@ -32,6 +32,29 @@ struct ICHost {
     std::vector<int> bwd_ell_w, bwd_ell_off, bwd_ell_col, bwd_ell_src;
 };
 
+// A dense front of the direct solver: its columns are the ranks c0 .. c0 + nc - 1
+// of the elimination ordering, followed by nr rows of its ancestors.
+struct DFront {
+    int c0, nc, nr;
+    int kid0, nkid;          // children (fronts), in kids
+    int a0, na;              // entries of A, in entries
+    int rel0;                // its nr rows' places in the parent front, in rel
+    int w0;                  // its nc + nr layout rows, in rows; also its place in the solve's workspace
+    long long off;           // its (nc + nr)^2 values
+};
+struct DEntry {
+    int i, j, src;           // place in the front, entry of the layout CSR
+};
+
+struct DirectHost {
+    std::vector<DFront> fronts;
+    std::vector<int> kids, rel, rows;
+    std::vector<DEntry> entries;
+    // fronts by height in the tree (leaves first): level l is ids[level[l]] ..
+    std::vector<int> level, ids;
+    long long nval = 0;
+};
+
 struct ICDev {
     int nnzL, nlev_fwd, nlev_bwd, nell_fwd, nell_bwd;
     int *key, *Lrowptr, *Lcolidx, *Lapos, *Lkey, *Ucolptr, *Urow, *Umap;
@@ -140,12 +163,10 @@ struct Mesh {
 };
 
 Mesh* mesh_build(int dim, int n, const double* coords, int ne, const int* el);
-// The complete Cholesky pattern of F for the direct solver: a nested-
-// dissection ordering of the nodes by their coordinates and the symbolic
-// factor (fill included, Lapos -1 where A has no entry), with the column
-// view, levels and ELL layouts of ICHost.  Throws TG_ERR_UNSUPPORTED past
-// max_nnz factor entries.
-void direct_pattern(const MeshHost& m, ICHost& c, long long max_nnz);
+// The fronts of a complete factor of F for the direct solver, from a nested
+// dissection of the nodes by their coordinates.  Throws TG_ERR_UNSUPPORTED past
+// max_nnz entries of the sparse factor (fill included).
+void direct_pattern(const MeshHost& m, DirectHost& c, long long max_nnz);
 void qvec_gaussian_host(const MeshHost& m, const double* cnt, double w, bool neumann, double* q);
 // Element_Unstructured::GContains for element e (padded bounding box, then
 // the padded local test)

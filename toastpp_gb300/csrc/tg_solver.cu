@@ -17,6 +17,7 @@
 #include "../../include/toastgpu.h"
 #include "tg_jac.cuh"
 #include "tg_cluster.cuh"
+#include "tg_direct.cuh"
 #include "tg_gmres.cuh"
 #include "tg_grid.cuh"
 
@@ -335,12 +336,8 @@ struct Engine {
     const V* Lef = nullptr;    // factor values in the forward / backward level ELL layouts
     const V* Leb = nullptr;
     int ico = 0;               // IC ordering: 0 natural, 1 colour-major
-    // a factor pattern of the solver's own (the direct solver's complete
-    // factor) in place of the mesh's IC(0) pattern ico, when set
-    const ICHost* ich = nullptr;
-    const ICDev* icd = nullptr;
-    const ICHost& ic_host() const { return ich ? *ich : mesh->h.ic[ico]; }
-    const ICDev& ic_dev() const { return icd ? *icd : mesh->d.ic[ico]; }
+    const ICHost& ic_host() const { return mesh->h.ic[ico]; }
+    const ICDev& ic_dev() const { return mesh->d.ic[ico]; }
     int precon = 0;            // 0 none, 1 diag, 2 ich
     Profiler* prof = nullptr;
     DBuf w[9], part, cs, cnt, gbasis, gcol;
@@ -544,7 +541,7 @@ struct Engine {
     {
         const char* e = getenv("TOASTGPU_IC_PERSISTENT");
         if (e && (e[0] == '0' || e[0] == '1')) return e[0] == '1';
-        const auto key = std::make_tuple(mesh->uid * 4 + (icd ? 2 : ico), (int)sizeof(V) * 2 + (int)vt<V>::cplx, k);
+        const auto key = std::make_tuple(mesh->uid * 4 + ico, (int)sizeof(V) * 2 + (int)vt<V>::cplx, k);
         {
             std::lock_guard<std::mutex> g(g_tune_mu);
             auto it = g_ictune.find(key);
@@ -653,7 +650,7 @@ struct Engine {
         const ICDev& ic = ic_dev();
         int cw = colw(k), ncg = (k + cw - 1) / cw, rpw = 32 / cw;
         std::vector<const void*> key = {(const void*)(size_t)k, in, out, cst, L, dinv, Lef, Leb, mesh,
-                                        (const void*)(size_t)ico, (const void*)icd, (const void*)(size_t)persistent};
+                                        (const void*)(size_t)ico, (const void*)(size_t)persistent};
         const bool wide = k >= 32 && k <= 256;
         if (persistent) {
             if (!sweep.p) {
@@ -730,17 +727,17 @@ struct Engine {
         else throw Error{TG_ERR_UNSUPPORTED, "solver method not implemented on the GPU"};
     }
 
-    // LSOLVER_DIRECT: X = F^-1 B by the two sweeps of the complete factor
-    // (CholeskySolve, crmatrix_imp.hpp:2297-2306), then the true residual
-    // b - A x for the per-column result (0 iterations, status 0)
-    void direct_solve(int k, const V* B, V* X, ColState* cst)
+    // LSOLVER_DIRECT: X = F^-1 B by sweeps(), then the true residual b - A x for
+    // the per-column result (0 iterations, status 0)
+    template <class SW>
+    void direct_solve(int k, const V* B, V* X, ColState* cst, SW sweeps)
     {
         const MeshDev& m = mesh->d;
         const size_t nk = (size_t)m.n * k;
         double* pt = parts(k, 1);
         launch(dot_tiles_kernel<V>, ntiles(), rowblk(k), 0, st, m.n, k, k, B, B, nullptr, nullptr, pt, 1, ntiles(), nullptr);
         finalize<1>(k, cst, PH_BNORM);
-        ic_apply(k, B, X, nullptr);
+        sweeps();
         V* R = vec(0, nk);
         spmm(k, X, R, nullptr, false, nullptr, nullptr, 0);
         launch(resid_kernel<V>, cdiv_u(nk, 256), 256, 0, st, m.n, k, k, B, R, nullptr);
@@ -1908,10 +1905,9 @@ struct tg_solver_s {
     DBuf absA, berr_max;              // |entries| of F in FP32, per-column backward-error maxima
     DBuf valff;                       // F as float-float (the mixed path's residual products)
     DBuf results;                     // per-column results, compact, for the final read
-    // direct solver: the complete factor's pattern (host and device)
-    std::unique_ptr<ICHost> dh;
-    ICDev dd{};
-    DBuf dbuf[20];
+    // direct solver: its fronts (host and device), and the solves' workspace
+    std::unique_ptr<DirectHost> dh;
+    DBuf dfr, dkids, drel, drows, dent, dids, dw, dblk;
     Bounce bnc;                       // small device-to-host reads
     int jw_D = 0, jw_ready = 0;       // slots per node; bit 0 FP64 weights built, bit 1 FP32, bit 2 float-float
     Profiler prof;
@@ -1933,31 +1929,88 @@ static int fail(const Error& e)
     return e.code;
 }
 
-// the direct solver's factor pattern, built on the host once per solver and
-// uploaded (TG_SOLVER_DIRECT)
+// the direct solver's fronts, built on the host once per solver and uploaded
+// (TG_SOLVER_DIRECT)
 static void direct_setup(tg_solver s)
 {
-    s->dh = std::make_unique<ICHost>();
-    ICHost& c = *s->dh;
+    s->dh = std::make_unique<DirectHost>();
+    DirectHost& c = *s->dh;
     direct_pattern(s->mesh->h, c, 1LL << 28);
-    ICDev& g = s->dd;
-    const int n = s->mesh->h.n;
-    g.nnzL = c.Lrowptr[n];
-    g.nlev_fwd = (int)c.fwd_lev_ptr.size() - 1;
-    g.nlev_bwd = (int)c.bwd_lev_ptr.size() - 1;
-    g.nell_fwd = (int)c.fwd_ell_col.size();
-    g.nell_bwd = (int)c.bwd_ell_col.size();
-    int** dst[20] = {&g.key, &g.Lrowptr, &g.Lcolidx, &g.Lapos, &g.Lkey, &g.Ucolptr, &g.Urow, &g.Umap,
-                     &g.fwd_lev_rows, &g.bwd_lev_rows, &g.fwd_ell_col, &g.fwd_ell_src, &g.bwd_ell_col, &g.bwd_ell_src,
-                     &g.fwd_lev_ptr, &g.bwd_lev_ptr, &g.fwd_ell_w, &g.bwd_ell_w, &g.fwd_ell_off, &g.bwd_ell_off};
-    const std::vector<int>* src[20] = {&c.key, &c.Lrowptr, &c.Lcolidx, &c.Lapos, &c.Lkey, &c.Ucolptr, &c.Urow, &c.Umap,
-                                       &c.fwd_lev_rows, &c.bwd_lev_rows, &c.fwd_ell_col, &c.fwd_ell_src,
-                                       &c.bwd_ell_col, &c.bwd_ell_src, &c.fwd_lev_ptr, &c.bwd_lev_ptr, &c.fwd_ell_w,
-                                       &c.bwd_ell_w, &c.fwd_ell_off, &c.bwd_ell_off};
-    for (int t = 0; t < 20; t++) {
-        upload_sync(s->dbuf[t], *src[t]);
-        *dst[t] = s->dbuf[t].as<int>();
-    }
+    upload_sync(s->dfr, c.fronts);
+    upload_sync(s->dkids, c.kids);
+    upload_sync(s->drel, c.rel);
+    upload_sync(s->drows, c.rows);
+    upload_sync(s->dent, c.entries);
+    upload_sync(s->dids, c.ids);
+}
+
+// L D L^T of the matrix of the last reset, level by level of the fronts' tree
+template <class V>
+static void direct_factor(tg_solver s)
+{
+    const DirectHost& c = *s->dh;
+    const V* A = s->val64.as<V>();
+    V* F = (V*)s->L64.ensure((size_t)std::max(c.nval, 1LL) * sizeof(V));
+    V* dinv = (V*)s->dinv64.ensure((size_t)s->mesh->d.n * sizeof(V));
+    V* blk = (V*)s->dblk.ensure((size_t)s->mesh->d.n * DP * sizeof(V));
+    const DFront* fr = s->dfr.as<DFront>();
+    s->graphs.run(s->stream, {A, F, dinv, blk}, [&] {
+        for (size_t l = 0; l + 1 < c.level.size(); l++) {
+            const int* ids = s->dids.as<int>() + c.level[l];
+            const unsigned nf = (unsigned)(c.level[l + 1] - c.level[l]);
+            int fm = 0, ncm = 0;
+            for (int t = c.level[l]; t < c.level[l + 1]; t++) {
+                const DFront& d = c.fronts[c.ids[t]];
+                fm = std::max(fm, d.nc + d.nr);
+                ncm = std::max(ncm, d.nc);
+            }
+            // parts of a front: enough CTAs for the chip, not more than its columns give work
+            const unsigned parts = std::max(1u, std::min((unsigned)(fm + 7) / 8, 304u / std::max(1u, nf)));
+            launch(direct_assemble_kernel<V>, dim3(nf, parts), 256, 0, s->stream, fr, ids, s->dkids.as<int>(),
+                   s->drel.as<int>(), s->dent.as<DEntry>(), A, F);
+            for (int p0 = 0; p0 < ncm; p0 += DP) {
+                // rows below the shortest panel that starts at p0
+                int below = 0;
+                for (int t = c.level[l]; t < c.level[l + 1]; t++) {
+                    const DFront& d = c.fronts[c.ids[t]];
+                    if (p0 < d.nc) below = std::max(below, d.nc + d.nr - p0 - std::min(DP, d.nc - p0));
+                }
+                launch(direct_panel_kernel<V>, dim3(nf, std::max(1u, cdiv_u(below, DTR))), 128, 0, s->stream, fr, ids,
+                       p0, F, blk, dinv);
+                const unsigned nt = cdiv_u(below, DP);
+                for (unsigned t0 = 0, all = nt * (nt + 1) / 2; t0 < all; t0 += 65535)
+                    launch(direct_update_kernel<V>, dim3(nf, std::min(65535u, all - t0)), DP * DP, 0, s->stream, fr,
+                           ids, p0, (int)t0, (const V*)blk, F);
+            }
+        }
+    });
+}
+
+// X = F^-1 B (node-major, k columns): forward level by level, then backward
+template <class V>
+static void direct_sweeps(tg_solver s, int k, const V* B, V* X)
+{
+    const DirectHost& c = *s->dh;
+    const V* F = s->L64.as<V>();
+    const V* dinv = s->dinv64.as<V>();
+    const V* blk = s->dblk.as<V>();
+    V* W = (V*)s->dw.ensure(c.rows.size() * (size_t)k * sizeof(V));
+    const DFront* fr = s->dfr.as<DFront>();
+    ProfScope ps(&s->prof, PC_SWEEP, s->stream);
+    s->graphs.run(s->stream, {(const void*)(size_t)k, B, X, W, F, dinv, blk}, [&] {
+        const int nl = (int)c.level.size() - 1;
+        for (int h = 0; h < 2 * nl; h++) {
+            const int l = h < nl ? h : 2 * nl - 1 - h;
+            const int* ids = s->dids.as<int>() + c.level[l];
+            const dim3 g((unsigned)(c.level[l + 1] - c.level[l]), cdiv_u(k, DKC));
+            if (h < nl)
+                launch(direct_fwd_kernel<V>, g, 256, 0, s->stream, fr, ids, s->dkids.as<int>(), s->drel.as<int>(),
+                       s->drows.as<int>(), F, blk, k, B, X, W);
+            else
+                launch(direct_bwd_kernel<V>, g, 256, 0, s->stream, fr, ids, s->drows.as<int>(), F, blk, dinv, k, X,
+                       W);
+        }
+    });
 }
 
 #define API_BEGIN try {
@@ -1993,13 +2046,6 @@ static void setup_engine(tg_solver s, Engine<V64>& e64)
     e64.Leb = s->eb64.as<V64>();
     e64.prof = &s->prof;
     e64.ico = 0;
-    e64.ich = nullptr;
-    e64.icd = nullptr;
-    if (s->method == TG_SOLVER_DIRECT) {  // the complete factor as the "preconditioner"
-        e64.precon = TG_PRECON_ICH;
-        e64.ich = s->dh.get();
-        e64.icd = &s->dd;
-    }
 }
 
 // IC ordering the solver's preconditioner is factored in: the natural
@@ -2007,20 +2053,16 @@ static void setup_engine(tg_solver s, Engine<V64>& e64)
 // FP32 inner solves of the mixed path (unless the natural one is requested)
 static int ic_order(tg_solver s) { return (s->precision == TG_PREC_MIXED && s->inner_colour) ? 1 : 0; }
 
-// IC(0) in the mesh's ordering o, or the direct solver's complete factor, of
-// the matrix of the last reset
+// IC(0) in the mesh's ordering o of the matrix of the last reset
 template <class V64, class V32>
 static void factor_ic(tg_solver s)
 {
     const MeshDev& m = s->mesh->d;
     const V64* A = s->val64.as<V64>();
-    const bool direct = s->method == TG_SOLVER_DIRECT;
-    const bool mixed = s->precision == TG_PREC_MIXED && !direct;
-    // IC(0) in the mesh's ordering o, or the direct solver's complete
-    // factor: the same level-scheduled factorisation on either pattern
-    const int o = direct ? -1 : ic_order(s);
-    const ICDev& ic = direct ? s->dd : m.ic[o];
-    const ICHost& ch = direct ? *s->dh : s->mesh->h.ic[o];
+    const bool mixed = s->precision == TG_PREC_MIXED;
+    const int o = ic_order(s);
+    const ICDev& ic = m.ic[o];
+    const ICHost& ch = s->mesh->h.ic[o];
     V64* L = (V64*)s->L64.ensure((size_t)std::max(ic.nnzL, 1) * sizeof(V64));
     V64* dinv = (V64*)s->dinv64.ensure((size_t)m.n * sizeof(V64));
     std::vector<const void*> key = {A, L, dinv, s->mesh, (const void*)(size_t)(o + 1), (const void*)&ic};
@@ -2107,7 +2149,8 @@ static void do_reset(tg_solver s, const double* cmua, const double* ckap, const 
     s->ic_done = s->res_ready = false;
     // (a resident solve's matrices, or the factor where its columns do not fit,
     // follow at the solve)
-    if ((pre == TG_PRECON_ICH || direct) && !resident_ok(s)) factor_ic<V64, V32>(s);
+    if (direct) direct_factor<V64>(s);
+    else if (pre == TG_PRECON_ICH && !resident_ok(s)) factor_ic<V64, V32>(s);
     if (mixed) {
         launch(abs_values_kernel<V64>, cdiv_u(m.nnz, 256), 256, 0, s->stream, m.nnz, A,
                (float*)s->absA.ensure((size_t)m.nnz * sizeof(float)));
@@ -2503,7 +2546,7 @@ static void solve_nm_body(tg_solver s, int k, const V64* B, V64* X, ColState* co
     Engine<V64>& e64 = engine<V64>(s);
     setup_engine(s, e64);
     if (s->method == TG_SOLVER_DIRECT) {
-        e64.direct_solve(k, B, X, co);
+        e64.direct_solve(k, B, X, co, [&] { direct_sweeps<V64>(s, k, B, X); });
         return;
     }
     if (s->precision == TG_PREC_FP64) {
