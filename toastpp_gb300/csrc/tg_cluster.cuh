@@ -49,6 +49,22 @@ struct ResArgs {
 template <class V64, class V32>
 void (*resident_kernel(int lv))(ResArgs<V64, V32>);
 
+// Both sweeps of the IC(0) apply in one launch: a cluster per lv columns
+template <class V>
+struct IcClArgs {
+    IcSweepDev f, b;
+    const V *vf, *vb;           // entries of the factor in the sweeps' layouts
+    const V* dinv;
+    const V* in;                // right-hand sides, node-major, k columns
+    V* out;                     // result
+    int n, k, cs;
+    int mofs;                   // byte offset of the levels and rows in shared memory
+    const ColState* st;         // columns with active != 1 keep their values (null: all)
+};
+constexpr int IC_NT = 256;      // threads of a CTA
+template <class V>
+void (*ic_cluster_kernel_of(int lv))(IcClArgs<V>);
+
 // G of the approximate inverse from A's values in CSR order, a warp per row
 constexpr int FSAI_WARPS = 4;
 template <class V>

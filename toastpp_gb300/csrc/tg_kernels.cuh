@@ -688,135 +688,6 @@ __global__ void __launch_bounds__(256) ic_level_ell(const int* __restrict__ rows
     }
 }
 
-// ---------------------------------------------------------------------------
-// The whole IC(0) apply (forward then backward sweep) as ONE persistent
-// cooperative launch: every warp walks the rows of a level (warp-strided),
-// and the levels are separated by a grid barrier instead of a kernel
-// boundary.  A level of the 30k cylinder's colour ordering takes about 2 us
-// of dependent gathers, against 5.6 us per level as separate launches.
-//
-// Blocks of 1024 threads, one or two per SM, so that few blocks arrive at
-// each barrier's counter.  The barrier spins with a bound: a block that
-// waits more than about half a second (it cannot, in a cooperative launch, whose blocks are all resident)
-// sets *err and goes on, later barriers stop waiting, the launch ends with
-// wrong values and the host reports the flag as an error.
-// ---------------------------------------------------------------------------
-template <class V>
-struct IcSweepArgs {
-    int nlev_f, nlev_b;
-    const int *lev_f, *lev_b;           // first row of each level (nlev + 1)
-    const int *w_f, *w_b, *off_f, *off_b;  // ELL width and offset per level
-    const int *rows_f, *rows_b, *ecol_f, *ecol_b;
-    const V *eval_f, *eval_b;
-    int k, ld;
-    const V* dinv;
-    const V* b;                         // right-hand side (forward sweep)
-    V* y;                               // result (written by both sweeps)
-    const ColState* st;
-    unsigned* bar;                      // barrier arrival count, zero at launch
-    int* err;                           // set when a barrier wait gave up
-};
-
-__device__ __forceinline__ void grid_barrier_bounded(unsigned* count, unsigned target, int* err)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(count, 1u);
-        if (!*(volatile int*)err) {
-            for (unsigned it = 0;; it++) {
-                unsigned v;
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-                if (v >= target) break;
-                if (it > (1u << 20)) { atomicExch(err, 1); break; }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-}
-
-// one row (ELL slot) of a level, columns lane + 32 j: the body of
-// ic_level_ell.  Plain loads of y are safe after the barrier: its fences
-// and acquire load order them after every other block's writes of the
-// earlier levels (the grid synchronisation pattern of cooperative groups).
-template <class V, int NJ, bool FWD>
-__device__ __forceinline__ void ic_ell_row(int slot, int lane, const int* __restrict__ rows, int w,
-                                           const int* __restrict__ ecol, const V* __restrict__ eval, int k, int ld,
-                                           const V* __restrict__ dinv, const V* __restrict__ b, V* __restrict__ y,
-                                           const ColState* __restrict__ st)
-{
-    const int i = rows[slot];
-    const V di = dinv[i];
-    V acc[NJ];
-#pragma unroll
-    for (int j = 0; j < NJ; j++) {
-        int c = lane + 32 * j;
-        acc[j] = c < k ? (FWD ? b[(size_t)i * ld + c] : y[(size_t)i * ld + c]) : vzero<V>();
-    }
-    constexpr int UNR = 4;
-    for (int base = 0; base < w; base += 32) {
-        const int cnt = min(32, w - base);
-        int my_c = -1;
-        V my_v = vzero<V>();
-        if (lane < cnt) {
-            my_c = ecol[(size_t)slot * w + base + lane];
-            my_v = eval[(size_t)slot * w + base + lane];
-        }
-        for (int e = 0; e < cnt; e += UNR) {
-            int cc[UNR];
-            V av[UNR];
-#pragma unroll
-            for (int u = 0; u < UNR; u++) {
-                cc[u] = __shfl_sync(0xffffffffu, my_c, min(e + u, 31));
-                av[u] = shfl(my_v, min(e + u, 31));
-            }
-            V g[UNR][NJ];
-#pragma unroll
-            for (int u = 0; u < UNR; u++)
-#pragma unroll
-                for (int j = 0; j < NJ; j++) {
-                    int c = lane + 32 * j;
-                    g[u][j] = (e + u < cnt && cc[u] >= 0 && c < k) ? y[(size_t)cc[u] * ld + c] : vzero<V>();
-                }
-#pragma unroll
-            for (int u = 0; u < UNR; u++)
-                if (e + u < cnt && cc[u] >= 0)
-#pragma unroll
-                    for (int j = 0; j < NJ; j++) acc[j] = vfms(acc[j], av[u], g[u][j]);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NJ; j++) {
-        int c = lane + 32 * j;
-        if (c < k && !(st && st[c].active != 1)) y[(size_t)i * ld + c] = vmul(acc[j], di);
-    }
-}
-
-template <class V, int NJ>
-__global__ void __launch_bounds__(1024) ic_sweep_persistent(IcSweepArgs<V> a)
-{
-    const int lane = threadIdx.x & 31;
-    const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int nw = (int)((gridDim.x * blockDim.x) >> 5);
-    unsigned nbar = 0;
-    for (int l = 0; l < a.nlev_f; l++) {
-        if (l) grid_barrier_bounded(a.bar, gridDim.x * ++nbar, a.err);
-        const int r0 = a.lev_f[l], nr = a.lev_f[l + 1] - r0, w = a.w_f[l], eo = a.off_f[l];
-        for (int slot = gw; slot < nr; slot += nw)
-            ic_ell_row<V, NJ, true>(slot, lane, a.rows_f + r0, w, a.ecol_f + eo, a.eval_f + eo, a.k, a.ld, a.dinv,
-                                    a.b, a.y, a.st);
-    }
-    for (int l = 0; l < a.nlev_b; l++) {
-        grid_barrier_bounded(a.bar, gridDim.x * ++nbar, a.err);
-        const int r0 = a.lev_b[l], nr = a.lev_b[l + 1] - r0, w = a.w_b[l], eo = a.off_b[l];
-        for (int slot = gw; slot < nr; slot += nw)
-            ic_ell_row<V, NJ, false>(slot, lane, a.rows_b + r0, w, a.ecol_b + eo, a.eval_b + eo, a.k, a.ld, a.dinv,
-                                     a.b, a.y, a.st);
-    }
-}
-
 // factor values into the ELL layouts (padding -> 0)
 template <class V>
 __global__ void ell_gather_kernel(int cnt, const int* __restrict__ src, const V* __restrict__ L, V* __restrict__ out)

@@ -678,10 +678,15 @@ Mesh::~Mesh()
             void* q[] = {p.second->ca, p.second->cg, p.second->ct, p.second->pofs, p.second->push};
             for (void* x : q) if (x) cudaFree(x);
         }
+    for (auto& p : ic_parts)
+        if (p.second)
+            for (IcSweepDev* w : {&p.second->f, &p.second->b}) {
+                void* q[] = {w->lev, w->pl, w->rows, w->col, w->src, w->push};
+                for (void* x : q) if (x) cudaFree(x);
+            }
     for (auto& g : d.ic) {
         void* q[] = {g.key, g.Lrowptr, g.Lcolidx, g.Lapos, g.Lkey, g.Ucolptr, g.Urow, g.Umap, g.fwd_lev_rows,
-                     g.bwd_lev_rows, g.fwd_ell_col, g.fwd_ell_src, g.bwd_ell_col, g.bwd_ell_src, g.fwd_lev_ptr,
-                     g.bwd_lev_ptr, g.fwd_ell_w, g.bwd_ell_w, g.fwd_ell_off, g.bwd_ell_off};
+                     g.bwd_lev_rows, g.fwd_ell_col, g.fwd_ell_src, g.bwd_ell_col, g.bwd_ell_src};
         for (void* p : q) if (p) cudaFree(p);
     }
 }
@@ -728,6 +733,7 @@ const PartDev* Mesh::part(int cs)
         auto local = [&](const SellHost& s, std::vector<unsigned short>& c) {
             for (int o = s.ptr[s0]; o < s.ptr[s1]; o++) c[o] = (unsigned short)slot[s.col[o]];
         };
+        P->halo.push_back(halo);
         local(h.sa, ca);
         local(h.sg, cg);
         local(h.st, ct);
@@ -747,8 +753,88 @@ const PartDev* Mesh::part(int cs)
     P->ct = upload(ct);
     P->pofs = upload(pofs);
     P->push = upload(push);
+    P->copies = std::move(places);
     const PartDev* p = P.get();
     parts[cs] = std::move(P);
+    return p;
+}
+
+const IcPartDev* Mesh::ic_part(int cs, int o)
+{
+    const PartDev* P = part(cs);
+    if (!P) return nullptr;
+    std::lock_guard<std::mutex> lk(part_mu);
+    auto it = ic_parts.find({cs, o});
+    if (it != ic_parts.end()) return it->second.get();
+    const int n = h.n, ns = (n + 31) / 32;
+    const ICHost& c = h.ic[o];
+    auto I = std::make_unique<IcPartDev>();
+    std::vector<int> owner(n), place(n);
+    std::vector<std::vector<unsigned>> at(n);  // halo places of each row
+    std::vector<int> first(cs + 1);
+    for (int r = 0; r <= cs; r++) first[r] = std::min(n, (int)((long long)ns * r / cs) * 32);
+    for (int r = 0; r < cs; r++) {
+        for (int i = first[r]; i < first[r + 1]; i++) owner[i] = r;
+        for (const uint2& t : P->copies[r]) at[first[r] + t.x].push_back(t.y);
+    }
+    auto sweep = [&](bool fwd, IcSweepDev& w) {
+        const std::vector<int>&ptr = fwd ? c.fwd_lev_ptr : c.bwd_lev_ptr, &rows = fwd ? c.fwd_lev_rows : c.bwd_lev_rows;
+        const int nlev = (int)ptr.size() - 1;
+        std::vector<int4> lev((size_t)cs * nlev, int4{0, 0, 0, 0});
+        std::vector<int2> pl((size_t)cs * nlev, int2{0, 0});
+        std::vector<unsigned short> rw, col;
+        std::vector<int> src, mine;
+        std::vector<uint2> push;
+        for (int r = 0; r < cs; r++) {
+            for (int i = first[r]; i < first[r + 1]; i++) place[i] = i - first[r];
+            const int own = first[r + 1] - first[r];
+            for (size_t t = 0; t < P->halo[r].size(); t++) place[P->halo[r][t]] = own + (int)t;
+            for (int l = 0; l < nlev; l++) {
+                mine.clear();
+                int width = 0;
+                for (int t = ptr[l]; t < ptr[l + 1]; t++) {
+                    const int p = rows[t];
+                    if (owner[p] != r) continue;
+                    mine.push_back(p);
+                    width = std::max(width, fwd ? c.Lrowptr[p + 1] - c.Lrowptr[p] : c.Ucolptr[p + 1] - c.Ucolptr[p]);
+                }
+                // rows of about the same number of entries share a warp
+                std::stable_sort(mine.begin(), mine.end(), [&](int x, int y) {
+                    return fwd ? c.Lrowptr[x + 1] - c.Lrowptr[x] > c.Lrowptr[y + 1] - c.Lrowptr[y]
+                               : c.Ucolptr[x + 1] - c.Ucolptr[x] > c.Ucolptr[y + 1] - c.Ucolptr[y];
+                });
+                const int nr = (int)mine.size(), off = (int)col.size();
+                lev[(size_t)r * nlev + l] = int4{(int)rw.size(), nr, width, off};
+                col.resize(off + (size_t)nr * width, 0xffff);
+                src.resize(off + (size_t)nr * width, -1);
+                pl[(size_t)r * nlev + l].x = (int)push.size();
+                for (int s = 0; s < nr; s++) {
+                    const int p = mine[s];
+                    rw.push_back((unsigned short)place[p]);
+                    // forward: ascending rank; backward: descending, the order CholeskySubst subtracts them
+                    for (int e = 0; e < (fwd ? c.Lrowptr[p + 1] - c.Lrowptr[p] : c.Ucolptr[p + 1] - c.Ucolptr[p]); e++) {
+                        const int q = fwd ? c.Lrowptr[p] + e : c.Ucolptr[p + 1] - 1 - e;
+                        col[off + (size_t)e * nr + s] = (unsigned short)place[fwd ? c.Lcolidx[q] : c.Urow[q]];
+                        src[off + (size_t)e * nr + s] = fwd ? q : c.Umap[q];
+                    }
+                    for (unsigned t : at[p]) push.push_back(uint2{(unsigned)place[p], t});
+                }
+                pl[(size_t)r * nlev + l].y = (int)push.size() - pl[(size_t)r * nlev + l].x;
+            }
+        }
+        w.nlev = nlev;
+        w.nell = (int)col.size();
+        w.lev = upload(lev);
+        w.pl = upload(pl);
+        w.rows = upload(rw);
+        w.col = upload(col);
+        w.src = upload(src);
+        w.push = upload(push);
+    };
+    sweep(true, I->f);
+    sweep(false, I->b);
+    const IcPartDev* p = I.get();
+    ic_parts[{cs, o}] = std::move(I);
     return p;
 }
 
@@ -837,12 +923,6 @@ Mesh* mesh_build(int dim, int n, const double* coords, int ne, const int* el)
         g.fwd_ell_src = upload(c.fwd_ell_src);
         g.bwd_ell_col = upload(c.bwd_ell_col);
         g.bwd_ell_src = upload(c.bwd_ell_src);
-        g.fwd_lev_ptr = upload(c.fwd_lev_ptr);
-        g.bwd_lev_ptr = upload(c.bwd_lev_ptr);
-        g.fwd_ell_w = upload(c.fwd_ell_w);
-        g.bwd_ell_w = upload(c.bwd_ell_w);
-        g.fwd_ell_off = upload(c.fwd_ell_off);
-        g.bwd_ell_off = upload(c.bwd_ell_off);
     }
     return M;
 }

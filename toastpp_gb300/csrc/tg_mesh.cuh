@@ -60,9 +60,6 @@ struct ICDev {
     int *key, *Lrowptr, *Lcolidx, *Lapos, *Lkey, *Ucolptr, *Urow, *Umap;
     int *fwd_lev_rows, *bwd_lev_rows;
     int *fwd_ell_col, *fwd_ell_src, *bwd_ell_col, *bwd_ell_src;
-    // per level: first row (nlev + 1 entries), ELL width and ELL offset, for
-    // the persistent sweep kernel
-    int *fwd_lev_ptr, *bwd_lev_ptr, *fwd_ell_w, *bwd_ell_w, *fwd_ell_off, *bwd_ell_off;
 };
 
 // A sparsity pattern in slices of 32 rows: entry e of row r at ptr[r / 32] +
@@ -147,6 +144,24 @@ struct PartDev {
     int npush;                             // halo copies of a CTA: the largest of the CTAs
     int* pofs;
     uint2* push;
+    std::vector<std::vector<int>> halo;    // host: halo rows of each CTA
+    std::vector<std::vector<uint2>> copies;  // host: the halo copies of each CTA's rows
+};
+
+// The level schedule of an IC(0) sweep split the same way: per CTA and level
+// (CTA-major) {first row, rows, ELL width, ELL offset} and {first copy,
+// copies}; rows as own slots, entry e of row s of a level at offset + e * rows
+// + s with the column as a slot, and the halo copies of the level's rows.
+struct IcSweepDev {
+    int4* lev;
+    int2* pl;
+    unsigned short *rows, *col;
+    int* src;                              // the entry in L
+    uint2* push;
+    int nlev, nell;
+};
+struct IcPartDev {
+    IcSweepDev f, b;
 };
 
 struct Mesh {
@@ -158,6 +173,9 @@ struct Mesh {
     const PartDev* part(int cs);
     std::mutex part_mu;
     std::map<int, std::unique_ptr<PartDev>> parts;
+    // the schedule of ordering o (null where part(cs) is)
+    const IcPartDev* ic_part(int cs, int o);
+    std::map<std::pair<int, int>, std::unique_ptr<IcPartDev>> ic_parts;
     long long uid = 0;  // unique per mesh built in this process
     ~Mesh();
 };

@@ -719,6 +719,142 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
     cl_sync(cs);
 }
 
+// ---------------------------------------------------------------------------
+// The IC(0) apply of the batched methods (FP64 path, natural ordering) as one
+// launch.  A level per launch took 6 us, of which less than two were work: 190
+// us an apply for 32 complex FP64 columns of the 12.5k-node disc (32 levels),
+// 105 as clusters (560 -> 270 us on a 19.6k-node cylinder, 142 -> 57 for 8
+// columns of a 1.3k-node disc).  y stays in shared memory with the halo rows of
+// the CTA's matrix rows; at the end of a level its rows go to the other CTAs'
+// halos and the cluster's barrier follows.  What the next level needs and no
+// level writes (its rows, columns, factor entries, right-hand sides, pivots)
+// loads before that barrier, so that after it a row is shared-memory reads and
+// its sum.  (Loading it a whole level ahead, in a second register set, was
+// slower: FP64 issue bounds a level, not these loads.)  The rows of a level lie
+// by their number of entries, so that a warp's rows end together.  Every row's sum runs in the same order as in the level kernels:
+// the results are the same to the bit.
+// ---------------------------------------------------------------------------
+template <class V, int LV>
+__global__ void __launch_bounds__(IC_NT) ic_cluster_kernel(IcClArgs<V> a)
+{
+    using VN = VecN<LV, V>;
+    constexpr int WP = 8;  // entries of a row in flight
+    extern __shared__ __align__(16) unsigned char cl_sm[];
+    V* y = reinterpret_cast<V*>(cl_sm);  // [slots][LV]
+    const int tid = threadIdx.x, cs = a.cs, rank = cs > 1 ? cl_rank() : 0;
+    const int c0 = blockIdx.x / cs * LV, ns = (a.n + 31) >> 5, R0 = (int)((long long)ns * rank / cs) * 32;
+    const size_t ld = a.k;
+    bool on[LV], live = false;
+#pragma unroll
+    for (int j = 0; j < LV; j++) {
+        on[j] = c0 + j < a.k && (!a.st || a.st[c0 + j].active == 1);
+        live |= on[j];
+    }
+    if (!live) return;  // the same in every CTA of the cluster
+    // the levels, their halo copies and the rows of both sweeps
+    const int total = a.f.nlev + a.b.nlev;
+    int4* lev = reinterpret_cast<int4*>(cl_sm + a.mofs);
+    int2* pl = reinterpret_cast<int2*>(lev + total);
+    unsigned short* rows = reinterpret_cast<unsigned short*>(pl + total);
+    {
+        const int4* lf = a.f.lev + rank * a.f.nlev;
+        const int4* lb = a.b.lev + rank * a.b.nlev;
+        const int f0 = lf[0].x, b0 = lb[0].x, own = lf[a.f.nlev - 1].x + lf[a.f.nlev - 1].y - f0;
+        for (int t = tid; t < total; t += IC_NT) {
+            const bool fwd = t < a.f.nlev;
+            int4 L = fwd ? lf[t] : lb[t - a.f.nlev];
+            L.x += fwd ? -f0 : own - b0;  // place in rows
+            lev[t] = L;
+            pl[t] = fwd ? a.f.pl[rank * a.f.nlev + t] : a.b.pl[rank * a.b.nlev + t - a.f.nlev];
+        }
+        for (int t = tid; t < own; t += IC_NT) { rows[t] = a.f.rows[f0 + t]; rows[own + t] = a.b.rows[b0 + t]; }
+    }
+    cl_sync(cs);        // every CTA runs before any stores into another's shared memory
+    const V* in = a.in + (size_t)R0 * ld + c0;
+    V* out = a.out + (size_t)R0 * ld + c0;
+    const V* dinv = a.dinv + R0;
+    int slot = 0, c[WP];
+    V v[WP], di = vzero<V>();
+    VN rhs;
+    uint2 pe = make_uint2(0u, 0u);
+    // row s of level L: its first entries, pivot and, forward, right-hand side
+    auto fetch = [&](const IcSweepDev& w, const V* val, const int4& L, int s, bool fwd) {
+        slot = rows[L.x + s];
+#pragma unroll
+        for (int u = 0; u < WP; u++)
+            if (u < L.z) { c[u] = w.col[L.w + u * L.y + s]; v[u] = val[L.w + u * L.y + s]; }
+        di = dinv[slot];
+        if (fwd)
+#pragma unroll
+            for (int j = 0; j < LV; j++) rhs.v[j] = on[j] ? in[(size_t)slot * ld + j] : vzero<V>();
+    };
+    int4 L = lev[0];
+    int2 P = pl[0];
+    if (tid < L.y) fetch(a.f, a.vf, L, tid, true);
+    if (tid < P.y) pe = a.f.push[P.x + tid];
+    for (int l = 0; l < total; l++) {
+        const bool fwd = l < a.f.nlev;
+        const IcSweepDev& w = fwd ? a.f : a.b;
+        const V* val = fwd ? a.vf : a.vb;
+        for (int s = tid; s < L.y; s += IC_NT) {
+            if (s != tid) fetch(w, val, L, s, fwd);
+            VN acc = fwd ? rhs : *reinterpret_cast<const VN*>(y + slot * LV);
+            for (int e = 0;;) {
+#pragma unroll
+                for (int u = 0; u < WP; u++)
+                    if (e + u < L.z && c[u] != 0xffff) {
+                        const VN g = *reinterpret_cast<const VN*>(y + c[u] * LV);
+#pragma unroll
+                        for (int j = 0; j < LV; j++) acc.v[j] = vfms(acc.v[j], v[u], g.v[j]);
+                    }
+                e += WP;
+                if (e >= L.z) break;
+#pragma unroll
+                for (int u = 0; u < WP; u++)
+                    if (e + u < L.z) { c[u] = w.col[L.w + (e + u) * L.y + s]; v[u] = val[L.w + (e + u) * L.y + s]; }
+            }
+#pragma unroll
+            for (int j = 0; j < LV; j++) acc.v[j] = vmul(acc.v[j], di);
+            *reinterpret_cast<VN*>(y + slot * LV) = acc;
+            if (!fwd)
+#pragma unroll
+                for (int j = 0; j < LV; j++)
+                    if (on[j]) out[(size_t)slot * ld + j] = acc.v[j];
+        }
+        if (l + 1 == total) break;
+        if (cs > 1) {
+            __syncthreads();
+            for (int t = tid; t < P.y; t += IC_NT) {
+                if (t != tid) pe = w.push[P.x + t];
+                const VN x = *reinterpret_cast<const VN*>(y + pe.x * LV);
+                cl_store_bytes<sizeof(VN)>(cl_map(y + (pe.y & 0xffffu) * LV, (int)(pe.y >> 16)), &x);
+            }
+        }
+        const bool nf = l + 1 < a.f.nlev;
+        const IcSweepDev& nw = nf ? a.f : a.b;
+        L = lev[l + 1];
+        P = pl[l + 1];
+        if (tid < L.y) fetch(nw, nf ? a.vf : a.vb, L, tid, nf);
+        if (tid < P.y) pe = nw.push[P.x + tid];
+        cl_sync(cs);
+    }
+    cl_sync(cs);  // no CTA leaves while another may still write its shared memory
+}
+
+template <class V>
+void (*ic_cluster_kernel_of(int lv))(IcClArgs<V>)
+{
+    if constexpr (sizeof(V) == 4)
+        if (lv == 4) return ic_cluster_kernel<V, 4>;
+    if constexpr (sizeof(V) <= 8)
+        if (lv == 2) return ic_cluster_kernel<V, 2>;
+    return ic_cluster_kernel<V, 1>;
+}
+template void (*ic_cluster_kernel_of<double>(int))(IcClArgs<double>);
+template void (*ic_cluster_kernel_of<float>(int))(IcClArgs<float>);
+template void (*ic_cluster_kernel_of<cd>(int))(IcClArgs<cd>);
+template void (*ic_cluster_kernel_of<cf>(int))(IcClArgs<cf>);
+
 template <class V64, class V32>
 void (*resident_kernel(int lv))(ResArgs<V64, V32>)
 {

@@ -42,7 +42,7 @@ static std::atomic<long long> g_nlaunch{0};
 // SpMM variant chosen per (mesh, value type, k), shared by every solver of the process
 static std::mutex g_tune_mu;
 static std::map<std::tuple<long long, int, int>, int> g_tune;
-// IC apply variant (persistent sweep or per-level launches) per (mesh and
+// IC apply variant (cluster sweep or per-level launches) per (mesh and
 // pattern, value type, k), chosen like the SpMM variant
 static std::map<std::tuple<long long, int, int>, bool> g_ictune;
 static std::string g_tune_log;  // one line per decision: candidates with their best launch time
@@ -109,6 +109,30 @@ static inline void launch_cluster(void (*k)(KArgs...), unsigned ng, int cs, int 
     cluster_config(cfg, at, ng, cs, nt, sm, st);
     TG_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...));
     g_nlaunch.fetch_add(1, std::memory_order_relaxed);
+}
+
+constexpr size_t CL_SMEM = 212 * 1024;  // dynamic shared memory of the cluster kernels at most
+
+// clusters of a kernel that the device runs at a time (0: the shape is refused)
+static int clusters_at_once(const void* kern, unsigned ng, int cs, int nt, size_t sm, cudaStream_t st)
+{
+    int at_once = 0;
+    if (cs > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        cluster_config(cfg, at, ng, cs, nt, sm, st);
+        if (cs > 8) TG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        if (cudaOccupancyMaxActiveClusters(&at_once, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return at_once;
+    }
+    int dev = 0, nsm = 0;
+    TG_CUDA(cudaGetDevice(&dev));
+    TG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&at_once, kern, nt, sm));
+    TG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    return at_once * nsm;
 }
 
 // Raise a kernel's dynamic shared-memory limit to the device's opt-in
@@ -341,7 +365,15 @@ struct Engine {
     int precon = 0;            // 0 none, 1 diag, 2 ich
     Profiler* prof = nullptr;
     DBuf w[9], part, cs, cnt, gbasis, gcol;
-    DBuf sweep;  // persistent IC sweep: [0] error flag, [1] barrier count
+    // factor entries in the cluster sweep's layouts, per (CTAs, ordering): captured
+    // graphs hold the buffers, so each layout has its own
+    struct ClValues {
+        DBuf f, b;
+        long long ver = -1;
+    };
+    std::map<std::pair<int, int>, ClValues> clv;
+    long long fver = 0;        // version of the factor behind L
+    std::map<int, std::pair<int, int>> ic_shapes;  // k -> (columns, CTAs) of a cluster; CTAs 0: none fits
     Bounce bnc;
     GraphCache graphs;
 
@@ -531,16 +563,92 @@ struct Engine {
         }
     }
 
-    // The persistent sweep (ic_sweep_persistent, one cooperative launch for
-    // the whole apply) or a launch per level: both compute every row with the
-    // same sums in the same order (bit-identical results).  The first apply
-    // of a (mesh, pattern, value type, k) in the process times both (best of
-    // three, in a graph each) and keeps the faster for the process;
-    // TOASTGPU_IC_PERSISTENT=0 / 1 fixes the choice.
-    bool ic_persistent(int k, const V* in, V* out, const ColState* cst)
+    // Columns and CTAs of a cluster of the cluster sweep: all columns at once on
+    // the chip, with the fewest rows per CTA; (0, 0) where nothing fits
+    std::pair<int, int> ic_shape(int k)
+    {
+        auto it = ic_shapes.find(k);
+        if (it != ic_shapes.end()) return it->second;
+        std::pair<int, int> best{0, 0};
+        double tbest = 1e300;
+        for (int cs = 1; cs <= 8; cs *= 2) {
+            if (mesh->d.n / cs > 16384 || (cs > 1 && mesh->d.n / cs < 200)) continue;
+            const PartDev* P = mesh->part(cs);
+            if (!P) continue;
+            for (int lv = 1; lv * (int)sizeof(V) <= 16 && (lv == 1 || lv < 2 * k); lv *= 2) {
+                const size_t sm = ic_smem(*P, lv);
+                if (sm > CL_SMEM) continue;
+                auto kern = ic_cluster_kernel_of<V>(lv);
+                allow_smem((const void*)kern);
+                const int at_once = clusters_at_once((const void*)kern, (k + lv - 1) / lv, cs, IC_NT, sm, st);
+                if (at_once < 1) continue;
+                const int waves = ((k + lv - 1) / lv + at_once - 1) / at_once;
+                // a level: barrier and loads, then the rows of a thread
+                const ICHost& c = ic_host();
+                const double lv_rows = (double)mesh->d.n / std::max<size_t>(1, c.fwd_lev_ptr.size() - 1) / cs;
+                const double t = waves * ((cs > 1 ? 2.0 : 1.0) + std::ceil(lv_rows / IC_NT) * lv * sizeof(S) / 4.0);
+                if (t < tbest) { tbest = t; best = {lv, cs}; }
+            }
+        }
+        if (ic_shapes.size() >= 64) ic_shapes.clear();
+        return ic_shapes[k] = best;
+    }
+
+    // shared memory of a CTA: the vector, then levels and rows of both sweeps
+    size_t ic_vec_bytes(const PartDev& P, int lv) const { return ((size_t)P.slots * lv * sizeof(V) + 15) / 16 * 16; }
+    size_t ic_smem(const PartDev& P, int lv)
+    {
+        const ICHost& c = ic_host();
+        const size_t nlev = c.fwd_lev_ptr.size() + c.bwd_lev_ptr.size() - 2;
+        return ic_vec_bytes(P, lv) + nlev * (sizeof(int4) + sizeof(int2)) + (size_t)2 * P.own * 2;
+    }
+
+    // the factor's entries in the layouts of clusters of cs CTAs
+    void ic_cluster_values(int cs)
+    {
+        ClValues& c = clv[{cs, ico}];
+        if (c.ver == fver) return;
+        const IcPartDev* I = mesh->ic_part(cs, ico);
+        V* f = (V*)c.f.ensure((size_t)std::max(I->f.nell, 1) * sizeof(V));
+        V* b = (V*)c.b.ensure((size_t)std::max(I->b.nell, 1) * sizeof(V));
+        launch(ell_gather_kernel<V>, cdiv_u(std::max(I->f.nell, 1), 256), 256, 0, st, I->f.nell, I->f.src, L, f);
+        launch(ell_gather_kernel<V>, cdiv_u(std::max(I->b.nell, 1), 256), 256, 0, st, I->b.nell, I->b.src, L, b);
+        c.ver = fver;
+    }
+
+    // before a solve (and outside a capture): the cluster sweep's entries, where k columns use it
+    void ic_prepare(int k)
+    {
+        if (precon == 2 && ic_clustered(k)) ic_cluster_values(ic_shape(k).second);
+    }
+
+    // TOASTGPU_IC_PERSISTENT=0 / 1: per-level launches / the cluster sweep
+    int ic_forced() const
     {
         const char* e = getenv("TOASTGPU_IC_PERSISTENT");
-        if (e && (e[0] == '0' || e[0] == '1')) return e[0] == '1';
+        return e && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : -1;
+    }
+    bool ic_clustered(int k)
+    {
+        if (!ic_shape(k).second) return false;
+        const int f = ic_forced();
+        if (f >= 0) return f == 1;
+        const auto key = std::make_tuple(mesh->uid * 4 + ico, (int)sizeof(V) * 2 + (int)vt<V>::cplx, k);
+        std::lock_guard<std::mutex> g(g_tune_mu);
+        auto it = g_ictune.find(key);
+        return it != g_ictune.end() && it->second;
+    }
+
+    // The cluster sweep (one launch, tg_resident.cu) or a launch per level: both
+    // compute every row with the same sums in the same order (bit-identical
+    // results).  The first apply of a (mesh, ordering, value type, k) in the
+    // process times both (best of three, in a graph each) and keeps the faster
+    // for the process.
+    bool ic_use_cluster(int k, const V* in, V* out, const ColState* cst)
+    {
+        if (!ic_shape(k).second) return false;
+        const int f = ic_forced();
+        if (f >= 0) return f == 1;
         const auto key = std::make_tuple(mesh->uid * 4 + ico, (int)sizeof(V) * 2 + (int)vt<V>::cplx, k);
         {
             std::lock_guard<std::mutex> g(g_tune_mu);
@@ -549,12 +657,13 @@ struct Engine {
         }
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         TG_CUDA(cudaStreamIsCapturing(st, &cs));
-        if (cs != cudaStreamCaptureStatusNone) return false;
+        if (cs != cudaStreamCaptureStatusNone || in == out) return false;
         float best[2] = {1e30f, 1e30f};
         cudaEvent_t ev[2];
         for (auto& x : ev) TG_CUDA(cudaEventCreate(&x));
         for (int r = 0; r < 4; r++)
             for (int v = 0; v < 2; v++) {
+                if (v) ic_cluster_values(ic_shape(k).second);
                 TG_CUDA(cudaEventRecord(ev[0], st));
                 ic_apply_variant(k, in, out, cst, v == 1);
                 TG_CUDA(cudaEventRecord(ev[1], st));
@@ -569,103 +678,57 @@ struct Engine {
         auto res = g_ictune.emplace(key, p);
         if (res.second) {
             char line[200];
-            snprintf(line, sizeof line, "mesh %lld %s k=%d: ic per-level %.1fus persistent %.1fus -> %s\n",
-                     (long long)mesh->uid, vt_name<V>(), k, best[0] * 1e3f, best[1] * 1e3f,
-                     p ? "persistent" : "per-level");
+            snprintf(line, sizeof line, "mesh %lld %s k=%d: ic per-level %.1fus cluster %.1fus -> %s\n",
+                     (long long)mesh->uid, vt_name<V>(), k, best[0] * 1e3f, best[1] * 1e3f, p ? "cluster" : "per-level");
             g_tune_log += line;
         }
         return res.first->second;
     }
-    template <int NJ>
-    void launch_sweep_persistent(int k, const V* in, V* out, const ColState* cst)
+
+    void launch_ic_cluster(int k, const V* in, V* out, const ColState* cst)
     {
-        const ICHost& ch = ic_host();
-        const ICDev& ic = ic_dev();
-        auto kern = ic_sweep_persistent<V, NJ>;
-        static int grid[64] = {};
-        int dev = 0;
-        TG_CUDA(cudaGetDevice(&dev));
-        if (dev < 0 || dev >= 64) throw Error{TG_ERR_CUDA, "device index out of range"};
-        if (!grid[dev]) {
-            int nb = 0, nsm = 0;
-            TG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 1024, 0));
-            TG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-            grid[dev] = std::max(1, nb) * nsm;
-        }
-        IcSweepArgs<V> a;
-        a.nlev_f = (int)ch.fwd_lev_ptr.size() - 1;
-        a.nlev_b = (int)ch.bwd_lev_ptr.size() - 1;
-        a.lev_f = ic.fwd_lev_ptr; a.lev_b = ic.bwd_lev_ptr;
-        a.w_f = ic.fwd_ell_w; a.w_b = ic.bwd_ell_w; a.off_f = ic.fwd_ell_off; a.off_b = ic.bwd_ell_off;
-        a.rows_f = ic.fwd_lev_rows; a.rows_b = ic.bwd_lev_rows;
-        a.ecol_f = ic.fwd_ell_col; a.ecol_b = ic.bwd_ell_col;
-        a.eval_f = Lef; a.eval_b = Leb;
-        a.k = k; a.ld = k; a.dinv = dinv; a.b = in; a.y = out; a.st = cst;
-        int* fl = sweep.as<int>();
-        a.err = fl;
-        a.bar = (unsigned*)(fl + 1);
-        TG_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned), st));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)grid[dev]);
-        cfg.blockDim = dim3(1024);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        TG_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
-        g_nlaunch.fetch_add(1, std::memory_order_relaxed);
+        const auto sh = ic_shape(k);
+        const IcPartDev* I = mesh->ic_part(sh.second, ico);
+        const PartDev& P = *mesh->part(sh.second);
+        IcClArgs<V> a;
+        a.mofs = (int)ic_vec_bytes(P, sh.first);
+        a.f = I->f; a.b = I->b;
+        const ClValues& c = clv[{sh.second, ico}];
+        a.vf = c.f.template as<V>(); a.vb = c.b.template as<V>(); a.dinv = dinv;
+        a.in = in; a.out = out; a.n = mesh->d.n; a.k = k; a.cs = sh.second; a.st = cst;
+        launch_cluster(ic_cluster_kernel_of<V>(sh.first), cdiv_u(k, sh.first), sh.second, IC_NT,
+                       ic_smem(P, sh.first), st, a);
     }
 
-    // the barrier flag of the persistent sweep: set when a wait gave up
-    void check_sweep()
-    {
-        if (!sweep.p) return;
-        int h[2] = {0, 0};
-        bnc.fetch(h, sweep.p, sizeof(h), st);
-        if (h[0]) {
-            TG_CUDA(cudaMemsetAsync(sweep.p, 0, sizeof(int), st));
-            throw Error{TG_ERR_CUDA, "IC(0) sweep: a grid barrier wait gave up (results discarded)"};
-        }
-    }
-
-    // out = M^-1 in for the IC(0) preconditioner: the forward and backward
-    // level kernels, captured once per (k, buffers) and replayed as one graph
-    // (k in 32..256: one persistent cooperative launch for both sweeps)
+    // out = M^-1 in for the IC(0) preconditioner: one launch on clusters, or the
+    // forward and backward level kernels, captured once per (k, buffers) and
+    // replayed as one graph
     void ic_apply(int k, const V* in, V* out, const ColState* cst)
     {
-        const bool wide = k >= 32 && k <= 256;
-        // (the tuning runs repeat the apply: they need in and out apart)
-        const bool persistent = wide && in != out && ic_persistent(k, in, out, cst);
+        const bool cluster = ic_use_cluster(k, in, out, cst);
+        if (cluster) {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            TG_CUDA(cudaStreamIsCapturing(st, &cs));
+            // (in a capture the values are in place: the solve began with ic_prepare)
+            if (cs == cudaStreamCaptureStatusNone) ic_cluster_values(ic_shape(k).second);
+        }
         ProfScope ps(prof, PC_SWEEP, st);
-        ic_apply_variant(k, in, out, cst, persistent);
+        ic_apply_variant(k, in, out, cst, cluster);
     }
 
-    void ic_apply_variant(int k, const V* in, V* out, const ColState* cst, bool persistent)
+    void ic_apply_variant(int k, const V* in, V* out, const ColState* cst, bool cluster)
     {
         const MeshDev& m = mesh->d;
         const ICHost& ch = ic_host();
         const ICDev& ic = ic_dev();
-        int cw = colw(k), ncg = (k + cw - 1) / cw, rpw = 32 / cw;
-        std::vector<const void*> key = {(const void*)(size_t)k, in, out, cst, L, dinv, Lef, Leb, mesh,
-                                        (const void*)(size_t)ico, (const void*)(size_t)persistent};
-        const bool wide = k >= 32 && k <= 256;
-        if (persistent) {
-            if (!sweep.p) {
-                sweep.ensure(2 * sizeof(int));
-                TG_CUDA(cudaMemsetAsync(sweep.p, 0, 2 * sizeof(int), st));
-            }
-            graphs.run(st, key, [&] {
-                switch ((k + 31) / 32) {
-#define TG_SW(J) case J: launch_sweep_persistent<J>(k, in, out, cst); break;
-                TG_SW(1) TG_SW(2) TG_SW(3) TG_SW(4) TG_SW(5) TG_SW(6) TG_SW(7) TG_SW(8)
-#undef TG_SW
-                }
-            });
+        if (cluster) {
+            launch_ic_cluster(k, in, out, cst);
             return;
         }
+        int cw = colw(k), ncg = (k + cw - 1) / cw, rpw = 32 / cw;
+        std::vector<const void*> key = {(const void*)(size_t)k, in, out, cst, L, dinv, Lef, Leb, mesh,
+                                        (const void*)(size_t)ico};
+        const bool wide = k >= 32 && k <= 256;
         graphs.run(st, key, [&] {
             const std::vector<int>& fp = ch.fwd_lev_ptr;
             for (size_t l = 0; l + 1 < fp.size(); l++) {
@@ -1884,6 +1947,7 @@ struct tg_solver_s {
     int jflip = 0;
     bool reset_done = false;
     bool ic_done = false;      // the factor of the current matrix is in place
+    long long fver = 0;        // factorisations so far
     bool res_ready = false;    // and the resident solve's matrices
     std::map<int, ClShape> shapes;  // by number of columns
     DBuf sa32, sg32, st32, xff, xkeep;  // resident solve: sliced matrices, split solution, kept guess
@@ -2046,6 +2110,7 @@ static void setup_engine(tg_solver s, Engine<V64>& e64)
     e64.Leb = s->eb64.as<V64>();
     e64.prof = &s->prof;
     e64.ico = 0;
+    e64.fver = s->fver;
 }
 
 // IC ordering the solver's preconditioner is factored in: the natural
@@ -2091,6 +2156,7 @@ static void factor_ic(tg_solver s)
                (V32*)s->dinv32.ensure(m.n * sizeof(V32)));
     }
     s->ic_done = true;
+    s->fver++;
 }
 
 // the resident solve's matrices of the last reset: A in slices, G, and G^T
@@ -2385,8 +2451,6 @@ static void solve_reliable(tg_solver s, int k, const V64* B, V64* X, ColState* c
     launch(rel_finish_kernel, ek, 128, 0, s->stream, k, co, ci);
 }
 
-constexpr size_t CL_SMEM = 212 * 1024;
-
 // How k columns go to clusters: the lv columns of a cluster, its CTAs and
 // threads, by the estimated time of an iteration times the waves of clusters.
 // The estimate (clock cycles) is a fixed part of barriers and reductions, and
@@ -2434,22 +2498,7 @@ static ClShape resident_shape(tg_solver s, int k)
             c.nt = std::max(64, (P.own + rounds * 32 - 1) / (rounds * 32) * 32);
             auto kern = resident_kernel<V64, V32>(lv);
             allow_smem((const void*)kern);
-            int at_once = 0;
-            if (cs > 1) {
-                cudaLaunchConfig_t cfg = {};
-                cudaLaunchAttribute at[1];
-                cluster_config(cfg, at, (k + lv - 1) / lv, cs, c.nt, c.sm, s->stream);
-                if (cs > 8) TG_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-                if (cudaOccupancyMaxActiveClusters(&at_once, (const void*)kern, &cfg) != cudaSuccess) {
-                    cudaGetLastError();
-                    continue;
-                }
-            } else {
-                int nsm = 0;
-                TG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&at_once, kern, c.nt, c.sm));
-                TG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, mesh->device));
-                at_once *= nsm;
-            }
+            const int at_once = clusters_at_once((const void*)kern, (k + lv - 1) / lv, cs, c.nt, c.sm, s->stream);
             if (at_once < 1) continue;
             const int waves = ((k + lv - 1) / lv + at_once - 1) / at_once;
             const double fix = 9e3 + (cs > 1 ? 800.0 * std::log2((double)cs) * std::log2((double)cs) : 0.0);
@@ -2524,19 +2573,7 @@ static bool solve_resident(tg_solver s, int k, const V64* B, V64* X, ColState* c
 }
 
 template <class V64, class V32>
-static void solve_nm_body(tg_solver s, int k, const V64* B, V64* X, ColState* co, bool zero_guess);
-
-// solve_nm_body, then the persistent sweep's barrier flag of both engines
-template <class V64, class V32>
 static void solve_nm(tg_solver s, int k, const V64* B, V64* X, ColState* co, bool zero_guess = false)
-{
-    solve_nm_body<V64, V32>(s, k, B, X, co, zero_guess);
-    engine<V64>(s).check_sweep();
-    if (s->precision == TG_PREC_MIXED) engine<V32>(s).check_sweep();
-}
-
-template <class V64, class V32>
-static void solve_nm_body(tg_solver s, int k, const V64* B, V64* X, ColState* co, bool zero_guess)
 {
     const MeshDev& m = s->mesh->d;
     int n = m.n;
@@ -2550,6 +2587,7 @@ static void solve_nm_body(tg_solver s, int k, const V64* B, V64* X, ColState* co
         return;
     }
     if (s->precision == TG_PREC_FP64) {
+        e64.ic_prepare(k);
         e64.solve(s->method, k, B, X, co, zero_guess);
         return;
     }
@@ -2584,6 +2622,8 @@ static void solve_nm_body(tg_solver s, int k, const V64* B, V64* X, ColState* co
     e32.Leb = s->eb32.as<V32>();
     e32.prof = &s->prof;
     e32.ico = ic_order(s);
+    e32.fver = s->fver;
+    e32.ic_prepare(k);
     V64* R = (V64*)s->tmp.ensure(nk * sizeof(V64));
     V32* R32 = (V32*)s->B32.ensure(nk * sizeof(V32));
     V32* E32 = (V32*)s->X32.ensure(nk * sizeof(V32));
