@@ -16,7 +16,7 @@
 // group of sources walks the sources' links and writes its column of every
 // link row.
 #pragma once
-#include "tg_kernels.cuh"
+#include "tg_jac.cuh"
 
 namespace tg {
 
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) grid_planes_kernel(GridDev G, int k, cons
 // columns c < k0 from x0, the others from x1.  A thread per grid point keeps
 // its row of B (at most four entries for linear elements) in registers for
 // MAPC columns; neighbouring grid points gather from neighbouring nodes.
-constexpr int MAPC = 8;
+constexpr int MAPC = 8, MAPU = 4;
 template <class A, class V>
 __global__ void __launch_bounds__(256) grid_map_cm_kernel(GridDev G, int n, int k, int k0, const V* __restrict__ x0,
                                                           const V* __restrict__ x1, A* __restrict__ gm)
@@ -124,18 +124,37 @@ __global__ void __launch_bounds__(256) grid_map_cm_kernel(GridDev G, int n, int 
         col[j] = j < nj ? G.col[j0 + j] : 0;
         w[j] = j < nj ? (R)G.val[j0 + j] : (R)0;
     }
-    const int c1 = min(k, (int)(blockIdx.y + 1) * MAPC);
-    for (int c = blockIdx.y * MAPC; c < c1; c++) {
-        const V* x = c < k0 ? x0 + (size_t)c * n : x1 + (size_t)(c - k0) * n;
-        A acc = vzero<A>();
-        if (nj <= 4) {
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                if (j < nj) acc = vadd(acc, vscale(vcast<A, V>(x[col[j]]), w[j]));
-        } else {
+    const int c0 = blockIdx.y * MAPC, c1 = min(k, c0 + MAPC);
+    auto column = [&](int c) { return c < k0 ? x0 + (size_t)c * n : x1 + (size_t)(c - k0) * n; };
+    if (nj > 4) {
+        for (int c = c0; c < c1; c++) {
+            const V* x = column(c);
+            A acc = vzero<A>();
             for (int j = j0; j < j0 + nj; j++) acc = vadd(acc, vscale(vcast<A, V>(x[G.col[j]]), (R)G.val[j]));
+            gm[(size_t)c * G.glen + g] = acc;
         }
-        gm[(size_t)c * G.glen + g] = acc;
+        return;
+    }
+    // the gathers of MAPU columns are in flight together (a missing entry
+    // gathers node 0 and is not added)
+    for (int c = c0; c < c1; c += MAPU) {
+        V v[MAPU][4];
+#pragma unroll
+        for (int u = 0; u < MAPU; u++) {
+            const V* x = column(min(c + u, c1 - 1));
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[u][j] = x[col[j]];
+        }
+#pragma unroll
+        for (int u = 0; u < MAPU; u++) {
+            A acc = vzero<A>();
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const A t = vadd(acc, vscale(vcast<A, V>(v[u][j]), w[j]));
+                acc = j < nj ? t : acc;
+            }
+            if (c + u < c1) gm[(size_t)(c + u) * G.glen + g] = acc;
+        }
     }
 }
 
@@ -171,15 +190,32 @@ __global__ void __launch_bounds__(256) grid_planes_cm_kernel(GridDev G, int k, i
             if (bhi) hi[mk][d] = g + st[d];
             if ((blo && bhi) || (in && (blo || bhi))) w[mk][d] = (R)((blo && bhi ? 0.5 : 1.0) * G.ih[d]);
         }
-    const int c1 = min(k, (int)(blockIdx.y + 1) * MAPC);
-    for (int c = blockIdx.y * MAPC; c < c1; c++) {
-        const A* x = gm + (size_t)c * G.glen;
-        const int mk = (c < kmask || mask_rest) ? 1 : 0;
-        A* P = planes + (size_t)c * np * G.slen + s;
-        P[0] = x[g];
+    const int c0 = blockIdx.y * MAPC, c1 = min(k, c0 + MAPC);
+    for (int c = c0; c < c1; c += MAPU) {
+        A v[MAPU], vl[MAPU][3], vh[MAPU][3];
 #pragma unroll
-        for (int d = 0; d < 3; d++)
-            if (d < G.dim) P[(size_t)(d + 1) * G.slen] = vscale(vsub(x[hi[mk][d]], x[lo[mk][d]]), w[mk][d]);
+        for (int u = 0; u < MAPU; u++) {
+            const int cu = min(c + u, c1 - 1);
+            const bool mk = cu < kmask || mask_rest;
+            const A* x = gm + (size_t)cu * G.glen;
+            v[u] = x[g];
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                if (d < G.dim) {
+                    vl[u][d] = x[mk ? lo[1][d] : lo[0][d]];
+                    vh[u][d] = x[mk ? hi[1][d] : hi[0][d]];
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < MAPU; u++) {
+            if (c + u >= c1) break;
+            const bool mk = c + u < kmask || mask_rest;
+            A* P = planes + (size_t)(c + u) * np * G.slen + s;
+            P[0] = v[u];
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                if (d < G.dim) P[(size_t)(d + 1) * G.slen] = vscale(vsub(vh[u][d], vl[u][d]), mk ? w[1][d] : w[0][d]);
+        }
     }
 }
 
@@ -194,20 +230,26 @@ __device__ __forceinline__ cd cdiv_smith(cd a, cd b)
     return cd{(a.x * r + a.y) / den, (a.y * r - a.x) / den};
 }
 
-// The factor of each link's row: sc / y for log data (Smith's division for
-// complex y), sc for linear data (y null), in FP64, then cast to the
-// Jacobian's arithmetic type
+// One launch before the grid and element kernels: the factor of each link's
+// row, sc / y for log data (Smith's division for complex y), sc for linear
+// data (y null), formed in FP64 and cast to the Jacobian's arithmetic type;
+// and with x given the cast of the cnt0 source and cnt1 detector values into
+// it, one after the other (three launches of 2-4 us each as separate kernels).
 template <class C, class V64>
-__global__ void grid_yscale_kernel(int nqm, const V64* __restrict__ y, double sc, C* __restrict__ ysc)
+__global__ void grid_prep_kernel(size_t cnt0, const V64* __restrict__ x0, size_t cnt1, const V64* __restrict__ x1,
+                                 C* __restrict__ x, int nqm, const V64* __restrict__ y, double sc,
+                                 C* __restrict__ ysc)
 {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= nqm) return;
-    if constexpr (vt<V64>::cplx) {
-        const cd r = y ? cdiv_smith(cd{1.0, 0.0}, y[l]) : cd{1.0, 0.0};
-        ysc[l] = vcast<C, cd>(cd{r.x * sc, r.y * sc});
-    } else {
-        ysc[l] = vcast<C, double>(y ? sc / y[l] : sc);
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i < (size_t)nqm) {
+        if constexpr (vt<V64>::cplx) {
+            const cd r = y ? cdiv_smith(cd{1.0, 0.0}, y[i]) : cd{1.0, 0.0};
+            ysc[i] = vcast<C, cd>(cd{r.x * sc, r.y * sc});
+        } else {
+            ysc[i] = vcast<C, double>(y ? sc / y[i] : sc);
+        }
     }
+    if (x && i < cnt0 + cnt1) x[i] = vcast<C, V64>(i < cnt0 ? x0[i] : x1[i - cnt0]);
 }
 
 // J stores bypass L2 retention (evict-first), so the 2.4 GB stream of rows
@@ -215,29 +257,97 @@ __global__ void grid_yscale_kernel(int nqm, const V64* __restrict__ y, double sc
 __device__ __forceinline__ void st_stream(float* p, float v) { __stcs(p, v); }
 __device__ __forceinline__ void st_stream(double* p, double v) { __stcs(p, v); }
 
-// The links of a block's GQ sources for LT detectors at a time, in shared
-// memory: the link index (or -1) and its factor, read by every thread of the
-// block from there instead of from the pair table and the factor array
-// (element_jacobian_kernel: 4.10 -> 3.76 ms on the 3D cylinder; the grid
-// kernel, at 80 registers with it, lost as much at 48^3 as it gained at 32^3).
+// The links of a block's GQ sources and at most LT detectors in shared
+// memory: which sources link to the detector, the offset of the link's J row
+// and its factor, read by every thread of the block from there instead of from
+// the pair table and the factor array.
 constexpr int LT = 64;
 template <class V, int GQ>
 struct LinkTile {
-    int l[GQ][LT];
+    unsigned on[LT];
+    long long row[GQ][LT];
     V y[GQ][LT];
-    // detectors m0 .. m0 + LT - 1 of sources q0 .. q0 + GQ - 1; the caller
-    // syncs the block before (the previous tile's readers) and after
-    __device__ __forceinline__ void fill(int m0, int q0, int nq, int nm, const int* __restrict__ pair,
-                                         const V* __restrict__ ysc)
+    // detectors m0 .. m1 - 1 of sources q0 .. q0 + GQ - 1; rows of cols
+    // entries, the first of link l0
+    __device__ __forceinline__ void fill(int m0, int m1, int q0, int nq, int nm, const int* __restrict__ pair,
+                                         const V* __restrict__ ysc, long long cols, int l0)
     {
-        for (int i = threadIdx.x; i < GQ * LT; i += blockDim.x) {
-            const int g = i / LT, j = i % LT, m = m0 + j;
-            const int k = (m < nm && q0 + g < nq) ? pair[(size_t)(q0 + g) * nm + m] : -1;
-            l[g][j] = k;
-            y[g][j] = k >= 0 ? ysc[k] : vzero<V>();
+        for (int j = threadIdx.x; j < m1 - m0; j += blockDim.x) {
+            unsigned b = 0;
+            for (int g = 0; g < GQ && q0 + g < nq; g++) {
+                const int k = pair[(size_t)(q0 + g) * nm + m0 + j];
+                if (k < 0) continue;
+                b |= 1u << g;
+                row[g][j] = (k - l0) * cols;
+                y[g][j] = ysc[k];
+            }
+            on[j] = b;
         }
+        __syncthreads();
     }
 };
+
+// Sums of products f h of one link: F a source's value, H a detector's, both in
+// the form the sum takes.  Complex FP32 runs on packed pairs: the sums of
+// (hr, hr) f and (hi, hi) f, whose difference and sum cross-wise is the product
+// (a packed multiply-add is one instruction for two, and these kernels are
+// bound by instruction issue).
+template <class V>
+struct LinkSum {
+    using F = V;
+    using H = V;
+    V a = vzero<V>();
+    static __device__ __forceinline__ F src(V f) { return f; }
+    static __device__ __forceinline__ H det(V h) { return h; }
+    static __device__ __forceinline__ V prod(F f, H h) { return vmul(f, h); }
+    static __device__ __forceinline__ F sub(F a, F b) { return vsub(a, b); }
+    __device__ __forceinline__ void add(F f, H h) { a = vfma(a, f, h); }
+    __device__ __forceinline__ V get() const { return a; }
+};
+template <>
+struct LinkSum<cf> {
+    using F = unsigned long long;
+    struct H {
+        unsigned long long r, i;
+    };
+    unsigned long long p = 0ull, q = 0ull;
+    // one product alone: a rounding fewer, and no more instructions
+    static __device__ __forceinline__ cf prod(F f, H h)
+    {
+        const float2 a = f2_unpack(f);
+        return vmul(cf{a.x, a.y}, cf{f2_unpack(h.r).x, f2_unpack(h.i).x});
+    }
+    static __device__ __forceinline__ F src(cf f) { return f2_pack(f.x, f.y); }
+    static __device__ __forceinline__ H det(cf h) { return H{f2_pack(h.x, h.x), f2_pack(h.y, h.y)}; }
+    static __device__ __forceinline__ F sub(F a, F b) { return f2_sub(a, b); }
+    __device__ __forceinline__ void add(F f, H h)
+    {
+        p = f2_fma(h.r, f, p);
+        q = f2_fma(h.i, f, q);
+    }
+    __device__ __forceinline__ cf get() const
+    {
+        const float2 a = f2_unpack(p), b = f2_unpack(q);
+        return cf{a.x - b.y, a.y + b.x};
+    }
+};
+
+// the four (real: two) J entries of a link at column e of rows row and row +
+// half: mua in the first, kappa in the second half of the columns
+template <class V, class JT>
+__device__ __forceinline__ void put_link(JT* __restrict__ j0, long long row, long long half, long long kap, V pm, V pk)
+{
+    JT* r = j0 + row;
+    if constexpr (vt<V>::cplx) {
+        st_stream(r, (JT)re(pm));
+        st_stream(r + kap, (JT)re(pk));
+        st_stream(r + half, (JT)im(pm));
+        st_stream(r + half + kap, (JT)im(pk));
+    } else {
+        st_stream(r, (JT)pm);
+        st_stream(r + half, (JT)pk);
+    }
+}
 
 // One thread per (solution point, group of GQ sources): the sources' planes
 // stay in registers while the detectors' planes stream past, each loaded once
@@ -252,58 +362,59 @@ struct LinkTile {
 // and [Im mua | Im kap] at nQM + l (2 slen columns); real mua at l and kap at
 // nQM + l (slen).  With l0 > 0 the kernel serves the sources of one chunk
 // whose links are l0 .. l0 + nqm - 1: row l - l0 and nqm + l - l0.
+// blockIdx.z: chunks of mc detectors, at most LT.
+// FP32 is bound by the plane loads' latency and the J stream (32^3 points, 80 x
+// 80 links, 2.4 GB: 455 us, 5.3 TB/s of the 7.6 a plain write stream reaches;
+// groups of 4 and 256 threads 480, of 8 and 256 470), FP64 by its pipe (7
+// products an entry pair: 6.5 ms, of which the products take 6.2).  8 sources a
+// group for FP32: half the plane loads of 4; 4 for FP64: 8 leaves one warp in
+// two idle at medium sizes (disc 40^2, 15 x 17: 79 -> 98 us).  Two points a
+// thread on packed pairs halve the instructions but lose (FP32 complex 577 ->
+// 967 us: eight store streams a warp).
 template <class V, class JT, int GQ, int NP>
-__global__ void __launch_bounds__(256) grid_jacobian_kernel(int slen, int nq, int nm, int nqm, const V* __restrict__ Fp,
+__global__ void __launch_bounds__(128) grid_jacobian_kernel(int slen, int nq, int nm, int nqm, const V* __restrict__ Fp,
                                                             const V* __restrict__ Ap, const int* __restrict__ pair,
-                                                            const V* __restrict__ ysc, JT* __restrict__ J, int l0)
+                                                            const V* __restrict__ ysc, JT* __restrict__ J, int l0,
+                                                            int mc)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x, q0 = blockIdx.y * GQ;
+    using LS = LinkSum<V>;
+    __shared__ LinkTile<V, GQ> tile;
+    const int q0 = blockIdx.y * GQ, m0 = blockIdx.z * mc, m1 = min(m0 + mc, nm);
+    constexpr bool CPLX = vt<V>::cplx;
+    const long long cols = CPLX ? 2 * (long long)slen : (long long)slen, half = nqm * cols;
+    tile.fill(m0, m1, q0, nq, nm, pair, ysc, cols, l0);
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= slen) return;
-    V f[GQ][NP];
+    typename LS::F f[GQ][NP];
 #pragma unroll
     for (int g = 0; g < GQ; g++)
 #pragma unroll
-        for (int d = 0; d < NP; d++) f[g][d] = Fp[((size_t)min(q0 + g, nq - 1) * NP + d) * slen + s];
-    constexpr bool CPLX = vt<V>::cplx;
-    const size_t cols = CPLX ? 2 * (size_t)slen : (size_t)slen;
+        for (int d = 0; d < NP; d++) f[g][d] = LS::src(Fp[((size_t)min(q0 + g, nq - 1) * NP + d) * slen + s]);
+    JT* j0 = J + s;
     V an[NP];
+    const V* ap = Ap + (size_t)m0 * NP * slen + s;
 #pragma unroll
-    for (int d = 0; d < NP; d++) an[d] = Ap[(size_t)d * slen + s];
-    for (int m = 0; m < nm; m++) {
-        V a[NP];
+    for (int d = 0; d < NP; d++) an[d] = ap[(size_t)d * slen];
+    for (int m = m0; m < m1; m++) {
+        const int jt = m - m0;
+        const unsigned on = tile.on[jt];
+        typename LS::H a[NP];
+        ap += (size_t)NP * slen;
 #pragma unroll
         for (int d = 0; d < NP; d++) {
-            a[d] = an[d];
-            if (m + 1 < nm) an[d] = Ap[((size_t)(m + 1) * NP + d) * slen + s];
+            a[d] = LS::det(an[d]);
+            if (m + 1 < m1) an[d] = ap[(size_t)d * slen];
         }
-        int lk[GQ];
-        bool any = false;
+        if (!on) continue;
 #pragma unroll
         for (int g = 0; g < GQ; g++) {
-            lk[g] = q0 + g < nq ? pair[(size_t)(q0 + g) * nm + m] : -1;
-            any |= lk[g] >= 0;
-        }
-        if (!any) continue;
+            if (!(on >> g & 1)) continue;
+            LS pk;
+            const V pm = LS::prod(f[g][0], a[0]);
 #pragma unroll
-        for (int g = 0; g < GQ; g++) {
-            const int l = lk[g];
-            if (l < 0) continue;
-            const V y = ysc[l];
-            V t = vmul(f[g][1], a[1]);
-#pragma unroll
-            for (int d = 2; d < NP; d++) t = vfma(t, f[g][d], a[d]);
-            const V pm = vmul(vmul(f[g][0], a[0]), y), pk = vmul(t, y);
-            JT* r0 = J + (size_t)(l - l0) * cols + s;
-            JT* r1 = J + (size_t)(l - l0 + nqm) * cols + s;
-            if constexpr (CPLX) {
-                st_stream(r0, (JT)re(pm));
-                st_stream(r1, (JT)im(pm));
-                st_stream(r0 + slen, (JT)re(pk));
-                st_stream(r1 + slen, (JT)im(pk));
-            } else {
-                st_stream(r0, (JT)pm);
-                st_stream(r1, (JT)pk);
-            }
+            for (int d = 1; d < NP; d++) pk.add(f[g][d], a[d]);
+            const V y = tile.y[g][jt];
+            put_link<V, JT>(j0, tile.row[g][jt], half, slen, vmul(pm, y), vmul(pk.get(), y));
         }
     }
 }
@@ -311,102 +422,111 @@ __global__ void __launch_bounds__(256) grid_jacobian_kernel(int slen, int nq, in
 // Element-basis Jacobian (GenerateJacobian_mesh with elbasis, jacobian.cc:
 // 441-497; CW 738-802 and the LOG scaling 178-193), with IntFG_el /
 // IntGradFGradG_el (884-939): per element e and link (q, m),
-// sum_ij f_i g_j IntFF(i,j) and sum_ij f_i g_j IntDD(i,j), formed as
-// sum_i f_i h_i with h = W g once per (element, detector) and shared by the
-// group's GQ sources.  IntFF(i,j) = size (1 + [i = j]) / 12 (triangles) or
-// / 20 (tetrahedra), so h_i = size / 12 (or 20) (a_i + sum_j a_j).  NN nodes
-// per element (3 or 4).  Fields source-major in the natural numbering.
-// ysc[l] = -1 / y for LOG data, -1 for LINEAR.  J: complex (2 nQM) x (2 ne)
-// rows -Re / -Im, kappa at column ne + e; real (2 nQM) x ne [mua ; kappa].
+// sum_ij f_i g_j IntFF(i,j) and sum_ij f_i g_j IntDD(i,j).  With h = IntFF g
+// (size (1 + [i = j]) / 12 for triangles, / 20 for tetrahedra) the first is
+// sum_i f_i h_i; the rows and columns of IntDD sum to zero, so with the
+// differences d_i = f_i - f_0 the second is
+// sum_{i,j > 0} d_i IntDD(i,j) (g_j - g_0): no cancellation between its terms
+// (FP32, error in L2 against FP64: 61-ring disc 5.4e-7 -> 0.9e-7), and NN - 1
+// products.  FP64 keeps the d_i and forms the first sum from them too, f_0
+// sum_i h_i + sum_{i > 0} d_i h_i: subtractions per link would cost its pipe a
+// sixth.  The detector's side is formed once per (element, detector) and shared
+// by the group's GQ sources.
+// NN nodes per element (3 or 4).  Fields source-major in the natural
+// numbering.  ysc[l] = -1 / y for LOG data, -1 for LINEAR.  J: complex
+// (2 nQM) x (2 ne) rows -Re / -Im, kappa at column ne + e; real (2 nQM) x ne
+// [mua ; kappa].
+// blockIdx.z: chunks of mc detectors, at most LT.
+// FP32 is bound by instruction issue, then by the J stream (38.9k tetrahedra,
+// 80 x 80 links, 4 GB: 838 -> 734 us a call, 5.4 TB/s), FP64 by its pipe (21.1
+// -> 17.6 ms; 9 complex products a link are 15.4).  8 sources a group: the detector's
+// side costs as much as 4 links (groups of 4 / 6 / 8: 960 / 810 / 726 us FP32,
+// 20.1 / 18.5 / 17.6 ms FP64).
 template <class V, class JT, int GQ, int NN>
-__global__ void __launch_bounds__(256) element_jacobian_kernel(MeshDev m, int nq, int nm, int nqm,
+__global__ void __launch_bounds__(128) element_jacobian_kernel(MeshDev m, int nq, int nm, int nqm,
                                                                const V* __restrict__ F, const V* __restrict__ A,
                                                                const int* __restrict__ pair,
-                                                               const V* __restrict__ ysc, JT* __restrict__ J)
+                                                               const V* __restrict__ ysc, JT* __restrict__ J,
+                                                               int mc)
 {
+    using LS = LinkSum<V>;
     __shared__ LinkTile<V, GQ> tile;
-    const int q0 = blockIdx.y * GQ;
-    // threads past ne take part in the tile fills only
-    const bool act = blockIdx.x * blockDim.x + threadIdx.x < m.ne;
-    const int e = min((int)(blockIdx.x * blockDim.x + threadIdx.x), m.ne - 1);
+    const int q0 = blockIdx.y * GQ, m0 = blockIdx.z * mc, m1 = min(m0 + mc, nm);
+    constexpr bool CPLX = vt<V>::cplx;
+    const long long cols = CPLX ? 2 * (long long)m.ne : (long long)m.ne, half = nqm * cols;
+    tile.fill(m0, m1, q0, nq, nm, pair, ysc, cols, 0);
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= m.ne) return;
     using R = typename vt<V>::R;
     const int n = m.n;
     const int* nd = m.el + (size_t)e * NN;
     const double* r = m.rec + (size_t)e * EL_REC;
-    const R cff = (R)((NN == 3 ? 1.0 / 12.0 : 1.0 / 20.0) * r[0]);
-    R wdd[NN][NN];
+    constexpr double ff = NN == 3 ? 1.0 / 12.0 : 1.0 / 20.0;
+    const R cff = (R)(ff * r[0]), cf0 = (R)(ff * (NN + 1) * r[0]);
+    R wdd[NN - 1][NN - 1];
     int node[NN];
 #pragma unroll
-    for (int i = 0; i < NN; i++) {
-        node[i] = nd[i];
+    for (int i = 0; i < NN; i++) node[i] = nd[i];
 #pragma unroll
-        for (int j = 0; j < NN; j++)
+    for (int i = 1; i < NN; i++)
+#pragma unroll
+        for (int j = 1; j < NN; j++)
             // IntDD: the record's value for triangles, 4 x it for tetrahedra
-            wdd[i][j] = (R)((NN == 4 ? 4.0 : 1.0) * r[1 + i * NN + j]);
+            wdd[i - 1][j - 1] = (R)((NN == 4 ? 4.0 : 1.0) * r[1 + i * NN + j]);
+    constexpr bool DIFF = sizeof(JT) == 8;
+    typename LS::F f[GQ][NN];
+#pragma unroll
+    for (int g = 0; g < GQ; g++) {
+        const V* x = F + (size_t)min(q0 + g, nq - 1) * n;
+        const V x0 = x[node[0]];
+        f[g][0] = LS::src(x0);
+#pragma unroll
+        for (int i = 1; i < NN; i++) f[g][i] = LS::src(DIFF ? vsub(x[node[i]], x0) : x[node[i]]);
     }
-    V f[GQ][NN];
-#pragma unroll
-    for (int g = 0; g < GQ; g++)
-#pragma unroll
-        for (int i = 0; i < NN; i++) f[g][i] = F[(size_t)min(q0 + g, nq - 1) * n + node[i]];
-    constexpr bool CPLX = vt<V>::cplx;
-    const size_t cols = CPLX ? 2 * (size_t)m.ne : (size_t)m.ne;
+    JT* j0 = J + e;
     // the next detector's nodal values load while this one's entries form
     V an[NN];
+    const V* ap = A + (size_t)m0 * n;
 #pragma unroll
-    for (int j = 0; j < NN; j++) an[j] = A[node[j]];
-    for (int mm = 0; mm < nm; mm++) {
-        const int jt = mm % LT;
-        if (jt == 0) {
-            __syncthreads();
-            tile.fill(mm, q0, nq, nm, pair, ysc);
-            __syncthreads();
-        }
+    for (int j = 0; j < NN; j++) an[j] = ap[node[j]];
+    for (int mm = m0; mm < m1; mm++) {
+        const int jt = mm - m0;
+        const unsigned on = tile.on[jt];
         V a[NN];
+        ap += n;
 #pragma unroll
         for (int j = 0; j < NN; j++) {
             a[j] = an[j];
-            if (mm + 1 < nm) an[j] = A[(size_t)(mm + 1) * n + node[j]];
+            if (mm + 1 < m1) an[j] = ap[node[j]];
         }
-        bool any = false;
+        if (!on) continue;
+        // h_i = cff (g_i + sum_j g_j); sum_i h_i = cff (NN + 1) sum_j g_j
+        typename LS::H hm[NN], hk[NN - 1];
+        V sa = a[0];
 #pragma unroll
-        for (int g = 0; g < GQ; g++) any |= tile.l[g][jt] >= 0;
-        if (!any || !act) continue;
-        V hm[NN], hk[NN];
-        V sa = vzero<V>();
+        for (int j = 1; j < NN; j++) sa = vadd(sa, a[j]);
+        hm[0] = LS::det(DIFF ? vscale(sa, cf0) : vscale(vadd(sa, a[0]), cff));
 #pragma unroll
-        for (int j = 0; j < NN; j++) sa = vadd(sa, a[j]);
+        for (int i = 1; i < NN; i++) hm[i] = LS::det(vscale(vadd(sa, a[i]), cff));
 #pragma unroll
-        for (int i = 0; i < NN; i++) {
-            hm[i] = vscale(vadd(sa, a[i]), cff);
-            hk[i] = vscale(a[0], wdd[i][0]);
+        for (int j = 1; j < NN; j++) a[j] = vsub(a[j], a[0]);
 #pragma unroll
-            for (int j = 1; j < NN; j++) hk[i] = vadd(hk[i], vscale(a[j], wdd[i][j]));
+        for (int i = 0; i < NN - 1; i++) {
+            V h = vscale(a[1], wdd[i][0]);
+#pragma unroll
+            for (int j = 1; j < NN - 1; j++) h = vadd(h, vscale(a[j + 1], wdd[i][j]));
+            hk[i] = LS::det(h);
         }
 #pragma unroll
         for (int g = 0; g < GQ; g++) {
-            const int l = tile.l[g][jt];
-            if (l < 0) continue;
-            V pm = vmul(f[g][0], hm[0]), pk = vmul(f[g][0], hk[0]);
+            if (!(on >> g & 1)) continue;
+            LS pm, pk;
 #pragma unroll
-            for (int i = 1; i < NN; i++) {
-                pm = vfma(pm, f[g][i], hm[i]);
-                pk = vfma(pk, f[g][i], hk[i]);
-            }
+            for (int i = NN - 1; i >= 0; i--) pm.add(f[g][i], hm[i]);
+#pragma unroll
+            for (int i = 0; i < NN - 1; i++) pk.add(DIFF ? f[g][i + 1] : LS::sub(f[g][i + 1], f[g][0]), hk[i]);
             const V y = tile.y[g][jt];
-            pm = vmul(pm, y);
-            pk = vmul(pk, y);
-            JT* r0 = J + (size_t)l * cols;
-            JT* r1 = J + (size_t)(l + nqm) * cols;
-            if constexpr (CPLX) {
-                st_stream(r0 + e, (JT)re(pm));
-                st_stream(r1 + e, (JT)im(pm));
-                st_stream(r0 + m.ne + e, (JT)re(pk));
-                st_stream(r1 + m.ne + e, (JT)im(pk));
-            } else {
-                st_stream(r0 + e, (JT)pm);
-                st_stream(r1 + e, (JT)pk);
-            }
+            put_link<V, JT>(j0, tile.row[g][jt], half, m.ne, vmul(pm.get(), y), vmul(pk.get(), y));
         }
     }
 }

@@ -3033,6 +3033,29 @@ static void api_jacobian(tg_solver s, int nq, const double* dphi, int nm, const 
 // GenerateJacobian_cw_grid, 516-712, and the LOG scaling of
 // GenerateJacobian_cw, 178-193).  Fields are source-major in the natural
 // numbering; FP64 arithmetic for an FP64 J, FP32 for an FP32 J.
+template <class C, class V64>
+static void grid_prep(tg_solver s, int nq, const V64* F, int nm, const V64* A, C* x, int nqm, const V64* y, double sc,
+                      C* ysc)
+{
+    const size_t n = s->mesh->d.n, cnt = x ? (size_t)(nq + nm) * n : 0;
+    launch(grid_prep_kernel<C, V64>, cdiv_u(std::max<size_t>(cnt, nqm), 256), 256, 0, s->stream, nq * n, F, nm * n, A,
+           x, nqm, y, sc, ysc);
+}
+
+// Detectors per block of the grid and element Jacobian kernels, for a grid of
+// so many blocks a chunk: no more than a tile holds, and where the blocks leave
+// SMs idle fewer, down to 4 (a block's sources are loaded once per chunk; 1216
+// = 152 SMs x 8 blocks).  FP64, 100 MHz, one chunk against this rule: disc with
+// 40^2 pixels and 15 x 17 links 149 -> 79 us, 61-ring disc with 31 x 33 232 ->
+// 174 us, 24^3 with 40 x 41 947 -> 784 us; 1216 / 2432 / 4864 blocks within the
+// runs' difference but for FP32 elements (2D, 31 x 33: 87 / 92 / 96 us).
+static int detector_chunk(int nm, size_t blocks)
+{
+    const size_t want = cdiv_u(1216, std::max<size_t>(1, blocks));
+    const size_t chunks = std::max<size_t>(1, std::min<size_t>(want, cdiv_u(nm, 4)));
+    return std::max(1, std::min(LT, (int)cdiv_u(nm, chunks)));
+}
+
 template <class V64, class C>
 static void grid_jac_run(tg_solver s, const tg_raster_s& r, int nq, const V64* F, int nm, const V64* A,
                          const V64* yl, const LinkHost& L, int logscale, void* Jd)
@@ -3048,37 +3071,36 @@ static void grid_jac_run(tg_solver s, const tg_raster_s& r, int nq, const V64* F
     // adjoint gradient for complex data only (jacobian.cc:348-350 against 557)
     C* gm = (C*)s->io_c.ensure((size_t)r.glen * k * sizeof(C));
     C* P = (C*)s->gplanes_q.ensure((size_t)k * np * r.gslen * sizeof(C));
+    C* ysc = (C*)s->gy.ensure((size_t)nqm * sizeof(C));
     const dim3 mg(cdiv_u(r.glen, 256), cdiv_u(k, MAPC));
     if constexpr (std::is_same<C, V64>::value) {
+        grid_prep<C, V64>(s, nq, F, nm, A, nullptr, nqm, logscale ? yl : nullptr, -r.voxel(), ysc);
         launch(grid_map_cm_kernel<C, V64>, mg, 256, 0, s->stream, G, n, k, nq, F, A, gm);
     } else {
         C* X = (C*)s->tmp.ensure((size_t)k * n * sizeof(C));
-        launch(cast_kernel<C, V64>, cdiv_u((size_t)nq * n, 256), 256, 0, s->stream, (size_t)nq * n, F, X);
-        launch(cast_kernel<C, V64>, cdiv_u((size_t)nm * n, 256), 256, 0, s->stream, (size_t)nm * n, A,
-               X + (size_t)nq * n);
+        grid_prep<C, V64>(s, nq, F, nm, A, X, nqm, logscale ? yl : nullptr, -r.voxel(), ysc);
         launch(grid_map_cm_kernel<C, C>, mg, 256, 0, s->stream, G, n, k, nq, (const C*)X,
                (const C*)(X + (size_t)nq * n), gm);
     }
     launch(grid_planes_cm_kernel<C>, dim3(cdiv_u(r.gslen, 256), cdiv_u(k, MAPC)), 256, 0, s->stream, G, k, nq,
            vt<V64>::cplx ? 1 : 0, (const C*)gm, P);
-    C* ysc = (C*)s->gy.ensure((size_t)nqm * sizeof(C));
-    launch(grid_yscale_kernel<C, V64>, cdiv_u(nqm, 256), 256, 0, s->stream, nqm, logscale ? yl : nullptr, -r.voxel(),
-           ysc);
     using JT = typename vt<C>::R;
-    constexpr int GQ = 4, TB = 256;
+    constexpr int GQ = sizeof(JT) == 4 ? 8 : 4, TB = 128;
     const C* Pm = P + (size_t)nq * np * r.gslen;
     // the rows of the links l0 .. l0 + nqmc - 1 of sources q0 .. q0 + nqc - 1
     // on the grid points inside the mesh
     auto rows = [&](int q0, int nqc, int l0, int nqmc, JT* out) {
-        const dim3 jg(cdiv_u(r.gslen, TB), cdiv_u(nqc, GQ));
+        const unsigned jx = cdiv_u(r.gslen, TB), jy = cdiv_u(nqc, GQ);
+        const int mc = detector_chunk(nm, (size_t)jx * jy);
+        const dim3 jg(jx, jy, cdiv_u(nm, mc));
         const C* Pq = P + (size_t)q0 * np * r.gslen;
         const int* pq = pr + (size_t)q0 * nm;
         if (r.dim == 3)
             launch(grid_jacobian_kernel<C, JT, GQ, 4>, jg, TB, 0, s->stream, r.gslen, nqc, nm, nqmc, Pq, Pm, pq,
-                   (const C*)ysc, out, l0);
+                   (const C*)ysc, out, l0, mc);
         else
             launch(grid_jacobian_kernel<C, JT, GQ, 3>, jg, TB, 0, s->stream, r.gslen, nqc, nm, nqmc, Pq, Pm, pq,
-                   (const C*)ysc, out, l0);
+                   (const C*)ysc, out, l0, mc);
     };
     if (!r.hasG) {
         rows(0, nq, 0, nqm, (JT*)Jd);
@@ -3148,25 +3170,25 @@ static void element_jac_run(tg_solver s, int nq, const V64* F, int nm, const V64
     const int n = m.n, nqm = (int)L.q.size();
     const int* pr = links_pair_to_device(s, L);
     const C *Fc = (const C*)F, *Ac = (const C*)A;
+    C* x = nullptr;
     if constexpr (!std::is_same<C, V64>::value) {
-        C* f = (C*)s->gplanes_q.ensure((size_t)nq * n * sizeof(C));
-        C* a = (C*)s->gplanes_m.ensure((size_t)nm * n * sizeof(C));
-        launch(cast_kernel<C, V64>, cdiv_u((size_t)nq * n, 256), 256, 0, s->stream, (size_t)nq * n, F, f);
-        launch(cast_kernel<C, V64>, cdiv_u((size_t)nm * n, 256), 256, 0, s->stream, (size_t)nm * n, A, a);
-        Fc = f;
-        Ac = a;
+        x = (C*)s->gplanes_q.ensure((size_t)(nq + nm) * n * sizeof(C));
+        Fc = x;
+        Ac = x + (size_t)nq * n;
     }
     C* ysc = (C*)s->gy.ensure((size_t)nqm * sizeof(C));
-    launch(grid_yscale_kernel<C, V64>, cdiv_u(nqm, 256), 256, 0, s->stream, nqm, logscale ? yl : nullptr, -1.0, ysc);
+    grid_prep<C, V64>(s, nq, F, nm, A, x, nqm, logscale ? yl : nullptr, -1.0, ysc);
     using JT = typename vt<C>::R;
-    constexpr int GQ = 6, TB = 128;
-    const dim3 eg(cdiv_u(m.ne, TB), cdiv_u(nq, GQ));
+    constexpr int GQ = 8, TB = 128;
+    const unsigned ex = cdiv_u(m.ne, TB), ey = cdiv_u(nq, GQ);
+    const int mc = detector_chunk(nm, (size_t)ex * ey);
+    const dim3 eg(ex, ey, cdiv_u(nm, mc));
     if (m.dim == 3)
         launch(element_jacobian_kernel<C, JT, GQ, 4>, eg, TB, 0, s->stream, m, nq, nm, nqm, Fc, Ac, (const int*)pr,
-               (const C*)ysc, (JT*)Jd);
+               (const C*)ysc, (JT*)Jd, mc);
     else
         launch(element_jacobian_kernel<C, JT, GQ, 3>, eg, TB, 0, s->stream, m, nq, nm, nqm, Fc, Ac, (const int*)pr,
-               (const C*)ysc, (JT*)Jd);
+               (const C*)ysc, (JT*)Jd, mc);
 }
 
 template <class V64, class V32>
