@@ -364,11 +364,12 @@ __device__ __forceinline__ void put_link(JT* __restrict__ j0, long long row, lon
 // whose links are l0 .. l0 + nqm - 1: row l - l0 and nqm + l - l0.
 // blockIdx.z: chunks of mc detectors, at most LT.
 // FP32 is bound by the plane loads' latency and the J stream (32^3 points, 80 x
-// 80 links, 2.4 GB: 455 us, 5.3 TB/s of the 7.6 a plain write stream reaches;
-// groups of 4 and 256 threads 480, of 8 and 256 470), FP64 by its pipe (7
-// products an entry pair: 6.5 ms, of which the products take 6.2).  8 sources a
-// group for FP32: half the plane loads of 4; 4 for FP64: 8 leaves one warp in
-// two idle at medium sizes (disc 40^2, 15 x 17: 79 -> 98 us).  Two points a
+// 80 links, 2.4 GB: 644 -> 578 us a call; this kernel for 40 x 80 252 -> 241 us,
+// 5 TB/s of the 7.6 a plain write stream reaches, with 82 -> 56 instructions a
+// link; groups of 4 and 256 threads 256 us), FP64 by its pipe (6 complex
+// products a link: 6.5 ms, of which they take about 6.2).  8 sources a group for
+// FP32: half the plane loads of 4; 4 for FP64, where 8 leaves SMs idle at medium
+// sizes (disc 40^2, 15 x 17: 79 -> 98 us a call).  Two points a
 // thread on packed pairs halve the instructions but lose (FP32 complex 577 ->
 // 967 us: eight store streams a warp).
 template <class V, class JT, int GQ, int NP>

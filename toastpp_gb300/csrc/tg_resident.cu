@@ -744,9 +744,11 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
 // level writes (its rows, columns, factor entries, right-hand sides, pivots)
 // loads before that barrier, so that after it a row is shared-memory reads and
 // its sum.  (Loading it a whole level ahead, in a second register set, was
-// slower: FP64 issue bounds a level, not these loads.)  The rows of a level lie
-// by their number of entries, so that a warp's rows end together.  Every row's sum runs in the same order as in the level kernels:
-// the results are the same to the bit.
+// slower: the barriers and each row's serial FP64 sum bound a level, not these
+// loads; the FP64 pipe is a quarter busy.)  The rows of a level lie
+// by their number of entries, so that a warp's rows end together.  Every row's
+// sum runs in the same order as in the level kernels: the results are the same
+// to the bit.
 // ---------------------------------------------------------------------------
 template <class V, int LV>
 __global__ void __launch_bounds__(IC_NT) ic_cluster_kernel(IcClArgs<V> a)
