@@ -656,6 +656,11 @@ static void gather_maps(MeshHost& m)
         }
 }
 
+// cudaMemcpy from pageable memory returns once the data is staged, and the
+// solvers' streams do not wait for the legacy stream that carries it: whoever
+// uploads waits here before the data is handed on.
+static void uploads_done() { TG_CUDA(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 template <class T>
 static T* upload(const std::vector<T>& v)
 {
@@ -753,6 +758,7 @@ const PartDev* Mesh::part(int cs)
     P->ct = upload(ct);
     P->pofs = upload(pofs);
     P->push = upload(push);
+    uploads_done();
     P->copies = std::move(places);
     const PartDev* p = P.get();
     parts[cs] = std::move(P);
@@ -833,6 +839,7 @@ const IcPartDev* Mesh::ic_part(int cs, int o)
     };
     sweep(true, I->f);
     sweep(false, I->b);
+    uploads_done();
     const IcPartDev* p = I.get();
     ic_parts[{cs, o}] = std::move(I);
     return p;
@@ -924,6 +931,7 @@ Mesh* mesh_build(int dim, int n, const double* coords, int ne, const int* el)
         g.bwd_ell_col = upload(c.bwd_ell_col);
         g.bwd_ell_src = upload(c.bwd_ell_src);
     }
+    uploads_done();
     return M;
 }
 

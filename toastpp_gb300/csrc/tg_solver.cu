@@ -1877,7 +1877,11 @@ template <class T>
 void upload_sync(DBuf& b, const std::vector<T>& v)
 {
     void* p = b.ensure(std::max<size_t>(1, v.size()) * sizeof(T));
-    if (!v.empty()) TG_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    if (v.empty()) return;
+    TG_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    // (from pageable memory the copy may still be under way, on the legacy
+    // stream, which the solvers' streams do not wait for)
+    TG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
 }
 
 }  // namespace
