@@ -223,6 +223,7 @@ struct ResCols {
     float bn[CL_MAXCG], err[CL_MAXCG], fs[CL_MAXCG], thr[CL_MAXCG], trig[CL_MAXCG];
     double bnorm[CL_MAXCG], oerr[CL_MAXCG], scale[CL_MAXCG], berr[CL_MAXCG];
     int outer[CL_MAXCG], on[CL_MAXCG], rel[CL_MAXCG], its[CL_MAXCG], st[CL_MAXCG], ost[CL_MAXCG], nupd[CL_MAXCG], met[CL_MAXCG];
+    int fail[CL_MAXCG];  // the column ended short of its bounds for another reason than the iteration limit
 };
 
 template <class V64, class V, int LV>
@@ -394,7 +395,7 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
         S.outer[c] = S.on[c] = on;
         S.scale[c] = pow2_floor(er);
         S.bn[c] = S.err[c] = (float)(er / S.scale[c]);
-        S.rel[c] = S.its[c] = S.st[c] = S.ost[c] = S.nupd[c] = S.met[c] = 0;
+        S.rel[c] = S.its[c] = S.st[c] = S.ost[c] = S.nupd[c] = S.met[c] = S.fail[c] = 0;
         S.trig[c] = a.trig;
         S.alpha[c] = S.beta[c] = S.zr[c] = vzero<V>();
     }
@@ -648,6 +649,7 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
             } else if (limit || ++S.nupd[c] >= a.max_upd || !isfinite(er)) {
                 S.outer[c] = S.on[c] = S.rel[c] = 0;
                 S.ost[c] = 1;
+                S.fail[c] = !limit || !isfinite(er);
             } else {
                 // a true residual above the recursive one: the process no longer
                 // follows the FP64 system and restarts from it.  (Off the rounding
@@ -728,6 +730,7 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
         O.berr = S.berr[tid];
         O.its = S.its[tid];
         O.status = S.outer[tid] ? 1 : S.ost[tid];
+        O.rel = S.fail[tid];
         O.active = 0;
     }
     cl_sync(cs);

@@ -2515,15 +2515,17 @@ static ClShape resident_shape(tg_solver s, int k)
     return best;
 }
 
-// Columns that ended without reaching their bounds for another reason than
-// the iteration limit
+// Whether a column ended short of its bounds for another reason than the
+// iteration limit (ColState::rel as the resident kernel leaves it; the limit
+// counts the cluster's iterations, so a column that waited for a correction
+// may end at it with fewer of its own)
 static __global__ void resident_failed_kernel(int k, const ColState* __restrict__ co, int* __restrict__ out)
 {
     __shared__ int f;
     if (threadIdx.x == 0) f = 0;
     __syncthreads();
     for (int c = threadIdx.x; c < k; c += blockDim.x)
-        if (co[c].status != 0 && co[c].its < co[c].maxit) atomicOr(&f, 1);
+        if (co[c].rel) atomicOr(&f, 1);
     __syncthreads();
     if (threadIdx.x == 0) *out = f;
 }
