@@ -1519,6 +1519,16 @@ __global__ void gather_cols_kernel(int n, int k, int kf, const int* __restrict__
     dst[t] = src[i * k + idx[j]];
 }
 
+// dst columns idx (n x k) = src (n x kf)
+template <class V>
+__global__ void scatter_cols_kernel(int n, int k, int kf, const int* __restrict__ idx, const V* __restrict__ src,
+                                    V* __restrict__ dst)
+{
+    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (size_t)n * kf) return;
+    dst[t / kf * k + idx[t % kf]] = src[t];
+}
+
 // r[:, idx] = b[:, idx] - ax (ax: n x kf)
 template <class V>
 __global__ void scatter_resid_kernel(int n, int k, int kf, const int* __restrict__ idx, const V* __restrict__ b,

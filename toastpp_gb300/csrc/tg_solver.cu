@@ -1955,6 +1955,7 @@ struct tg_solver_s {
     bool res_ready = false;    // and the resident solve's matrices
     std::map<int, ClShape> shapes;  // by number of columns
     DBuf sa32, sg32, st32, xff, xkeep;  // resident solve: sliced matrices, split solution, kept guess
+    DBuf fb_idx, fb_b, fb_x, fb_cs;     // and the block of its failed columns
     DBuf val64, val32, L64, L32, dinv64, dinv32, idiag64, idiag32, params;
     DBuf ef64, eb64, ef32, eb32;  // factor values in the level ELL layouts
     Engine<double> er64;
@@ -2515,19 +2516,12 @@ static ClShape resident_shape(tg_solver s, int k)
     return best;
 }
 
-// Whether a column ended short of its bounds for another reason than the
-// iteration limit (ColState::rel as the resident kernel leaves it; the limit
-// counts the cluster's iterations, so a column that waited for a correction
-// may end at it with fewer of its own)
-static __global__ void resident_failed_kernel(int k, const ColState* __restrict__ co, int* __restrict__ out)
+// the failed columns' results (rel_compact_kernel's list) into the block's
+static __global__ void resident_results_kernel(int kf, const int* __restrict__ idx, const ColState* __restrict__ cf,
+                                               ColState* __restrict__ co)
 {
-    __shared__ int f;
-    if (threadIdx.x == 0) f = 0;
-    __syncthreads();
-    for (int c = threadIdx.x; c < k; c += blockDim.x)
-        if (co[c].rel) atomicOr(&f, 1);
-    __syncthreads();
-    if (threadIdx.x == 0) *out = f;
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < kf) co[idx[j]] = cf[j];
 }
 
 // the shape for k columns, chosen at their first solve
@@ -2542,10 +2536,14 @@ static const ClShape& shape_of(tg_solver s, int k)
     return it->second;
 }
 
-// The resident solve of k columns (R: the residual of a nonzero guess);
-// false: some column failed, X is to be restored and solved otherwise
+// The resident solve of k columns (R: the residual of a nonzero guess); the
+// number of columns that ended short of their bounds for another reason than
+// the iteration limit (a breakdown, or too many corrections), listed in
+// rel_idx.  (ColState::rel as the kernel leaves it; the limit counts the
+// cluster's iterations, so a column that waited for a correction may end at it
+// with fewer of its own.)
 template <class V64, class V32>
-static bool solve_resident(tg_solver s, int k, const V64* B, V64* X, ColState* co, V64* R, int maxit, bool zero_guess)
+static int solve_resident(tg_solver s, int k, const V64* B, V64* X, ColState* co, V64* R, int maxit, bool zero_guess)
 {
     const MeshDev& m = s->mesh->d;
     const ClShape& sh = shape_of<V64, V32>(s, k);
@@ -2572,11 +2570,15 @@ static bool solve_resident(tg_solver s, int k, const V64* B, V64* X, ColState* c
         launch_cluster(resident_kernel<V64, V32>(sh.lv), ng, sh.cs, sh.nt, sh.sm, s->stream, a);
     }
     int* df = (int*)s->rel_cnt.ensure(4 * sizeof(int));
-    launch(resident_failed_kernel, 1, 256, 0, s->stream, k, (const ColState*)co, df);
+    int* idx = (int*)s->rel_idx.ensure((size_t)(k + 1) * sizeof(int));
+    launch(rel_compact_kernel, 1, 256, 0, s->stream, k, (const ColState*)co, idx, df);
     int failed = 0;
     s->bnc.fetch(&failed, df, sizeof(int), s->stream);
-    return failed == 0;
+    return failed;
 }
+
+template <class V64, class V32>
+static void solve_mixed(tg_solver s, int k, const V64* B, V64* X, ColState* co, bool zero_guess, int maxit);
 
 template <class V64, class V32>
 static void solve_nm(tg_solver s, int k, const V64* B, V64* X, ColState* co, bool zero_guess = false)
@@ -2606,17 +2608,39 @@ static void solve_nm(tg_solver s, int k, const V64* B, V64* X, ColState* co, boo
             e64.spmm(k, X, R, nullptr, false, nullptr, nullptr, 0);
             launch(resid_kernel<V64>, cdiv_u(nk, 256), 256, 0, s->stream, n, k, k, B, R, nullptr);
         }
-        if (solve_resident<V64, V32>(s, k, B, X, co, R, maxit, zero_guess)) return;
-        // a breakdown, or a process that does not converge: the path below
-        // from the same start
-        if (zero_guess) TG_CUDA(cudaMemsetAsync(X, 0, nk * sizeof(V64), s->stream));
-        else TG_CUDA(cudaMemcpyAsync(X, s->xkeep.p, nk * sizeof(V64), cudaMemcpyDeviceToDevice, s->stream));
-        launch(init_cols_kernel, cdiv_u(k, 128), 128, 0, s->stream, k, co, s->tol, maxit);
+        const int kf = solve_resident<V64, V32>(s, k, B, X, co, R, maxit, zero_guess);
+        if (kf == 0) return;
+        // the columns that broke down or did not converge: the batched path
+        // from their start, in a block of their own
+        const size_t nkf = (size_t)n * kf;
+        const int* idx = (const int*)s->fb_idx.ensure((size_t)kf * sizeof(int));
+        TG_CUDA(cudaMemcpyAsync((void*)idx, s->rel_idx.p, (size_t)kf * sizeof(int), cudaMemcpyDeviceToDevice, s->stream));
+        V64* Bf = (V64*)s->fb_b.ensure(nkf * sizeof(V64));
+        V64* Xf = (V64*)s->fb_x.ensure(nkf * sizeof(V64));
+        ColState* cf = (ColState*)s->fb_cs.ensure(sizeof(ColState) * kf);
+        launch(gather_cols_kernel<V64>, cdiv_u(nkf, 256), 256, 0, s->stream, n, k, kf, idx, B, Bf);
+        if (zero_guess) TG_CUDA(cudaMemsetAsync(Xf, 0, nkf * sizeof(V64), s->stream));
+        else launch(gather_cols_kernel<V64>, cdiv_u(nkf, 256), 256, 0, s->stream, n, k, kf, idx,
+                    (const V64*)s->xkeep.p, Xf);
+        launch(init_cols_kernel, cdiv_u(kf, 128), 128, 0, s->stream, kf, cf, s->tol, maxit);
+        solve_mixed<V64, V32>(s, kf, Bf, Xf, cf, zero_guess, maxit);
+        launch(scatter_cols_kernel<V64>, cdiv_u(nkf, 256), 256, 0, s->stream, n, k, kf, idx, (const V64*)Xf, X);
+        launch(resident_results_kernel, cdiv_u(kf, 128), 128, 0, s->stream, kf, idx, (const ColState*)cf, co);
+        return;
     }
-    if (s->precon == TG_PRECON_ICH && !s->ic_done) {
-        factor_ic<V64, V32>(s);
-        setup_engine(s, e64);
-    }
+    solve_mixed<V64, V32>(s, k, B, X, co, zero_guess, maxit);
+}
+
+// The batched kernels of the mixed path; co initialised by the caller
+template <class V64, class V32>
+static void solve_mixed(tg_solver s, int k, const V64* B, V64* X, ColState* co, bool zero_guess, int maxit)
+{
+    const MeshDev& m = s->mesh->d;
+    const int n = m.n;
+    const size_t nk = (size_t)n * k;
+    if (s->precon == TG_PRECON_ICH && !s->ic_done) factor_ic<V64, V32>(s);
+    Engine<V64>& e64 = engine<V64>(s);
+    setup_engine(s, e64);
     // FP64 iterative refinement around FP32 / complex-FP32 inner solves:
     // r = b - F x in FP64, solve F e = r in FP32 to a loose tolerance,
     // x += e in FP64, until |r| <= tol |b| per column.
