@@ -475,6 +475,10 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
                 const V al = sdiv(S.zr[tid], smake<V>(red(tid, 0, false), CPLX ? red(tid, 1, false) : 0.f));
                 S.alpha[tid] = al;
                 if (!sfinite(al)) { S.on[tid] = 0; S.st[tid] = 2; }
+                // a direction of negative curvature: the system is not positive
+                // definite, and CG need not converge on it; the caller takes
+                // the column elsewhere
+                if (!CPLX && red(tid, 0, false) < 0.f) { S.on[tid] = S.outer[tid] = 0; S.ost[tid] = S.fail[tid] = 1; }
             }
             __syncthreads();
             bool on[LV], any = false;
