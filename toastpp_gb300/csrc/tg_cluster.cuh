@@ -42,6 +42,7 @@ struct ResArgs {
     float trig;                 // residual drop that triggers a correction
     double cwtol;               // componentwise bound (0: none)
     int maxit, max_upd, zero_guess;
+    int per;                    // iterations that a result counts as one
     int all64;                  // every residual product in FP64
 };
 

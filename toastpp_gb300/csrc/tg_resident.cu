@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
         O.bnorm = S.bnorm[tid];
         O.err = S.oerr[tid];
         O.berr = S.berr[tid];
-        O.its = S.its[tid];
+        O.its = (S.its[tid] + a.per - 1) / a.per;
         O.status = S.outer[tid] ? 1 : S.ost[tid];
         O.rel = S.fail[tid];
         O.active = 0;

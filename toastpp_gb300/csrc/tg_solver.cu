@@ -2561,8 +2561,14 @@ static int solve_resident(tg_solver s, int k, const V64* B, V64* X, ColState* co
     a.rowptr = m.rowptr; a.colidx = m.colidx;
     a.A64 = s->val64.as<V64>(); a.Aff = s->valff.p; a.absA = s->absA.as<float>();
     a.co = co;
-    a.trig = (float)s->inner_tol; a.cwtol = s->cw_tol; a.maxit = maxit; a.max_upd = 4 * std::max(1, s->max_outer);
+    a.trig = (float)s->inner_tol; a.cwtol = s->cw_tol; a.max_upd = 4 * std::max(1, s->max_outer);
     a.zero_guess = zero_guess ? 1 : 0;
+    // A limit bounds what it bounds on the batched path: for a CG request each
+    // inner solve between two FP64 residuals, of which there are max_outer; for a
+    // real BiCGSTAB request iterations of two products, counted in those here too.
+    a.per = !vt<V32>::cplx && s->method == TG_SOLVER_BICGSTAB ? 2 : 1;
+    a.maxit = (int)std::min<long long>((long long)maxit * (s->method == TG_SOLVER_CG ? std::max(1, s->max_outer) : a.per),
+                                       1 << 30);
     // float-float residuals carry about 2^-46 of |A||x|: finer tests than 1e-13 take FP64 ones
     a.all64 = !(s->tol >= 1e-13 && (s->cw_tol == 0 || s->cw_tol >= 1e-13));
     {
