@@ -1432,7 +1432,11 @@ static __global__ void rel_outer_kernel(int k, ColState* __restrict__ co, ColSta
     // follows the FP64 system (at the rounding floor of the FP64 residual the
     // true residual stops falling while the recursion goes on): resuming it
     // with the old directions stagnates, so it restarts from the true residual
-    // (off that floor the two agree to 1e-3)
+    // (off that floor COCG's two agree to 1e-3.  BiCGSTAB's recursive residual
+    // drifts with its peaks, and restarting it early costs nothing either: over
+    // 120 blocks of up to 32 columns, discs of 817 to 27.9k nodes, cylinders and
+    // boxes, real and complex, triggers 1e-4 and 1e-2, the line at 1.25 takes 0.87
+    // to 1.005 times the iterations of one at 8, over all 1 and 3.5 % fewer)
     if (O.err > 1.25 * I.err * I.scale) I.rel = 2;
     // rescale the process to the new residual (exact: powers of two)
     I.scale_prev = I.scale;
