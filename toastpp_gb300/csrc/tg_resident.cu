@@ -556,9 +556,11 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
             // 1: the trigger was reached, the process goes on; 2: it restarts
             S.rel[c] = S.outer[c] ? (S.on[c] ? (limit ? 1 : 0) : (S.st[c] == 0 ? 1 : 2)) : 0;
             // rows whose float-float residual may be off by more than a
-            // thousandth of the residual that the recursion expects are formed
-            // in FP64 (float-float carries about 2^-46 of |A||x|)
-            S.thr[c] = a.all64 ? -1.f : (float)((double)S.err[c] * 1e-3 * 70368744177664.0);
+            // thousandth of the residual to expect are formed in FP64 (float-float
+            // carries about 2^-46 of |A||x|): the recursion's, or where it grew (or
+            // is no number) and its correction is dropped, the last one
+            const float ex = S.err[c] <= S.bn[c] ? S.err[c] : S.bn[c];
+            S.thr[c] = a.all64 ? -1.f : (float)((double)ex * 1e-3 * 70368744177664.0);
         }
         __syncthreads();
         bool rel[LV], anyr = false;
