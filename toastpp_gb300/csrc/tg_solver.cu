@@ -373,7 +373,8 @@ struct Engine {
     };
     std::map<std::pair<int, int>, ClValues> clv;
     long long fver = 0;        // version of the factor behind L
-    std::map<int, std::pair<int, int>> ic_shapes;  // k -> (columns, CTAs) of a cluster; CTAs 0: none fits
+    // (k, ordering) -> (columns, CTAs) of a cluster; CTAs 0: none fits
+    std::map<std::pair<int, int>, std::pair<int, int>> ic_shapes;
     Bounce bnc;
     GraphCache graphs;
 
@@ -567,7 +568,7 @@ struct Engine {
     // the chip, with the fewest rows per CTA; (0, 0) where nothing fits
     std::pair<int, int> ic_shape(int k)
     {
-        auto it = ic_shapes.find(k);
+        auto it = ic_shapes.find({k, ico});
         if (it != ic_shapes.end()) return it->second;
         std::pair<int, int> best{0, 0};
         double tbest = 1e300;
@@ -591,7 +592,7 @@ struct Engine {
             }
         }
         if (ic_shapes.size() >= 64) ic_shapes.clear();
-        return ic_shapes[k] = best;
+        return ic_shapes[{k, ico}] = best;
     }
 
     // shared memory of a CTA: the vector, then levels and rows of both sweeps
