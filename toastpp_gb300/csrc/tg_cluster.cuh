@@ -67,9 +67,10 @@ template <class V>
 void (*ic_cluster_kernel_of(int lv))(IcClArgs<V>);
 
 // G of the approximate inverse from A's values in CSR order, a warp per row
-constexpr int FSAI_WARPS = 4;
-template <class V>
-void (*fsai_kernel_of())(int n, const int* rowptr, const int* colidx, const int* diagpos, const V* A, const int* gptr,
+// (two warps a CTA: a warp's complex FP64 matrix takes 17 KB of shared memory)
+constexpr int FSAI_WARPS = 2;
+template <class V64, class V>
+void (*fsai_kernel_of())(int n, const int* rowptr, const int* colidx, const int* diagpos, const V64* A, const int* gptr,
                          const int* gcol, const int* gcnt, V* gval);
 
 }  // namespace tg

@@ -114,7 +114,7 @@ struct FSum {
 };
 
 // FP32 scalar arithmetic of the recursions: a / b (Smith's scaling for complex
-// values), and the square root with non-negative real part
+// values); square root with non-negative real part
 __device__ __forceinline__ float sdiv(float a, float b) { return a / b; }
 __device__ __forceinline__ cf sdiv(cf a, cf b)
 {
@@ -128,18 +128,12 @@ __device__ __forceinline__ cf sdiv(cf a, cf b)
 template <class V> __device__ __forceinline__ V smake(float r, float i);
 template <> __device__ __forceinline__ float smake<float>(float r, float) { return r; }
 template <> __device__ __forceinline__ cf smake<cf>(float r, float i) { return cf{r, i}; }
-__device__ __forceinline__ float ssqrt(float a) { return sqrtf(a); }
-__device__ __forceinline__ cf ssqrt(cf z)
-{
-    const float r = hypotf(z.x, z.y);
-    if (r == 0.f) return cf{0.f, 0.f};
-    if (z.x >= 0.f) {
-        const float t = sqrtf(0.5f * (r + z.x));
-        return cf{t, z.y / (2.f * t)};
-    }
-    const float t = sqrtf(0.5f * (r - z.x));
-    return cf{fabsf(z.y) / (2.f * t), z.y < 0.f ? -t : t};
-}
+__device__ __forceinline__ double ssqrt(double a) { return sqrt(a); }
+__device__ __forceinline__ cd ssqrt(cd z) { return csqrt_d(z); }
+__device__ __forceinline__ bool sfinite(double a) { return isfinite(a); }
+__device__ __forceinline__ bool sfinite(cd a) { return isfinite(a.x) && isfinite(a.y); }
+__device__ __forceinline__ bool szero(double a) { return a == 0.0; }
+__device__ __forceinline__ bool szero(cd a) { return a.x == 0.0 && a.y == 0.0; }
 __device__ __forceinline__ bool sfinite(float a) { return isfinite(a); }
 __device__ __forceinline__ bool sfinite(cf a) { return isfinite(a.x) && isfinite(a.y); }
 __device__ __forceinline__ bool szero(float a) { return a == 0.f; }
@@ -149,27 +143,29 @@ __device__ __forceinline__ bool szero(cf a) { return a.x == 0.f && a.y == 0.f; }
 // G of the approximate inverse: a warp per row.  The row's pattern S (m
 // entries, ascending, the row itself last) is in the slice layout; the warp
 // gathers A(S, S) into shared memory, factors it L D L^T in place (lane =
-// row), and back-substitutes L^T y = e_m; the row is y / sqrt(d_m).  A row
-// whose pivots are not finite keeps its scaled diagonal alone.
+// row), and back-substitutes L^T y = e_m; the row is y / sqrt(d_m), formed in
+// FP64 from the FP64 matrix and cast, as the IC(0) factor is.  A row whose
+// pivots are not positive, or whose entries are no FP32 numbers, keeps its
+// scaled diagonal alone.
 // ---------------------------------------------------------------------------
-template <class V>
+template <class V64, class V>
 __global__ void __launch_bounds__(32 * FSAI_WARPS) fsai_kernel(int n, const int* __restrict__ rowptr,
                                                               const int* __restrict__ colidx,
                                                               const int* __restrict__ diagpos,
-                                                              const V* __restrict__ A, const int* __restrict__ gptr,
+                                                              const V64* __restrict__ A, const int* __restrict__ gptr,
                                                               const int* __restrict__ gcol,
                                                               const int* __restrict__ gcnt, V* __restrict__ gval)
 {
-    __shared__ V sm[FSAI_WARPS][FSAI_MAXM][FSAI_MAXM + 1];
+    __shared__ V64 sm[FSAI_WARPS][FSAI_MAXM][FSAI_MAXM + 1];
     __shared__ int ss[FSAI_WARPS][FSAI_MAXM];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * FSAI_WARPS + w;
     if (i >= n) return;
-    V(*M)[FSAI_MAXM + 1] = sm[w];
+    V64(*M)[FSAI_MAXM + 1] = sm[w];
     int* S = ss[w];
     const int m = gcnt[i], base = gptr[i >> 5] + (i & 31);
     if (lane < m) S[lane] = gcol[base + 32 * lane];
     for (int a = 0; a < m; a++)
-        if (lane < m) M[a][lane] = vzero<V>();
+        if (lane < m) M[a][lane] = vzero<V64>();
     __syncwarp();
     for (int a = 0; a < m; a++) {
         const int ra = S[a];
@@ -182,12 +178,12 @@ __global__ void __launch_bounds__(32 * FSAI_WARPS) fsai_kernel(int n, const int*
     __syncwarp();
     bool ok = true;
     for (int j = 0; j < m; j++) {
-        const V d = M[j][j];
-        ok &= sfinite(d) && !szero(d) && re(d) > 0.f;
+        const V64 d = M[j][j];
+        ok &= sfinite(d) && !szero(d) && re(d) > 0.0;
         if (!ok) break;  // the same value in every lane
-        V l = vzero<V>();
+        V64 l = vzero<V64>();
         if (lane > j && lane < m) {
-            l = sdiv(M[lane][j], d);
+            l = vdiv(M[lane][j], d);
             for (int c = j + 1; c <= lane; c++) M[lane][c] = vfms(M[lane][c], l, M[c][j]);
         }
         __syncwarp();
@@ -197,16 +193,15 @@ __global__ void __launch_bounds__(32 * FSAI_WARPS) fsai_kernel(int n, const int*
     V y = vzero<V>();
     if (ok) {
         // lane j holds y_j
-        y = lane == m - 1 ? vmake<V>(1.0, 0.0) : vzero<V>();
+        V64 t = lane == m - 1 ? vmake<V64>(1.0, 0.0) : vzero<V64>();
         for (int r = m - 1; r > 0; r--) {
-            const V yr = shfl(y, r);
-            if (lane < r) y = vfms(y, M[r][lane], yr);
+            const V64 tr = shfl(t, r);
+            if (lane < r) t = vfms(t, M[r][lane], tr);
         }
-        const V s = sdiv(vmake<V>(1.0, 0.0), ssqrt(M[m - 1][m - 1]));
-        y = vmul(y, s);
+        y = vcast<V, V64>(vmul(t, vrecip(ssqrt(M[m - 1][m - 1]))));
         ok = __all_sync(0xffffffffu, lane >= m || sfinite(y));
     }
-    if (!ok) y = lane == m - 1 ? sdiv(vmake<V>(1.0, 0.0), ssqrt(A[diagpos[i]])) : vzero<V>();
+    if (!ok) y = lane == m - 1 ? vcast<V, V64>(vrecip(ssqrt(A[diagpos[i]]))) : vzero<V>();
     if (lane < m) gval[base + 32 * lane] = y;
     // padding entries of the slice
     const int wd = (gptr[(i >> 5) + 1] - gptr[i >> 5]) >> 5;
@@ -890,14 +885,14 @@ void (*resident_kernel(int lv))(ResArgs<V64, V32>)
 template void (*resident_kernel<double, float>(int))(ResArgs<double, float>);
 template void (*resident_kernel<cd, cf>(int))(ResArgs<cd, cf>);
 
-template <class V>
-void (*fsai_kernel_of())(int, const int*, const int*, const int*, const V*, const int*, const int*, const int*, V*)
+template <class V64, class V>
+void (*fsai_kernel_of())(int, const int*, const int*, const int*, const V64*, const int*, const int*, const int*, V*)
 {
-    return fsai_kernel<V>;
+    return fsai_kernel<V64, V>;
 }
-template void (*fsai_kernel_of<float>())(int, const int*, const int*, const int*, const float*, const int*, const int*,
-                                         const int*, float*);
-template void (*fsai_kernel_of<cf>())(int, const int*, const int*, const int*, const cf*, const int*, const int*,
-                                      const int*, cf*);
+template void (*fsai_kernel_of<double, float>())(int, const int*, const int*, const int*, const double*, const int*,
+                                                 const int*, const int*, float*);
+template void (*fsai_kernel_of<cd, cf>())(int, const int*, const int*, const int*, const cd*, const int*, const int*,
+                                          const int*, cf*);
 
 }  // namespace tg

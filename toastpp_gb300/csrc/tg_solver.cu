@@ -2166,7 +2166,7 @@ static void factor_ic(tg_solver s)
 }
 
 // the resident solve's matrices of the last reset: A in slices, G, and G^T
-template <class V32>
+template <class V64, class V32>
 static void build_resident(tg_solver s)
 {
     const MeshDev& m = s->mesh->d;
@@ -2175,8 +2175,8 @@ static void build_resident(tg_solver s)
     V32* sg = (V32*)s->sg32.ensure((size_t)m.sg.len * sizeof(V32));
     V32* st = (V32*)s->st32.ensure((size_t)m.st.len * sizeof(V32));
     launch(ell_gather_kernel<V32>, cdiv_u(m.sa.len, 256), 256, 0, s->stream, m.sa.len, m.sa.src, A32, sa);
-    launch(fsai_kernel_of<V32>(), cdiv_u(m.n, FSAI_WARPS), 32 * FSAI_WARPS, 0, s->stream, m.n, m.rowptr, m.colidx,
-           m.diagpos, A32, m.sg.ptr, m.sg.col, m.gcnt, sg);
+    launch(fsai_kernel_of<V64, V32>(), cdiv_u(m.n, FSAI_WARPS), 32 * FSAI_WARPS, 0, s->stream, m.n, m.rowptr, m.colidx,
+           m.diagpos, (const V64*)s->val64.as<V64>(), m.sg.ptr, m.sg.col, m.gcnt, sg);
     launch(ell_gather_kernel<V32>, cdiv_u(m.st.len, 256), 256, 0, s->stream, m.st.len, m.st.src, sg, st);
     s->res_ready = true;
 }
@@ -2607,7 +2607,7 @@ static void solve_nm(tg_solver s, int k, const V64* B, V64* X, ColState* co, boo
         return;
     }
     if (resident_ok(s) && shape_of<V64, V32>(s, k).cs) {
-        if (!s->res_ready) build_resident<V32>(s);
+        if (!s->res_ready) build_resident<V64, V32>(s);
         V64* R = (V64*)s->tmp.ensure(nk * sizeof(V64));
         if (!zero_guess) {
             TG_CUDA(cudaMemcpyAsync(s->xkeep.ensure(nk * sizeof(V64)), X, nk * sizeof(V64), cudaMemcpyDeviceToDevice,
