@@ -113,21 +113,66 @@ struct FSum {
     }
 };
 
-// FP32 scalar arithmetic of the recursions: a / b (Smith's scaling for complex
-// values); square root with non-negative real part
-__device__ __forceinline__ float sdiv(float a, float b) { return a / b; }
-__device__ __forceinline__ cf sdiv(cf a, cf b)
+// The recursion's scalars (r.z, alpha, beta): unevaluated sums h + l of two
+// floats, about 2^-45 relative.  In FP64, as the batched methods keep them, the
+// divisions of one thread stood in every iteration's chain (1.8 us of it: 217
+// nodes 0.39 -> 0.47 ms a request); the vectors take alpha and beta as FP32
+// either way.
+struct Sc {
+    float h = 0.f, l = 0.f;
+};
+struct Scc {
+    Sc x, y;
+};
+template <class V> struct ScOf { using T = Sc; };
+template <> struct ScOf<cf> { using T = Scc; };
+
+__device__ __forceinline__ Sc sc_norm(float h, float l)  // |l| <= |h|
 {
-    if (fabsf(b.x) >= fabsf(b.y)) {
-        const float r = b.y / b.x, d = 1.0f / (b.x + b.y * r);
-        return cf{(a.x + a.y * r) * d, (a.y - a.x * r) * d};
-    }
-    const float r = b.x / b.y, d = 1.0f / (b.x * r + b.y);
-    return cf{(a.x * r + a.y) * d, (a.y * r - a.x) * d};
+    const float s = __fadd_rn(h, l);
+    return Sc{s, __fsub_rn(l, __fsub_rn(s, h))};
 }
-template <class V> __device__ __forceinline__ V smake(float r, float i);
-template <> __device__ __forceinline__ float smake<float>(float r, float) { return r; }
-template <> __device__ __forceinline__ cf smake<cf>(float r, float i) { return cf{r, i}; }
+__device__ __forceinline__ Sc sc_add(Sc a, Sc b)
+{
+    const float s = __fadd_rn(a.h, b.h), t = __fsub_rn(s, a.h);
+    return sc_norm(s, __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, t)), __fsub_rn(b.h, t)) + (a.l + b.l));
+}
+__device__ __forceinline__ Sc sc_neg(Sc a) { return Sc{-a.h, -a.l}; }
+__device__ __forceinline__ Sc sc_mul(Sc a, Sc b)
+{
+    const float p = __fmul_rn(a.h, b.h);
+    return sc_norm(p, __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.h, -p))));
+}
+__device__ __forceinline__ Sc sc_div(Sc a, Sc b)
+{
+    const float q = a.h / b.h;
+    // a - q b, exact in its leading terms
+    const float r = __fmaf_rn(-q, b.l, __fmaf_rn(-q, b.h, a.h) + a.l);
+    return sc_norm(q, r / b.h);
+}
+__device__ __forceinline__ Sc sc_scale(Sc a, float f) { return Sc{a.h * f, a.l * f}; }  // f: a power of two
+__device__ __forceinline__ Scc sc_scale(Scc a, float f) { return Scc{sc_scale(a.x, f), sc_scale(a.y, f)}; }
+// a conj(b) / |b|^2, with b scaled to between 1 and 2 first
+__device__ __forceinline__ Scc sc_div(Scc a, Scc b)
+{
+    const float m = fmaxf(fabsf(b.x.h), fabsf(b.y.h));
+    // 2^-e for m = 2^e (1 ..), e within +-126; zero, infinite and NaN m: 1
+    const int e = (int)(__float_as_uint(m) >> 23);
+    const float f = e > 0 && e < 254 ? __uint_as_float((unsigned)(254 - e) << 23) : 1.f;
+    a = sc_scale(a, f);
+    b = sc_scale(b, f);
+    const Sc d = sc_add(sc_mul(b.x, b.x), sc_mul(b.y, b.y));
+    return Scc{sc_div(sc_add(sc_mul(a.x, b.x), sc_mul(a.y, b.y)), d),
+               sc_div(sc_add(sc_mul(a.y, b.x), sc_neg(sc_mul(a.x, b.y))), d)};
+}
+__device__ __forceinline__ bool sc_zero(Sc a) { return a.h == 0.f; }
+__device__ __forceinline__ bool sc_zero(Scc a) { return a.x.h == 0.f && a.y.h == 0.f; }
+__device__ __forceinline__ bool sc_finite(Sc a) { return isfinite(a.h); }
+__device__ __forceinline__ bool sc_finite(Scc a) { return isfinite(a.x.h) && isfinite(a.y.h); }
+__device__ __forceinline__ float sc_cast(Sc a) { return a.h; }
+__device__ __forceinline__ cf sc_cast(Scc a) { return cf{a.x.h, a.y.h}; }
+
+// square root with non-negative real part
 __device__ __forceinline__ double ssqrt(double a) { return sqrt(a); }
 __device__ __forceinline__ cd ssqrt(cd z) { return csqrt_d(z); }
 __device__ __forceinline__ bool sfinite(double a) { return isfinite(a); }
@@ -136,8 +181,6 @@ __device__ __forceinline__ bool szero(double a) { return a == 0.0; }
 __device__ __forceinline__ bool szero(cd a) { return a.x == 0.0 && a.y == 0.0; }
 __device__ __forceinline__ bool sfinite(float a) { return isfinite(a); }
 __device__ __forceinline__ bool sfinite(cf a) { return isfinite(a.x) && isfinite(a.y); }
-__device__ __forceinline__ bool szero(float a) { return a == 0.f; }
-__device__ __forceinline__ bool szero(cf a) { return a.x == 0.f && a.y == 0.f; }
 
 // ---------------------------------------------------------------------------
 // G of the approximate inverse: a warp per row.  The row's pattern S (m
@@ -211,10 +254,12 @@ __global__ void __launch_bounds__(32 * FSAI_WARPS) fsai_kernel(int n, const int*
 // ---------------------------------------------------------------------------
 // The resident solve.
 // ---------------------------------------------------------------------------
-// per-column state of the process, in every CTA's shared memory
+// per-column state of the process, in every CTA's shared memory; alpha and beta
+// as the vectors' updates take them
 template <class V>
 struct ResCols {
-    V alpha[CL_MAXCG], beta[CL_MAXCG], zr[CL_MAXCG];
+    V alpha[CL_MAXCG], beta[CL_MAXCG];
+    typename ScOf<V>::T zr[CL_MAXCG];
     float bn[CL_MAXCG], err[CL_MAXCG], fs[CL_MAXCG], thr[CL_MAXCG], trig[CL_MAXCG];
     double bnorm[CL_MAXCG], oerr[CL_MAXCG], scale[CL_MAXCG], berr[CL_MAXCG];
     int outer[CL_MAXCG], on[CL_MAXCG], rel[CL_MAXCG], its[CL_MAXCG], st[CL_MAXCG], ost[CL_MAXCG], nupd[CL_MAXCG], met[CL_MAXCG];
@@ -337,7 +382,12 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
             if (mx) s.h = fmaxf(s.h, t.x);
             else { FSum u; u.h = t.x; u.l = t.y; s.add(u); }
         }
-        return s.h + s.l;
+        return sc_norm(s.h, s.l);
+    };
+    // the (bilinear) product of quantities 0 and 1
+    auto product = [&](int c) {
+        if constexpr (CPLX) return Scc{red(c, 0, false), red(c, 1, false)};
+        else return red(c, 0, false);
     };
     for (int t = tid; t < npush; t += NT) push[t] = a.push[a.pofs[rank] + t];
     // every CTA of the cluster runs before any stores into another's shared memory
@@ -392,7 +442,8 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
         S.bn[c] = S.err[c] = (float)(er / S.scale[c]);
         S.rel[c] = S.its[c] = S.st[c] = S.ost[c] = S.nupd[c] = S.met[c] = S.fail[c] = 0;
         S.trig[c] = a.trig;
-        S.alpha[c] = S.beta[c] = S.zr[c] = vzero<V>();
+        S.alpha[c] = S.beta[c] = vzero<V>();
+        S.zr[c] = typename ScOf<V>::T();
     }
     __syncthreads();
     for (int i = rb; i < R1; i += rs) {
@@ -467,13 +518,15 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
         reduce(v, 3, false);
         if (ph == 0) {
             if (tid < CG && S.on[tid]) {
-                const V al = sdiv(S.zr[tid], smake<V>(red(tid, 0, false), CPLX ? red(tid, 1, false) : 0.f));
-                S.alpha[tid] = al;
-                if (!sfinite(al)) { S.on[tid] = 0; S.st[tid] = 2; }
+                const auto pq = product(tid);
+                const auto al = sc_div(S.zr[tid], pq);
+                S.alpha[tid] = sc_cast(al);
+                if (!sc_finite(al)) { S.on[tid] = 0; S.st[tid] = 2; }
                 // a direction of negative curvature: the system is not positive
                 // definite, and CG need not converge on it; the caller takes
                 // the column elsewhere
-                if (!CPLX && red(tid, 0, false) < 0.f) { S.on[tid] = S.outer[tid] = 0; S.ost[tid] = S.fail[tid] = 1; }
+                if constexpr (!CPLX)
+                    if (pq.h < 0.f) { S.on[tid] = S.outer[tid] = 0; S.ost[tid] = S.fail[tid] = 1; }
             }
             __syncthreads();
             bool on[LV], any = false;
@@ -515,10 +568,10 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
         }
         if (tid < CG) {
             const int c = tid;
-            const V rz = smake<V>(red(c, 0, false), CPLX ? red(c, 1, false) : 0.f);
+            const auto rz = product(c);
             bool go = S.on[c];
             if (mode == 1 && go) {
-                S.err[c] = sqrtf(red(c, 2, false));
+                S.err[c] = sqrtf(red(c, 2, false).h);
                 S.its[c]++;
                 go = false;
                 if (S.err[c] <= S.trig[c] * S.bn[c]) { S.on[c] = 0; S.st[c] = 0; }
@@ -529,11 +582,11 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
             }
             if (mode == 2) go = S.rel[c] != 0;
             if (go) {
-                const V be = mode == 0 || S.rel[c] == 2 ? vzero<V>() : sdiv(rz, S.zr[c]);
-                S.beta[c] = be;
+                const auto be = mode == 0 || S.rel[c] == 2 ? typename ScOf<V>::T() : sc_div(rz, S.zr[c]);
+                S.beta[c] = sc_cast(be);
                 S.zr[c] = rz;
                 S.rel[c] = 0;
-                if (szero(rz) || !sfinite(rz) || !sfinite(be)) { S.on[c] = 0; S.st[c] = 2; }
+                if (sc_zero(rz) || !sc_finite(rz) || !sc_finite(be)) { S.on[c] = 0; S.st[c] = 2; }
             }
         }
         __syncthreads();
@@ -630,9 +683,10 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
         }
         if (tid < CG && S.rel[tid]) {
             const int c = tid;
-            const double er = sqrt((double)red(c, 0, false)) * S.scale[c], tol = a.co[cg0 + c].tol;
+            const Sc r2 = red(c, 0, false);
+            const double er = sqrt((double)r2.h + (double)r2.l) * S.scale[c], tol = a.co[cg0 + c].tol;
             S.oerr[c] = er;
-            if (a.cwtol > 0.0) S.berr[c] = red(c, 1, true);
+            if (a.cwtol > 0.0) S.berr[c] = red(c, 1, true).h;
             // A column that meets its bounds without much to spare takes one
             // correction more, of no more than what is missing: the bound alone
             // left the data gradient, which sums small differences of the data,
@@ -662,7 +716,7 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
                 const float f = (float)(old / S.scale[c]);
                 S.fs[c] = f;
                 S.bn[c] = (float)(er / S.scale[c]);
-                S.zr[c] = vscale(S.zr[c], f * f);
+                S.zr[c] = sc_scale(S.zr[c], f * f);
                 S.on[c] = 1;
                 S.st[c] = 0;
             }
