@@ -106,6 +106,14 @@ struct FSum {
         l += __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(x, b));
         h = s;
     }
+    // x^2 to about 2^-46
+    __device__ __forceinline__ void add_square(double x)
+    {
+        const float2 f = ff_split(x);
+        const float p = __fmul_rn(f.x, f.x);
+        l += __fmaf_rn(2.f * f.x, f.y, __fmaf_rn(f.x, f.x, -p));
+        add(p);
+    }
     __device__ __forceinline__ void add(const FSum& o)
     {
         l += o.l;
@@ -608,7 +616,7 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
             // carries about 2^-46 of |A||x|): the recursion's, or where it grew (or
             // is no number) and its correction is dropped, the last one
             const float ex = S.err[c] <= S.bn[c] ? S.err[c] : S.bn[c];
-            S.thr[c] = a.all64 ? -1.f : (float)((double)ex * 1e-3 * 70368744177664.0);
+            S.thr[c] = (float)((double)ex * 1e-3 * 70368744177664.0);
         }
         __syncthreads();
         bool rel[LV], anyr = false;
@@ -645,25 +653,33 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
                         float d = 0.f;
                         V64 ax;
                         f2x h = 0ull, l = 0ull;
+                        // (every product in FP64: a CG request's; complex systems only
+                        // for tolerances below 1e-13, and then both)
+                        if (CPLX || !a.all64) {
 #pragma unroll 2
-                        for (int e = e0; e < e1; e++) {
-                            const size_t o = (size_t)a.colidx[e] * k + c;
-                            if constexpr (CPLX) {
-                                const float4 f = ((const float4*)a.Aff)[e], xf = ((const float4*)a.Xff)[o];
-                                ff2_mac(h, l, f2_bcast(f.x), f2_bcast(f.y), f2_pack(xf.x, xf.z), f2_pack(xf.y, xf.w));
-                                ff2_mac(h, l, f2_pack(-f.z, f.z), f2_pack(-f.w, f.w), f2_pack(xf.z, xf.x),
-                                        f2_pack(xf.w, xf.y));
-                                d = fmaf(a.absA[e], fmaxf(fabsf(xf.x), fabsf(xf.z)), d);
-                            } else {
-                                const float2 f = ((const float2*)a.Aff)[e], xf = ((const float2*)a.Xff)[o];
-                                ff2_mac(h, l, f2_bcast(f.x), f2_bcast(f.y), f2_bcast(xf.x), f2_bcast(xf.y));
-                                d = fmaf(a.absA[e], fabsf(xf.x), d);
+                            for (int e = e0; e < e1; e++) {
+                                const size_t o = (size_t)a.colidx[e] * k + c;
+                                if constexpr (CPLX) {
+                                    const float4 f = ((const float4*)a.Aff)[e], xf = ((const float4*)a.Xff)[o];
+                                    ff2_mac(h, l, f2_bcast(f.x), f2_bcast(f.y), f2_pack(xf.x, xf.z),
+                                            f2_pack(xf.y, xf.w));
+                                    ff2_mac(h, l, f2_pack(-f.z, f.z), f2_pack(-f.w, f.w), f2_pack(xf.z, xf.x),
+                                            f2_pack(xf.w, xf.y));
+                                    d = fmaf(a.absA[e], fmaxf(fabsf(xf.x), fabsf(xf.z)), d);
+                                } else {
+                                    const float2 f = ((const float2*)a.Aff)[e], xf = ((const float2*)a.Xff)[o];
+                                    ff2_mac(h, l, f2_bcast(f.x), f2_bcast(f.y), f2_bcast(xf.x), f2_bcast(xf.y));
+                                    d = fmaf(a.absA[e], fabsf(xf.x), d);
+                                }
                             }
+                        } else {
+                            for (int e = e0; e < e1; e++)
+                                d = fmaf(a.absA[e], mag1f(a.X[(size_t)a.colidx[e] * k + c]), d);
                         }
                         const size_t o = (size_t)i * k + c;
                         const V64 b = a.B[o];
                         d += mag1f(b);
-                        if (d > S.thr[j] * (float)S.scale[j]) {
+                        if (a.all64 || d > S.thr[j] * (float)S.scale[j]) {
                             ax = vzero<V64>();
                             for (int e = e0; e < e1; e++) ax = vfma(ax, a.A64[e], a.X[(size_t)a.colidx[e] * k + c]);
                         } else {
@@ -676,7 +692,9 @@ __global__ void __launch_bounds__(CL_NT, 1) resident_cg_kernel(ResArgs<V64, V> a
                         const float m = mag1f(rv), qd = m == 0.f ? 0.f : (d > 0.f ? m / d : INFINITY);
                         // a NaN must not pass the test
                         w[j][1].h = qd <= w[j][1].h ? w[j][1].h : (qd == qd ? qd : INFINITY);
-                        w[j][0].add(nrm2(vcast<V, V64>(vscale(rv, 1.0 / S.scale[j]))));
+                        const V64 rs = vscale(rv, 1.0 / S.scale[j]);
+                        w[j][0].add_square(re(rs));
+                        if constexpr (CPLX) w[j][0].add_square(im(rs));
                     }
                 }
             reduce(w, 2, true);

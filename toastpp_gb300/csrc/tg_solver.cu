@@ -2571,7 +2571,8 @@ static int solve_resident(tg_solver s, int k, const V64* B, V64* X, ColState* co
     a.maxit = (int)std::min<long long>((long long)maxit * (s->method == TG_SOLVER_CG ? std::max(1, s->max_outer) : a.per),
                                        1 << 30);
     // float-float residuals carry about 2^-46 of |A||x|: finer tests than 1e-13 take FP64 ones
-    a.all64 = !(s->tol >= 1e-13 && (s->cw_tol == 0 || s->cw_tol >= 1e-13));
+    // and so do CG requests, as in the restarted refinement of the batched path
+    a.all64 = s->method == TG_SOLVER_CG || !(s->tol >= 1e-13 && (s->cw_tol == 0 || s->cw_tol >= 1e-13));
     {
         ProfScope ps(&s->prof, PC_VEC, s->stream);
         launch_cluster(resident_kernel<V64, V32>(sh.lv), ng, sh.cs, sh.nt, sh.sm, s->stream, a);
