@@ -185,17 +185,50 @@ __device__ __forceinline__ double ssqrt(double a) { return sqrt(a); }
 __device__ __forceinline__ cd ssqrt(cd z) { return csqrt_d(z); }
 __device__ __forceinline__ bool sfinite(double a) { return isfinite(a); }
 __device__ __forceinline__ bool sfinite(cd a) { return isfinite(a.x) && isfinite(a.y); }
-__device__ __forceinline__ bool szero(double a) { return a == 0.0; }
-__device__ __forceinline__ bool szero(cd a) { return a.x == 0.0 && a.y == 0.0; }
 __device__ __forceinline__ bool sfinite(float a) { return isfinite(a); }
 __device__ __forceinline__ bool sfinite(cf a) { return isfinite(a.x) && isfinite(a.y); }
 
 // ---------------------------------------------------------------------------
+// 1 / d and 1 / sqrt(d), Re d > 0, for values that have been scaled to about 1:
+// an FP32 seed and two Newton steps in FP64.  (A row's pivots are one chain:
+// with FP64 divisions and square
+// roots it took 25 us on 217 nodes, 19 so, 10 in FP32.)
+__device__ __forceinline__ double nr_recip(double d)
+{
+    double x = 1.f / (float)d;
+    x = fma(x, fma(-d, x, 1.0), x);
+    return fma(x, fma(-d, x, 1.0), x);
+}
+__device__ __forceinline__ cd nr_recip(cd d)
+{
+    const double t = nr_recip(nrm2(d));
+    return cd{d.x * t, -d.y * t};
+}
+__device__ __forceinline__ double nr_rsqrt(double d)
+{
+    double x = 1.f / sqrtf((float)d);
+    x = x * fma(-0.5 * d * x, x, 1.5);
+    return x * fma(-0.5 * d * x, x, 1.5);
+}
+__device__ __forceinline__ cd nr_rsqrt(cd d)
+{
+    // sqrt d = (t, Im d / 2t) with t^2 = (|d| + Re d) / 2, its inverse the conjugate over |d|
+    const float r = hypotf((float)d.x, (float)d.y), t = sqrtf(0.5f * (r + (float)d.x)), u = 1.f / r;
+    cd x{t * u, -((float)d.y / (2.f * t)) * u};
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const cd y = vmul(d, vmul(x, x));
+        x = vmul(x, cd{1.5 - 0.5 * y.x, -0.5 * y.y});
+    }
+    return x;
+}
+
 // G of the approximate inverse: a warp per row.  The row's pattern S (m
 // entries, ascending, the row itself last) is in the slice layout; the warp
 // gathers A(S, S) into shared memory, factors it L D L^T in place (lane =
 // row), and back-substitutes L^T y = e_m; the row is y / sqrt(d_m), formed in
-// FP64 from the FP64 matrix and cast, as the IC(0) factor is.  A row whose
+// FP64 from the FP64 matrix (scaled by a power of four of its diagonal) and
+// cast, as the IC(0) factor is.  A row whose
 // pivots are not positive, or whose entries are no FP32 numbers, keeps its
 // scaled diagonal alone.
 // ---------------------------------------------------------------------------
@@ -214,6 +247,10 @@ __global__ void __launch_bounds__(32 * FSAI_WARPS) fsai_kernel(int n, const int*
     V64(*M)[FSAI_MAXM + 1] = sm[w];
     int* S = ss[w];
     const int m = gcnt[i], base = gptr[i >> 5] + (i & 31);
+    const double dg = re(A[diagpos[i]]);
+    bool ok = isfinite(dg) && dg > 0.0;  // the same value in every lane, here and below
+    const int ex = ok ? ilogb(dg) >> 1 : 0;
+    const double sc = ldexp(1.0, -2 * ex);
     if (lane < m) S[lane] = gcol[base + 32 * lane];
     for (int a = 0; a < m; a++)
         if (lane < m) M[a][lane] = vzero<V64>();
@@ -223,18 +260,17 @@ __global__ void __launch_bounds__(32 * FSAI_WARPS) fsai_kernel(int n, const int*
         for (int p = rowptr[ra] + lane; p < rowptr[ra + 1]; p += 32) {
             const int c = colidx[p];
             for (int b = 0; b <= a; b++)
-                if (S[b] == c) M[a][b] = A[p];
+                if (S[b] == c) M[a][b] = vscale(A[p], sc);
         }
     }
     __syncwarp();
-    bool ok = true;
     for (int j = 0; j < m; j++) {
         const V64 d = M[j][j];
-        ok &= sfinite(d) && !szero(d) && re(d) > 0.0;
-        if (!ok) break;  // the same value in every lane
+        ok &= sfinite(d) && re(d) > 0.0;
+        if (!ok) break;
         V64 l = vzero<V64>();
         if (lane > j && lane < m) {
-            l = vdiv(M[lane][j], d);
+            l = vmul(M[lane][j], nr_recip(d));
             for (int c = j + 1; c <= lane; c++) M[lane][c] = vfms(M[lane][c], l, M[c][j]);
         }
         __syncwarp();
@@ -249,7 +285,7 @@ __global__ void __launch_bounds__(32 * FSAI_WARPS) fsai_kernel(int n, const int*
             const V64 tr = shfl(t, r);
             if (lane < r) t = vfms(t, M[r][lane], tr);
         }
-        y = vcast<V, V64>(vmul(t, vrecip(ssqrt(M[m - 1][m - 1]))));
+        y = vcast<V, V64>(vscale(vmul(t, nr_rsqrt(M[m - 1][m - 1])), ldexp(1.0, -ex)));
         ok = __all_sync(0xffffffffu, lane >= m || sfinite(y));
     }
     if (!ok) y = lane == m - 1 ? vcast<V, V64>(vrecip(ssqrt(A[diagpos[i]]))) : vzero<V>();
