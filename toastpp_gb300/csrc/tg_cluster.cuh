@@ -25,7 +25,7 @@ struct Sell {
 template <class V64, class V32>
 struct ResArgs {
     int n, k, cs;
-    int slots, own;             // rows of a gather buffer (own rows and halo) and own rows, the largest of the CTAs
+    int slots;                  // rows of a gather buffer (own rows and halo), the largest of the CTAs
     int msm, mofs_val, mofs_col, mofs_ptr, mofs_push;  // msm: the matrices go to shared memory, at these byte offsets
     Sell<V32> A, G, T;          // system matrix, approximate inverse and its transpose
     const int* pofs;            // per CTA: its halo copies in push,

@@ -217,51 +217,57 @@ static void halo_lists(MeshHost& m)
     }
 }
 
-// rows of (column, source index) as slices
-static void sell_slices(const std::vector<std::vector<std::pair<int, int>>>& rows, SellHost& s)
+// CSR rows as slices; src: each entry's index in its source array (null: its own)
+static void sell_slices(int n, const std::vector<int>& ptr, const std::vector<int>& col, const int* src, SellHost& s)
 {
-    const int n = (int)rows.size(), ns = (n + 31) / 32;
+    const int ns = (n + 31) / 32;
     s.ptr.assign(ns + 1, 0);
     for (int t = 0; t < ns; t++) {
-        size_t w = 0;
-        for (int r = t * 32; r < std::min(n, t * 32 + 32); r++) w = std::max(w, rows[r].size());
-        s.ptr[t + 1] = s.ptr[t] + 32 * (int)w;
+        int w = 0;
+        for (int r = t * 32; r < std::min(n, t * 32 + 32); r++) w = std::max(w, ptr[r + 1] - ptr[r]);
+        s.ptr[t + 1] = s.ptr[t] + 32 * w;
     }
-    s.col.assign(s.ptr[ns], 0);
+    s.col.resize(s.ptr[ns]);
     s.src.assign(s.ptr[ns], -1);
     for (int t = 0; t < ns; t++)
         for (int r = t * 32; r < t * 32 + 32; r++) {
-            const int w = (s.ptr[t + 1] - s.ptr[t]) / 32, own = std::min(r, n - 1);
-            for (int e = 0; e < w; e++) {
-                const int o = s.ptr[t] + 32 * e + (r & 31);
-                const bool in = r < n && e < (int)rows[r].size();
-                s.col[o] = in ? rows[r][e].first : own;
-                s.src[o] = in ? rows[r][e].second : -1;
+            const int w = (s.ptr[t + 1] - s.ptr[t]) / 32, o = s.ptr[t] + (r & 31), own = std::min(r, n - 1);
+            const int p0 = r < n ? ptr[r] : 0, m = r < n ? ptr[r + 1] - p0 : 0;
+            for (int e = 0; e < m; e++) {
+                s.col[o + 32 * e] = col[p0 + e];
+                s.src[o + 32 * e] = src ? src[p0 + e] : p0 + e;
             }
+            for (int e = m; e < w; e++) s.col[o + 32 * e] = own;
         }
 }
 
 static void sell_patterns(MeshHost& m)
 {
     const int n = m.n;
-    std::vector<std::vector<std::pair<int, int>>> rows(n), trows(n);
-    for (int r = 0; r < n; r++)
-        for (int e = m.lrowptr[r]; e < m.lrowptr[r + 1]; e++) rows[r].push_back({m.lcolidx[e], e});
-    sell_slices(rows, m.sa);
+    sell_slices(n, m.lrowptr, m.lcolidx, nullptr, m.sa);
+    // G: the columns up to the row's own, ascending
+    std::vector<int> gp(n + 1, 0), gc, tp(n + 1, 0);
     m.gcnt.assign(n, 0);
     for (int r = 0; r < n; r++) {
-        rows[r].clear();
         for (int e = m.lrowptr[r]; e < m.lrowptr[r + 1]; e++)
-            if (m.lcolidx[e] <= r) rows[r].push_back({m.lcolidx[e], -1});
-        std::sort(rows[r].begin(), rows[r].end());
-        m.gcnt[r] = (int)rows[r].size();
+            if (m.lcolidx[e] <= r) { gc.push_back(m.lcolidx[e]); tp[m.lcolidx[e] + 1]++; }
+        gp[r + 1] = (int)gc.size();
+        std::sort(gc.begin() + gp[r], gc.end());
+        m.gcnt[r] = gp[r + 1] - gp[r];
         m.gmax = std::max(m.gmax, m.gcnt[r]);
     }
-    sell_slices(rows, m.sg);
+    const std::vector<int> none(gc.size(), -1);
+    sell_slices(n, gp, gc, none.data(), m.sg);
+    // its transpose, rows in ascending order
+    for (int r = 0; r < n; r++) tp[r + 1] += tp[r];
+    std::vector<int> fill(tp.begin(), tp.end() - 1), tc(gc.size()), ts(gc.size());
     for (int r = 0; r < n; r++)
-        for (int e = 0; e < m.gcnt[r]; e++)
-            trows[rows[r][e].first].push_back({r, m.sg.ptr[r / 32] + 32 * e + (r & 31)});
-    sell_slices(trows, m.st);
+        for (int e = 0; e < m.gcnt[r]; e++) {
+            const int q = fill[gc[gp[r] + e]]++;
+            tc[q] = r;
+            ts[q] = m.sg.ptr[r / 32] + 32 * e + (r & 31);
+        }
+    sell_slices(n, tp, tc, ts.data(), m.st);
 }
 
 static void layout_order(MeshHost& m)
@@ -696,6 +702,39 @@ Mesh::~Mesh()
     }
 }
 
+PartSize Mesh::part_size(int cs)
+{
+    TG_CHECK(cs == 1 || cs == 2 || cs == 4 || cs == 8 || cs == 16, TG_ERR_ARG, "cluster size");
+    std::lock_guard<std::mutex> lk(part_mu);
+    const int n = h.n, ns = (n + 31) / 32;
+    auto first = [&](int r, int c) { return std::min(n, (int)((long long)ns * r / c) * 32); };
+    if (reach.empty()) {
+        // the sixteenths of the rows that refer to each row; the ranges of fewer
+        // CTAs are unions of them
+        reach.assign(n, 0);
+        for (int r = 0; r < 16; r++)
+            for (int i = first(r, 16); i < first(r + 1, 16); i++)
+                for (int e = h.lrowptr[i]; e < h.lrowptr[i + 1]; e++) reach[h.lcolidx[e]] |= (unsigned short)(1u << r);
+    }
+    PartSize S{};
+    std::vector<int> halo(cs, 0);
+    const int w = 16 / cs;
+    for (int r = 0; r < cs; r++) {
+        const int r0 = first(r, cs), r1 = first(r + 1, cs);
+        int push = 0;
+        for (int i = r0; i < r1; i++)
+            for (int q = 0; q < cs; q++)
+                if (q != r && (reach[i] >> (q * w) & ((1u << w) - 1))) { halo[q]++; push++; }
+        const int s0 = (int)((long long)ns * r / cs), s1 = (int)((long long)ns * (r + 1) / cs);
+        S.own = std::max(S.own, r1 - r0);
+        S.npush = std::max(S.npush, push);
+        S.nsl = std::max(S.nsl, s1 - s0);
+        S.len = std::max(S.len, h.sa.ptr[s1] - h.sa.ptr[s0] + h.sg.ptr[s1] - h.sg.ptr[s0] + h.st.ptr[s1] - h.st.ptr[s0]);
+    }
+    for (int r = 0; r < cs; r++) S.slots = std::max(S.slots, first(r + 1, cs) - first(r, cs) + halo[r]);
+    return S;
+}
+
 const PartDev* Mesh::part(int cs)
 {
     std::lock_guard<std::mutex> lk(part_mu);
@@ -703,8 +742,7 @@ const PartDev* Mesh::part(int cs)
     if (it != parts.end()) return it->second.get();
     const int n = h.n, ns = (n + 31) / 32;
     auto P = std::make_unique<PartDev>();
-    P->cs = cs;
-    P->slots = P->own = P->len = P->nsl = 0;
+    P->slots = 0;
     std::vector<unsigned short> ca(h.sa.col.size()), cg(h.sg.col.size()), ct(h.st.col.size());
     std::vector<std::vector<uint2>> places(cs);
     auto owner = [&](int row) {
@@ -725,9 +763,6 @@ const PartDev* Mesh::part(int cs)
             }
         std::sort(halo.begin(), halo.end());
         P->slots = std::max(P->slots, own + (int)halo.size());
-        P->own = std::max(P->own, own);
-        P->nsl = std::max(P->nsl, s1 - s0);
-        P->len = std::max(P->len, h.sa.ptr[s1] - h.sa.ptr[s0] + h.sg.ptr[s1] - h.sg.ptr[s0] + h.st.ptr[s1] - h.st.ptr[s0]);
         if (own + halo.size() > 65535) { parts[cs] = nullptr; return nullptr; }
         for (int i = r0; i < r1; i++) slot[i] = i - r0;
         for (size_t t = 0; t < halo.size(); t++) {
@@ -747,11 +782,9 @@ const PartDev* Mesh::part(int cs)
     }
     std::vector<uint2> push;
     std::vector<int> pofs(cs + 1, 0);
-    P->npush = 0;
     for (int r = 0; r < cs; r++) {
         push.insert(push.end(), places[r].begin(), places[r].end());
         pofs[r + 1] = (int)push.size();
-        P->npush = std::max(P->npush, (int)places[r].size());
     }
     P->ca = upload(ca);
     P->cg = upload(cg);
@@ -776,12 +809,18 @@ const IcPartDev* Mesh::ic_part(int cs, int o)
     const ICHost& c = h.ic[o];
     auto I = std::make_unique<IcPartDev>();
     std::vector<int> owner(n), place(n);
-    std::vector<std::vector<unsigned>> at(n);  // halo places of each row
-    std::vector<int> first(cs + 1);
+    std::vector<int> first(cs + 1), ap(n + 1, 0);  // halo places of row p: at[ap[p]] ..
     for (int r = 0; r <= cs; r++) first[r] = std::min(n, (int)((long long)ns * r / cs) * 32);
     for (int r = 0; r < cs; r++) {
         for (int i = first[r]; i < first[r + 1]; i++) owner[i] = r;
-        for (const uint2& t : P->copies[r]) at[first[r] + t.x].push_back(t.y);
+        for (const uint2& t : P->copies[r]) ap[first[r] + t.x + 1]++;
+    }
+    for (int i = 0; i < n; i++) ap[i + 1] += ap[i];
+    std::vector<unsigned> at(ap[n]);
+    {
+        std::vector<int> fill(ap.begin(), ap.end() - 1);
+        for (int r = 0; r < cs; r++)
+            for (const uint2& t : P->copies[r]) at[fill[first[r] + t.x]++] = t.y;
     }
     auto sweep = [&](bool fwd, IcSweepDev& w) {
         const std::vector<int>&ptr = fwd ? c.fwd_lev_ptr : c.bwd_lev_ptr, &rows = fwd ? c.fwd_lev_rows : c.bwd_lev_rows;
@@ -823,7 +862,7 @@ const IcPartDev* Mesh::ic_part(int cs, int o)
                         col[off + (size_t)e * nr + s] = (unsigned short)place[fwd ? c.Lcolidx[q] : c.Urow[q]];
                         src[off + (size_t)e * nr + s] = fwd ? q : c.Umap[q];
                     }
-                    for (unsigned t : at[p]) push.push_back(uint2{(unsigned)place[p], t});
+                    for (int t = ap[p]; t < ap[p + 1]; t++) push.push_back(uint2{(unsigned)place[p], at[t]});
                 }
                 pl[(size_t)r * nlev + l].y = (int)push.size() - pl[(size_t)r * nlev + l].x;
             }

@@ -133,15 +133,20 @@ struct MeshDev {
     int* gcnt;
 };
 
+// The largest of a split's CTAs (part): gather-buffer slots and own rows, slices
+// and entries of the three matrices, halo copies of its rows
+struct PartSize {
+    int slots, own, nsl, len, npush;
+    bool ok() const { return slots <= 65535; }  // slots are 16 bits
+};
+
 // The rows split into cs contiguous ranges (of whole slices), one per CTA of a
 // cluster: the slice columns as slots of the CTA's buffers (own rows, then its
 // halo, the other rows its rows refer to, ascending), and the copies of its
 // rows in other halos, {own slot, rank << 16 | slot there}, from pofs[rank].
 struct PartDev {
-    int cs, slots, own;                    // slots and own rows: the largest of the CTAs
-    int len, nsl;                          // entries of the three matrices and slices: the same
+    int slots;                             // the largest of the CTAs
     unsigned short *ca, *cg, *ct;          // columns of A, G and G^T
-    int npush;                             // halo copies of a CTA: the largest of the CTAs
     int* pofs;
     uint2* push;
     std::vector<std::vector<int>> halo;    // host: halo rows of each CTA
@@ -168,8 +173,11 @@ struct Mesh {
     MeshHost h;
     MeshDev d{};
     int device = 0;
-    // the split for clusters of cs CTAs, built at its first use; null when a
-    // CTA's slots pass 16 bits
+    // the sizes of the split for clusters of cs (1, 2, 4, 8, 16) CTAs, from one
+    // pass over the pattern for all of them: what a choice of cs needs
+    PartSize part_size(int cs);
+    std::vector<unsigned short> reach;
+    // the split itself, built at its first use; null when a CTA's slots pass 16 bits
     const PartDev* part(int cs);
     std::mutex part_mu;
     std::map<int, std::unique_ptr<PartDev>> parts;

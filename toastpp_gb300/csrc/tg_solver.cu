@@ -574,10 +574,10 @@ struct Engine {
         double tbest = 1e300;
         for (int cs = 1; cs <= 8; cs *= 2) {
             if (mesh->d.n / cs > 16384 || (cs > 1 && mesh->d.n / cs < 200)) continue;
-            const PartDev* P = mesh->part(cs);
-            if (!P) continue;
+            const PartSize P = mesh->part_size(cs);
+            if (!P.ok()) continue;
             for (int lv = 1; lv * (int)sizeof(V) <= 16 && (lv == 1 || lv < 2 * k); lv *= 2) {
-                const size_t sm = ic_smem(*P, lv);
+                const size_t sm = ic_smem(P, lv);
                 if (sm > CL_SMEM) continue;
                 auto kern = ic_cluster_kernel_of<V>(lv);
                 allow_smem((const void*)kern);
@@ -595,9 +595,18 @@ struct Engine {
         return ic_shapes[{k, ico}] = best;
     }
 
+    // sizes of the split of the last shape, kept: part_size counts them anew
+    PartSize ic_size(int cs)
+    {
+        if (psz_cs != cs) { psz = mesh->part_size(cs); psz_cs = cs; }
+        return psz;
+    }
+    PartSize psz{};
+    int psz_cs = 0;
+
     // shared memory of a CTA: the vector, then levels and rows of both sweeps
-    size_t ic_vec_bytes(const PartDev& P, int lv) const { return ((size_t)P.slots * lv * sizeof(V) + 15) / 16 * 16; }
-    size_t ic_smem(const PartDev& P, int lv)
+    size_t ic_vec_bytes(const PartSize& P, int lv) const { return ((size_t)P.slots * lv * sizeof(V) + 15) / 16 * 16; }
+    size_t ic_smem(const PartSize& P, int lv)
     {
         const ICHost& c = ic_host();
         const size_t nlev = c.fwd_lev_ptr.size() + c.bwd_lev_ptr.size() - 2;
@@ -690,7 +699,7 @@ struct Engine {
     {
         const auto sh = ic_shape(k);
         const IcPartDev* I = mesh->ic_part(sh.second, ico);
-        const PartDev& P = *mesh->part(sh.second);
+        const PartSize P = ic_size(sh.second);
         IcClArgs<V> a;
         a.mofs = (int)ic_vec_bytes(P, sh.first);
         a.f = I->f; a.b = I->b;
@@ -2480,14 +2489,12 @@ static ClShape resident_shape(tg_solver s, int k)
     for (int cs = 1; cs <= CL_MAXCS; cs *= 2) {
         if (cs > 1 && n / cs < 150) break;
         if (n / cs > 8000) continue;
-        const PartDev* part = mesh->part(cs);
-        if (!part) continue;
-        const PartDev& P = *part;
+        const PartSize P = mesh->part_size(cs);
+        if (!P.ok()) continue;
         for (int lv = 1; lv * sizeof(V32) <= 16 && (lv == 1 || lv < 2 * k); lv *= 2) {
             ClShape c;
             c.lv = lv;
             c.cs = cs;
-            c.part = part;
             // shared memory: vectors, halo copies, slice pointers, and the matrices where they fit
             const size_t mh = ((size_t)(3 * P.slots + P.own) * lv * sizeof(V32) + 15) / 16 * 16;
             const size_t mp = mh + (size_t)P.npush * 8, mv = (mp + (size_t)3 * (P.nsl + 1) * 4 + 15) / 16 * 16;
@@ -2514,6 +2521,7 @@ static ClShape resident_shape(tg_solver s, int k)
             if (t < tbest) { tbest = t; best = c; }
         }
     }
+    if (best.cs) best.part = mesh->part(best.cs);
     return best;
 }
 
@@ -2550,7 +2558,7 @@ static int solve_resident(tg_solver s, int k, const V64* B, V64* X, ColState* co
     const ClShape& sh = shape_of<V64, V32>(s, k);
     const unsigned ng = cdiv_u(k, sh.lv);
     ResArgs<V64, V32> a;
-    a.n = m.n; a.k = k; a.cs = sh.cs; a.slots = sh.part->slots; a.own = sh.part->own;
+    a.n = m.n; a.k = k; a.cs = sh.cs; a.slots = sh.part->slots;
     a.msm = sh.msm; a.mofs_val = sh.mofs_val; a.mofs_col = sh.mofs_col; a.mofs_ptr = sh.mofs_ptr;
     a.A = {m.sa.ptr, sh.part->ca, s->sa32.as<V32>()};
     a.G = {m.sg.ptr, sh.part->cg, s->sg32.as<V32>()};
