@@ -113,6 +113,14 @@ static inline void launch_cluster(void (*k)(KArgs...), unsigned ng, int cs, int 
 
 constexpr size_t CL_SMEM = 212 * 1024;  // dynamic shared memory of the cluster kernels at most
 
+static int sm_count()
+{
+    int dev = 0, nsm = 0;
+    TG_CUDA(cudaGetDevice(&dev));
+    TG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    return nsm;
+}
+
 // clusters of a kernel that the device runs at a time (0: the shape is refused)
 static int clusters_at_once(const void* kern, unsigned ng, int cs, int nt, size_t sm, cudaStream_t st)
 {
@@ -128,11 +136,8 @@ static int clusters_at_once(const void* kern, unsigned ng, int cs, int nt, size_
         }
         return at_once;
     }
-    int dev = 0, nsm = 0;
-    TG_CUDA(cudaGetDevice(&dev));
     TG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&at_once, kern, nt, sm));
-    TG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    return at_once * nsm;
+    return at_once * sm_count();
 }
 
 // Raise a kernel's dynamic shared-memory limit to the device's opt-in
@@ -2044,7 +2049,7 @@ static void direct_factor(tg_solver s)
                 ncm = std::max(ncm, d.nc);
             }
             // parts of a front: enough CTAs for the chip, not more than its columns give work
-            const unsigned parts = std::max(1u, std::min((unsigned)(fm + 7) / 8, 304u / std::max(1u, nf)));
+            const unsigned parts = std::max(1u, std::min((unsigned)(fm + 7) / 8, 2u * sm_count() / std::max(1u, nf)));
             launch(direct_assemble_kernel<V>, dim3(nf, parts), 256, 0, s->stream, fr, ids, s->dkids.as<int>(),
                    s->drel.as<int>(), s->dent.as<DEntry>(), A, F);
             for (int p0 = 0; p0 < ncm; p0 += DP) {
@@ -3090,14 +3095,14 @@ static void grid_prep(tg_solver s, int nq, const V64* F, int nm, const V64* A, C
 
 // Detectors per block of the grid and element Jacobian kernels, for a grid of
 // so many blocks a chunk: no more than a tile holds, and where the blocks leave
-// SMs idle fewer, down to 4 (a block's sources are loaded once per chunk; 1216
-// = 152 SMs x 8 blocks).  FP64, 100 MHz, one chunk against this rule: disc with
+// SMs idle fewer, down to 4 (a block's sources are loaded once per chunk): 8
+// blocks an SM.  FP64, 100 MHz, one chunk against this rule: disc with
 // 40^2 pixels and 15 x 17 links 149 -> 79 us, 61-ring disc with 31 x 33 232 ->
-// 174 us, 24^3 with 40 x 41 947 -> 784 us; 1216 / 2432 / 4864 blocks within the
+// 174 us, 24^3 with 40 x 41 947 -> 784 us; 8 / 16 / 32 blocks an SM within the
 // runs' difference but for FP32 elements (2D, 31 x 33: 87 / 92 / 96 us).
 static int detector_chunk(int nm, size_t blocks)
 {
-    const size_t want = cdiv_u(1216, std::max<size_t>(1, blocks));
+    const size_t want = cdiv_u((size_t)sm_count() * 8, std::max<size_t>(1, blocks));
     const size_t chunks = std::max<size_t>(1, std::min<size_t>(want, cdiv_u(nm, 4)));
     return std::max(1, std::min(LT, (int)cdiv_u(nm, chunks)));
 }
