@@ -42,9 +42,6 @@ static std::atomic<long long> g_nlaunch{0};
 // SpMM variant chosen per (mesh, value type, k), shared by every solver of the process
 static std::mutex g_tune_mu;
 static std::map<std::tuple<long long, int, int>, int> g_tune;
-// IC apply variant (cluster sweep or per-level launches) per (mesh and
-// pattern, value type, k), chosen like the SpMM variant
-static std::map<std::tuple<long long, int, int>, bool> g_ictune;
 static std::string g_tune_log;  // one line per decision: candidates with their best launch time
 static const char* spmm_name(int v)
 {
@@ -378,8 +375,10 @@ struct Engine {
     };
     std::map<std::pair<int, int>, ClValues> clv;
     long long fver = 0;        // version of the factor behind L
-    // (k, ordering) -> (columns, CTAs) of a cluster; CTAs 0: none fits
-    std::map<std::pair<int, int>, std::pair<int, int>> ic_shapes;
+    // columns and CTAs of a cluster of the cluster sweep (CTAs 0: none fits), and
+    // how many times the chip is filled; per (k, ordering)
+    struct IcShape { int lv = 0, cs = 0, waves = 0; };
+    std::map<std::pair<int, int>, IcShape> ic_shapes;
     Bounce bnc;
     GraphCache graphs;
 
@@ -571,11 +570,11 @@ struct Engine {
 
     // Columns and CTAs of a cluster of the cluster sweep: all columns at once on
     // the chip, with the fewest rows per CTA; (0, 0) where nothing fits
-    std::pair<int, int> ic_shape(int k)
+    IcShape ic_shape(int k)
     {
         auto it = ic_shapes.find({k, ico});
         if (it != ic_shapes.end()) return it->second;
-        std::pair<int, int> best{0, 0};
+        IcShape best;
         double tbest = 1e300;
         for (int cs = 1; cs <= 8; cs *= 2) {
             if (mesh->d.n / cs > 16384 || (cs > 1 && mesh->d.n / cs < 200)) continue;
@@ -593,7 +592,7 @@ struct Engine {
                 const ICHost& c = ic_host();
                 const double lv_rows = (double)mesh->d.n / std::max<size_t>(1, c.fwd_lev_ptr.size() - 1) / cs;
                 const double t = waves * ((cs > 1 ? 2.0 : 1.0) + std::ceil(lv_rows / IC_NT) * lv * sizeof(S) / 4.0);
-                if (t < tbest) { tbest = t; best = {lv, cs}; }
+                if (t < tbest) { tbest = t; best = {lv, cs, waves}; }
             }
         }
         if (ic_shapes.size() >= 64) ic_shapes.clear();
@@ -634,85 +633,54 @@ struct Engine {
     // before a solve (and outside a capture): the cluster sweep's entries, where k columns use it
     void ic_prepare(int k)
     {
-        if (precon == 2 && ic_clustered(k)) ic_cluster_values(ic_shape(k).second);
+        if (precon == 2 && ic_clustered(k)) ic_cluster_values(ic_shape(k).cs);
     }
 
-    // TOASTGPU_IC_PERSISTENT=0 / 1: per-level launches / the cluster sweep
-    int ic_forced() const
-    {
-        const char* e = getenv("TOASTGPU_IC_PERSISTENT");
-        return e && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : -1;
-    }
+    // Whether the apply of k columns is one launch on clusters (tg_resident.cu) or
+    // a launch per level; both compute every row with the same sums in the same
+    // order (bit-identical results).  By a rule, not by timing them: a choice timed
+    // at the first apply held for the process, whatever else the GPU ran just then
+    // (702 us for 106 columns beside 178 for 192 of one mesh).  The levels are
+    // launch-bound, 2 to 8 us each, and their time hardly grows with the columns;
+    // the clusters' grows with the rows of a level that each SM has to walk, rows *
+    // columns / (256 threads * SMs).  Measured both ways on 21 meshes (217 to 85k
+    // nodes, discs, cylinders, boxes), 1 to 256 columns, the four value types, 715
+    // applies: the lines cross at about 4 rounds, for complex FP32, whose levels
+    // are the cheapest for their work, at 1.4 (12.5k-node disc: 30 columns;
+    // 30.8k-node cylinder: 19); past that the levels win by up to 7x (box of 85k
+    // nodes, 160 complex FP32 columns: 268 against 1909 us), below it the clusters by
+    // up to 8 (1k-node cylinder, 256 complex FP64 columns: 141 against 1093 us).
+    // Where the columns need the chip more than once and a CTA has more than 6500
+    // rows, the levels (85k nodes, 32 FP64 columns: 467 against 820 us).  The rule
+    // loses 0.6 % of the time to the better of both over all of them, 42 % at worst.
+    // TOASTGPU_IC_PERSISTENT=0 / 1: per-level launches / the cluster sweep.
     bool ic_clustered(int k)
     {
-        if (!ic_shape(k).second) return false;
-        const int f = ic_forced();
-        if (f >= 0) return f == 1;
-        const auto key = std::make_tuple(mesh->uid * 4 + ico, (int)sizeof(V) * 2 + (int)vt<V>::cplx, k);
-        std::lock_guard<std::mutex> g(g_tune_mu);
-        auto it = g_ictune.find(key);
-        return it != g_ictune.end() && it->second;
+        const IcShape sh = ic_shape(k);
+        if (!sh.cs) return false;
+        const char* e = getenv("TOASTGPU_IC_PERSISTENT");
+        if (e && (e[0] == '0' || e[0] == '1')) return e[0] == '1';
+        const double lines = vt<V>::cplx && sizeof(V) == 8 ? 1.4 : 4.0;
+        const ICHost& c = ic_host();
+        const double rows = 2.0 * mesh->d.n / (double)(c.fwd_lev_ptr.size() + c.bwd_lev_ptr.size() - 2);
+        return rows * k <= lines * IC_NT * sm_count() && (sh.waves == 1 || mesh->d.n / sh.cs <= 6500);
     }
 
-    // The cluster sweep (one launch, tg_resident.cu) or a launch per level: both
-    // compute every row with the same sums in the same order (bit-identical
-    // results).  The first apply of a (mesh, ordering, value type, k) in the
-    // process times both (best of three, in a graph each) and keeps the faster
-    // for the process.
-    bool ic_use_cluster(int k, const V* in, V* out, const ColState* cst)
-    {
-        if (!ic_shape(k).second) return false;
-        const int f = ic_forced();
-        if (f >= 0) return f == 1;
-        const auto key = std::make_tuple(mesh->uid * 4 + ico, (int)sizeof(V) * 2 + (int)vt<V>::cplx, k);
-        {
-            std::lock_guard<std::mutex> g(g_tune_mu);
-            auto it = g_ictune.find(key);
-            if (it != g_ictune.end()) return it->second;
-        }
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        TG_CUDA(cudaStreamIsCapturing(st, &cs));
-        if (cs != cudaStreamCaptureStatusNone || in == out) return false;
-        float best[2] = {1e30f, 1e30f};
-        cudaEvent_t ev[2];
-        for (auto& x : ev) TG_CUDA(cudaEventCreate(&x));
-        for (int r = 0; r < 4; r++)
-            for (int v = 0; v < 2; v++) {
-                if (v) ic_cluster_values(ic_shape(k).second);
-                TG_CUDA(cudaEventRecord(ev[0], st));
-                ic_apply_variant(k, in, out, cst, v == 1);
-                TG_CUDA(cudaEventRecord(ev[1], st));
-                TG_CUDA(cudaEventSynchronize(ev[1]));
-                float ms = 0.f;
-                TG_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
-                if (r) best[v] = std::min(best[v], ms);  // the first round captures the graphs
-            }
-        for (auto& x : ev) cudaEventDestroy(x);
-        const bool p = best[1] < best[0];
-        std::lock_guard<std::mutex> g(g_tune_mu);
-        auto res = g_ictune.emplace(key, p);
-        if (res.second) {
-            char line[200];
-            snprintf(line, sizeof line, "mesh %lld %s k=%d: ic per-level %.1fus cluster %.1fus -> %s\n",
-                     (long long)mesh->uid, vt_name<V>(), k, best[0] * 1e3f, best[1] * 1e3f, p ? "cluster" : "per-level");
-            g_tune_log += line;
-        }
-        return res.first->second;
-    }
+    // the choice's part of a captured iteration's key
+    const void* ic_tag(int k) { return (const void*)(size_t)(precon == 2 && ic_clustered(k)); }
 
     void launch_ic_cluster(int k, const V* in, V* out, const ColState* cst)
     {
         const auto sh = ic_shape(k);
-        const IcPartDev* I = mesh->ic_part(sh.second, ico);
-        const PartSize P = ic_size(sh.second);
+        const IcPartDev* I = mesh->ic_part(sh.cs, ico);
+        const PartSize P = ic_size(sh.cs);
         IcClArgs<V> a;
-        a.mofs = (int)ic_vec_bytes(P, sh.first);
+        a.mofs = (int)ic_vec_bytes(P, sh.lv);
         a.f = I->f; a.b = I->b;
-        const ClValues& c = clv[{sh.second, ico}];
+        const ClValues& c = clv[{sh.cs, ico}];
         a.vf = c.f.template as<V>(); a.vb = c.b.template as<V>(); a.dinv = dinv;
-        a.in = in; a.out = out; a.n = mesh->d.n; a.k = k; a.cs = sh.second; a.st = cst;
-        launch_cluster(ic_cluster_kernel_of<V>(sh.first), cdiv_u(k, sh.first), sh.second, IC_NT,
-                       ic_smem(P, sh.first), st, a);
+        a.in = in; a.out = out; a.n = mesh->d.n; a.k = k; a.cs = sh.cs; a.st = cst;
+        launch_cluster(ic_cluster_kernel_of<V>(sh.lv), cdiv_u(k, sh.lv), sh.cs, IC_NT, ic_smem(P, sh.lv), st, a);
     }
 
     // out = M^-1 in for the IC(0) preconditioner: one launch on clusters, or the
@@ -720,12 +688,12 @@ struct Engine {
     // replayed as one graph
     void ic_apply(int k, const V* in, V* out, const ColState* cst)
     {
-        const bool cluster = ic_use_cluster(k, in, out, cst);
+        const bool cluster = in != out && ic_clustered(k);
         if (cluster) {
             cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
             TG_CUDA(cudaStreamIsCapturing(st, &cs));
             // (in a capture the values are in place: the solve began with ic_prepare)
-            if (cs == cudaStreamCaptureStatusNone) ic_cluster_values(ic_shape(k).second);
+            if (cs == cudaStreamCaptureStatusNone) ic_cluster_values(ic_shape(k).cs);
         }
         ProfScope ps(prof, PC_SWEEP, st);
         ic_apply_variant(k, in, out, cst, cluster);
@@ -1005,7 +973,7 @@ struct Engine {
                                                        vec(0, nk), vec(1, nk), vec(2, nk), vec(3, nk), vec(4, nk),
                                                        vec(5, nk), vec(6, nk), vec(7, nk), A, L, Lef, Leb, dinv, idiag,
                                                        (const void*)(size_t)precon, (const void*)(size_t)ico,
-                                                       parts(k, 2)};
+                                                       parts(k, 2), ic_tag(k)};
                 graphs.run(st, ukey, [&] {
                     for (int u = 0; u < 4; u++) bicg_iter(k, X, cst, 0);
                 });
@@ -1049,7 +1017,7 @@ struct Engine {
         const bool unit_graph = !(prof && prof->mask);
         const std::vector<const void*> ukey = {(const void*)"pcg-unit", (const void*)(size_t)k, X, cst, R, D, Q, Z, A,
                                                L, Lef, Leb, dinv, idiag, (const void*)(size_t)precon,
-                                               (const void*)(size_t)ico, part.p};
+                                               (const void*)(size_t)ico, part.p, ic_tag(k)};
         for (int it = 0; it < maxit;) {
             if (unit_graph && it >= 4 && (it & 3) == 0 && it + 4 <= maxit) {
                 graphs.run(st, ukey, [&] {
@@ -2389,7 +2357,7 @@ static void solve_reliable(tg_solver s, int k, const V64* B, V64* X, ColState* c
     const std::vector<const void*> ukey = {(const void*)"cocg-unit", (const void*)(size_t)k, X32, ci, R32,
                                            e32.vec(0, nk), e32.vec(1, nk), e32.vec(2, nk), e32.vec(3, nk),
                                            e32.A, e32.L, e32.Lef, e32.Leb, e32.dinv, (const void*)(size_t)e32.ico,
-                                           e32.part.p};
+                                           e32.part.p, e32.ic_tag(k)};
     int it = 0;
     bool pending = false;  // COCG: the second half (z, beta, p) of the last iteration
     for (;;) {
