@@ -174,16 +174,17 @@ __global__ void __launch_bounds__(DP * DP) direct_update_kernel(const DFront* __
 
 // Forward solve of a front: w = [b of its columns; 0] plus the children's
 // parts, y = L^-1 w on its columns (to X), the rest stays in w for its parent.
-// CTA = (front, DKC right-hand sides); w: [front rows][k].
+// CTA = (front of nf, DKC right-hand sides), in one grid dimension; w: [front
+// rows][k].
 template <class V>
 __global__ void __launch_bounds__(256) direct_fwd_kernel(const DFront* __restrict__ fr, const int* __restrict__ ids,
                                                         const int* __restrict__ kids, const int* __restrict__ rel,
                                                         const int* __restrict__ rows, const V* __restrict__ vals,
-                                                        const V* __restrict__ blk, int k, const V* __restrict__ B,
+                                                        const V* __restrict__ blk, int nf, int k, const V* __restrict__ B,
                                                         V* X, V* W)
 {
-    const DFront d = fr[ids[blockIdx.x]];
-    const int f = d.nc + d.nr, c0 = blockIdx.y * DKC, kc = min(DKC, k - c0), tid = threadIdx.x, nt = blockDim.x;
+    const DFront d = fr[ids[blockIdx.x % nf]];
+    const int f = d.nc + d.nr, c0 = blockIdx.x / nf * DKC, kc = min(DKC, k - c0), tid = threadIdx.x, nt = blockDim.x;
     const V* F = vals + d.off;
     V* w = W + (size_t)d.w0 * k + c0;
     const int* rw = rows + d.w0;
@@ -234,11 +235,12 @@ __global__ void __launch_bounds__(256) direct_fwd_kernel(const DFront* __restric
 template <class V>
 __global__ void __launch_bounds__(256) direct_bwd_kernel(const DFront* __restrict__ fr, const int* __restrict__ ids,
                                                         const int* __restrict__ rows, const V* __restrict__ vals,
-                                                        const V* __restrict__ blk, const V* __restrict__ dinv, int k,
+                                                        const V* __restrict__ blk, const V* __restrict__ dinv, int nf,
+                                                        int k,
                                                         V* X, V* W)
 {
-    const DFront d = fr[ids[blockIdx.x]];
-    const int f = d.nc + d.nr, c0 = blockIdx.y * DKC, kc = min(DKC, k - c0), tid = threadIdx.x, nt = blockDim.x;
+    const DFront d = fr[ids[blockIdx.x % nf]];
+    const int f = d.nc + d.nr, c0 = blockIdx.x / nf * DKC, kc = min(DKC, k - c0), tid = threadIdx.x, nt = blockDim.x;
     const V* F = vals + d.off;
     V* w = W + (size_t)d.w0 * k + c0;
     const int* rw = rows + d.w0;

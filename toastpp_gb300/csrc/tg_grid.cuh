@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(128) grid_jacobian_kernel(int slen, int nq, in
 // numbering.  ysc[l] = -1 / y for LOG data, -1 for LINEAR.  J: complex
 // (2 nQM) x (2 ne) rows -Re / -Im, kappa at column ne + e; real (2 nQM) x ne
 // [mua ; kappa].
-// blockIdx.z: chunks of mc detectors, at most LT.
+// blockIdx.z: chunks of mc detectors, at most LT, from detector mb on.
 // FP32 is bound by instruction issue, then by the J stream (38.9k tetrahedra,
 // 80 x 80 links, 4 GB: 838 -> 734 us a call, 5.4 TB/s), FP64 by its pipe (21.1
 // -> 17.6 ms; 9 complex products a link are 15.4).  8 sources a group: the detector's
@@ -448,11 +448,11 @@ __global__ void __launch_bounds__(128) element_jacobian_kernel(MeshDev m, int nq
                                                                const V* __restrict__ F, const V* __restrict__ A,
                                                                const int* __restrict__ pair,
                                                                const V* __restrict__ ysc, JT* __restrict__ J,
-                                                               int mc)
+                                                               int mc, int mb)
 {
     using LS = LinkSum<V>;
     __shared__ LinkTile<V, GQ> tile;
-    const int q0 = blockIdx.y * GQ, m0 = blockIdx.z * mc, m1 = min(m0 + mc, nm);
+    const int q0 = blockIdx.y * GQ, m0 = mb + blockIdx.z * mc, m1 = min(m0 + mc, nm);
     constexpr bool CPLX = vt<V>::cplx;
     const long long cols = CPLX ? 2 * (long long)m.ne : (long long)m.ne, half = nqm * cols;
     tile.fill(m0, m1, q0, nq, nm, pair, ysc, cols, 0);

@@ -2054,13 +2054,14 @@ static void direct_sweeps(tg_solver s, int k, const V* B, V* X)
         for (int h = 0; h < 2 * nl; h++) {
             const int l = h < nl ? h : 2 * nl - 1 - h;
             const int* ids = s->dids.as<int>() + c.level[l];
-            const dim3 g((unsigned)(c.level[l + 1] - c.level[l]), cdiv_u(k, DKC));
+            const int nf = c.level[l + 1] - c.level[l];
+            const unsigned g = (unsigned)nf * cdiv_u(k, DKC);
             if (h < nl)
                 launch(direct_fwd_kernel<V>, g, 256, 0, s->stream, fr, ids, s->dkids.as<int>(), s->drel.as<int>(),
-                       s->drows.as<int>(), F, blk, k, B, X, W);
+                       s->drows.as<int>(), F, blk, nf, k, B, X, W);
             else
-                launch(direct_bwd_kernel<V>, g, 256, 0, s->stream, fr, ids, s->drows.as<int>(), F, blk, dinv, k, X,
-                       W);
+                launch(direct_bwd_kernel<V>, g, 256, 0, s->stream, fr, ids, s->drows.as<int>(), F, blk, dinv, nf, k,
+                       X, W);
         }
     });
 }
@@ -3201,13 +3202,15 @@ static void element_jac_run(tg_solver s, int nq, const V64* F, int nm, const V64
     constexpr int GQ = 8, TB = 128;
     const unsigned ex = cdiv_u(m.ne, TB), ey = cdiv_u(nq, GQ);
     const int mc = detector_chunk(nm, (size_t)ex * ey);
-    const dim3 eg(ex, ey, cdiv_u(nm, mc));
-    if (m.dim == 3)
-        launch(element_jacobian_kernel<C, JT, GQ, 4>, eg, TB, 0, s->stream, m, nq, nm, nqm, Fc, Ac, (const int*)pr,
-               (const C*)ysc, (JT*)Jd, mc);
-    else
-        launch(element_jacobian_kernel<C, JT, GQ, 3>, eg, TB, 0, s->stream, m, nq, nm, nqm, Fc, Ac, (const int*)pr,
-               (const C*)ysc, (JT*)Jd, mc);
+    for (int m0 = 0; m0 < nm; m0 += mc * 65535) {  // a grid's z extent at a time
+        const dim3 eg(ex, ey, std::min(65535u, cdiv_u(nm - m0, mc)));
+        if (m.dim == 3)
+            launch(element_jacobian_kernel<C, JT, GQ, 4>, eg, TB, 0, s->stream, m, nq, nm, nqm, Fc, Ac, (const int*)pr,
+                   (const C*)ysc, (JT*)Jd, mc, m0);
+        else
+            launch(element_jacobian_kernel<C, JT, GQ, 3>, eg, TB, 0, s->stream, m, nq, nm, nqm, Fc, Ac, (const int*)pr,
+                   (const C*)ysc, (JT*)Jd, mc, m0);
+    }
 }
 
 template <class V64, class V32>
