@@ -419,7 +419,8 @@ int tg_gradient(tg_solver s, tg_raster r, int nq, const double *qvec, int nm, co
                 tg_result *res);
 
 /* the SpMM autotuner's decisions so far: one text line per (mesh, value type,
-   columns) with every candidate kernel's best launch time and the choice.
+   columns) with every candidate kernel's best launch time and the choice; and
+   the cluster shapes of the resident solves.
    The environment variable TOASTGPU_SPMM_VARIANT (spmm_halo, spmm_vec,
    spmm_wide or spmm_dot) fixes the variant wherever it applies. */
 int tg_tuner_log(char *buf, int len);

@@ -2168,9 +2168,15 @@ static void build_resident(tg_solver s)
 // BiCGSTAB request in its default mode, runs as one resident kernel
 // (tg_resident.cu); a mesh with a node of more than 31 neighbours before it in
 // the layout does not fit its preconditioner's row solver.
+// TOASTGPU_RESIDENT=0 / 1: never / also past the block size of resident_fits.
+static int resident_forced()
+{
+    const char* e = getenv("TOASTGPU_RESIDENT");
+    return e && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : -1;
+}
 static bool resident_ok(tg_solver s)
 {
-    return s->precision == TG_PREC_MIXED && s->precon == TG_PRECON_ICH && s->inner_colour &&
+    return resident_forced() != 0 && s->precision == TG_PREC_MIXED && s->precon == TG_PRECON_ICH && s->inner_colour &&
            (s->method == TG_SOLVER_CG || (s->method == TG_SOLVER_BICGSTAB && s->reliable == 2)) &&
            s->mesh->h.gmax <= FSAI_MAXM;
 }
@@ -2457,7 +2463,6 @@ static ClShape resident_shape(tg_solver s, int k)
     Mesh* mesh = s->mesh;
     const int n = mesh->d.n;
     ClShape best;
-    if ((size_t)n * k * sizeof(V32) > ((size_t)20 << 20)) return best;
     const double f = std::max(1.0, (double)mesh->d.nnz / n / 7.0);  // matrix entries against a 2D mesh's
     double tbest = 1e300;
     for (int cs = 1; cs <= CL_MAXCS; cs *= 2) {
@@ -2507,6 +2512,12 @@ static __global__ void resident_results_kernel(int kf, const int* __restrict__ i
     if (j < kf) co[idx[j]] = cf[j];
 }
 
+template <class V32>
+static bool resident_fits(tg_solver s, int k)
+{
+    return resident_forced() == 1 || (size_t)s->mesh->d.n * k * sizeof(V32) <= ((size_t)20 << 20);
+}
+
 // the shape for k columns, chosen at their first solve
 template <class V64, class V32>
 static const ClShape& shape_of(tg_solver s, int k)
@@ -2515,6 +2526,12 @@ static const ClShape& shape_of(tg_solver s, int k)
     if (it == s->shapes.end()) {
         if (s->shapes.size() >= 64) s->shapes.clear();
         it = s->shapes.emplace(k, resident_shape<V64, V32>(s, k)).first;
+        const ClShape& c = it->second;
+        char line[160];
+        snprintf(line, sizeof line, "mesh %lld %s k=%d: resident solve, %d columns a cluster of %d CTAs\n",
+                 (long long)s->mesh->uid, vt_name<V32>(), k, c.lv, c.cs);
+        std::lock_guard<std::mutex> g(g_tune_mu);
+        if (c.cs && g_tune_log.find(line) == std::string::npos) g_tune_log += line;
     }
     return it->second;
 }
@@ -2589,7 +2606,7 @@ static void solve_nm(tg_solver s, int k, const V64* B, V64* X, ColState* co, boo
         e64.solve(s->method, k, B, X, co, zero_guess);
         return;
     }
-    if (resident_ok(s) && shape_of<V64, V32>(s, k).cs) {
+    if (resident_ok(s) && resident_fits<V32>(s, k) && shape_of<V64, V32>(s, k).cs) {
         if (!s->res_ready) build_resident<V64, V32>(s);
         V64* R = (V64*)s->tmp.ensure(nk * sizeof(V64));
         if (!zero_guess) {
