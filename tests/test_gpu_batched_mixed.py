@@ -116,3 +116,20 @@ def test_hub_with_many_neighbours(freq, oracle_mod):
     x, res = s.calc_fields(B)
     assert capi.launch_count() - c0 > 40
     assert all(r[1] == 0 for r in res) and all(rel2(x[c], X[c]) < 1e-10 for c in range(5))
+
+
+@pytest.mark.parametrize("freq,mb", [(0.0, 20), (100.0, 14)])
+def test_block_size_rule(freq, mb):
+    """Past the rule's line (20 MB of vector; 14 for complex values on a 3D mesh
+    of more than 18000 nodes) the batched kernels run, up to it the resident one."""
+    P = workloads.box(27, 27, 25, seed=1, nq=64, freq_mhz=freq)
+    assert P.n > 18000
+    gm = capi.Mesh(P.coords, P.elems)
+    cm, ck, ca, qvec, _ = gpu_problem_inputs(P, gm)
+    s = capi.FwdSolver(gm, "BICGSTAB", 1e-10, "ICH", P.complex, maxit=2, precision="mixed")
+    s.reset(cm, ck, ca, capi.omega_of(freq))
+    line = (mb << 20) // (P.n * (8 if P.complex else 4))
+    for k, resident in ((line, True), (line + 1, False)):
+        c0 = capi.launch_count()
+        s.calc_fields(qvec[np.arange(k) % len(qvec)])
+        assert (capi.launch_count() - c0 < 20) == resident, (k, capi.launch_count() - c0)

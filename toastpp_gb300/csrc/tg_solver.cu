@@ -2452,11 +2452,7 @@ static void solve_reliable(tg_solver s, int k, const V64* B, V64* X, ColState* c
 // per round of a CTA's rows a latency and a shared-memory part; it was fitted
 // to sweeps of every shape on discs of 217 to 12.5k nodes and cylinders of
 // 4.6k and 30.8k nodes with 5 to 160 columns, where its choice is within 8 %
-// of the best one.  cs = 0: no shape fits the shared memory, or the columns
-// are so many that the batched kernels, which read the matrices once for all
-// of them, are faster: the crossing is at 20 MB of vector on the 30.8k-node
-// cylinder (80 complex columns: 21.0 against 21.5 ms; 20: 7.4 against 14.6;
-// 160: 42 against 31).
+// of the best one.  cs = 0: no shape fits the shared memory.
 template <class V64, class V32>
 static ClShape resident_shape(tg_solver s, int k)
 {
@@ -2512,10 +2508,22 @@ static __global__ void resident_results_kernel(int kf, const int* __restrict__ i
     if (j < kf) co[idx[j]] = cf[j];
 }
 
+// Whether a block is small enough for the resident solve: its time grows with
+// the columns, while the batched kernels read the matrices once for all of them.
+// 20 MB of vector, or 14 MB on large 3D meshes with complex values.  Measured
+// both ways at 5 to 60 MB, resident against batched: complex, 19.6k-node cylinder
+// 12.9 / 15.3 ms at 14 MB and 22.1 / 19.6 at 20; 30.8k nodes 15.9 / 17.6 and 26.0 /
+// 20.8; 45k nodes 21.4 / 21.5 and 32.1 / 24.9; boxes of 33k and 47k nodes 13.8 /
+// 17.0 and 20.5 / 19.9, 18.9 / 20.7 and 25.5 / 22.9.  Smaller 3D meshes, discs and
+// real systems cross later or not at all (12.6k-node cylinder, complex: 18.0 / 19.6
+// at 20 MB and 52.8 / 56.2 at 60; 12.5k-node disc 19.0 / 34.3 and 55.6 / 110;
+// 30.8k-node cylinder, real: 27.5 / 35.8 and 76 / 94): there the line is low.
 template <class V32>
 static bool resident_fits(tg_solver s, int k)
 {
-    return resident_forced() == 1 || (size_t)s->mesh->d.n * k * sizeof(V32) <= ((size_t)20 << 20);
+    const MeshDev& m = s->mesh->d;
+    const bool large = vt<V32>::cplx && m.dim == 3 && m.n > 18000;
+    return resident_forced() == 1 || (size_t)m.n * k * sizeof(V32) <= (size_t)(large ? 14 : 20) << 20;
 }
 
 // the shape for k columns, chosen at their first solve
