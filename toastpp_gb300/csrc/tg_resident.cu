@@ -151,13 +151,13 @@ __device__ __forceinline__ Sc sc_mul(Sc a, Sc b)
     const float p = __fmul_rn(a.h, b.h);
     return sc_norm(p, __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.h, -p))));
 }
-__device__ __forceinline__ Sc sc_div(Sc a, Sc b)
+// a / b, with f = 1 / b.h: a quotient, and its remainder's
+__device__ __forceinline__ Sc sc_div(Sc a, Sc b, float f)
 {
-    const float q = a.h / b.h;
-    // a - q b, exact in its leading terms
-    const float r = __fmaf_rn(-q, b.l, __fmaf_rn(-q, b.h, a.h) + a.l);
-    return sc_norm(q, r / b.h);
+    const float q = __fmul_rn(a.h, f);
+    return sc_norm(q, __fmaf_rn(-q, b.l, __fmaf_rn(-q, b.h, a.h) + a.l) * f);
 }
+__device__ __forceinline__ Sc sc_div(Sc a, Sc b) { return sc_div(a, b, 1.f / b.h); }
 __device__ __forceinline__ Sc sc_scale(Sc a, float f) { return Sc{a.h * f, a.l * f}; }  // f: a power of two
 __device__ __forceinline__ Scc sc_scale(Scc a, float f) { return Scc{sc_scale(a.x, f), sc_scale(a.y, f)}; }
 // a conj(b) / |b|^2, with b scaled to between 1 and 2 first
@@ -170,8 +170,9 @@ __device__ __forceinline__ Scc sc_div(Scc a, Scc b)
     a = sc_scale(a, f);
     b = sc_scale(b, f);
     const Sc d = sc_add(sc_mul(b.x, b.x), sc_mul(b.y, b.y));
-    return Scc{sc_div(sc_add(sc_mul(a.x, b.x), sc_mul(a.y, b.y)), d),
-               sc_div(sc_add(sc_mul(a.y, b.x), sc_neg(sc_mul(a.x, b.y))), d)};
+    const float g = 1.f / d.h;
+    return Scc{sc_div(sc_add(sc_mul(a.x, b.x), sc_mul(a.y, b.y)), d, g),
+               sc_div(sc_add(sc_mul(a.y, b.x), sc_neg(sc_mul(a.x, b.y))), d, g)};
 }
 __device__ __forceinline__ bool sc_zero(Sc a) { return a.h == 0.f; }
 __device__ __forceinline__ bool sc_zero(Scc a) { return a.x.h == 0.f && a.y.h == 0.f; }
@@ -183,27 +184,65 @@ __device__ __forceinline__ cf sc_cast(Scc a) { return cf{a.x.h, a.y.h}; }
 // square root with non-negative real part
 __device__ __forceinline__ double ssqrt(double a) { return sqrt(a); }
 __device__ __forceinline__ cd ssqrt(cd z) { return csqrt_d(z); }
-__device__ __forceinline__ bool sfinite(double a) { return isfinite(a); }
-__device__ __forceinline__ bool sfinite(cd a) { return isfinite(a.x) && isfinite(a.y); }
 __device__ __forceinline__ bool sfinite(float a) { return isfinite(a); }
 __device__ __forceinline__ bool sfinite(cf a) { return isfinite(a.x) && isfinite(a.y); }
 
 // ---------------------------------------------------------------------------
-// 1 / d and 1 / sqrt(d), Re d > 0, for values that have been scaled to about 1:
-// an FP32 seed and two Newton steps in FP64.  (A row's pivots are one chain:
-// with FP64 divisions and square
-// roots it took 25 us on 217 nodes, 19 so, 10 in FP32.)
-__device__ __forceinline__ double nr_recip(double d)
+// An entry of a row's matrix: a real value as Sc, a complex one as (re, im) of
+// the high and of the low floats
+struct alignas(16) Pc {
+    f2x h, l;
+};
+template <class V> struct PairOf { using T = Sc; };
+template <> struct PairOf<cf> { using T = Pc; };
+__device__ __forceinline__ Scc p_sc(Pc a)
 {
-    double x = 1.f / (float)d;
-    x = fma(x, fma(-d, x, 1.0), x);
-    return fma(x, fma(-d, x, 1.0), x);
+    const float2 h = f2_unpack(a.h), l = f2_unpack(a.l);
+    return Scc{sc_norm(h.x, l.x), sc_norm(h.y, l.y)};
 }
-__device__ __forceinline__ cd nr_recip(cd d)
+__device__ __forceinline__ Pc p_sc(Scc a) { return Pc{f2_pack(a.x.h, a.y.h), f2_pack(a.x.l, a.y.l)}; }
+__device__ __forceinline__ void p_set(Sc& p, double x)
 {
-    const double t = nr_recip(nrm2(d));
-    return cd{d.x * t, -d.y * t};
+    const float2 f = ff_split(x);
+    p = Sc{f.x, f.y};
 }
+__device__ __forceinline__ void p_set(Pc& p, cd x)
+{
+    const float2 a = ff_split(x.x), b = ff_split(x.y);
+    p = Pc{f2_pack(a.x, b.x), f2_pack(a.y, b.y)};
+}
+__device__ __forceinline__ double p_get(Sc a) { return (double)a.h + (double)a.l; }
+__device__ __forceinline__ cd p_get(Pc a)
+{
+    const float2 h = f2_unpack(a.h), l = f2_unpack(a.l);
+    return cd{(double)h.x + (double)l.x, (double)h.y + (double)l.y};
+}
+__device__ __forceinline__ float p_re(Sc a) { return a.h; }
+__device__ __forceinline__ float p_re(Pc a) { return f2_unpack(a.h).x; }
+__device__ __forceinline__ bool p_finite(Sc a) { return isfinite(a.h); }
+__device__ __forceinline__ bool p_finite(Pc a) { const float2 h = f2_unpack(a.h); return isfinite(h.x) && isfinite(h.y); }
+__device__ __forceinline__ Sc p_div(Sc a, Sc b) { return sc_div(a, b); }
+__device__ __forceinline__ Pc p_div(Pc a, Pc b) { return p_sc(sc_div(p_sc(a), p_sc(b))); }
+// c - a b
+__device__ __forceinline__ Sc p_nms(Sc c, Sc a, Sc b) { return sc_add(c, sc_neg(sc_mul(a, b))); }
+__device__ __forceinline__ Pc p_nms(Pc c, Pc a, Pc b)
+{
+    const float2 ah = f2_unpack(a.h), al = f2_unpack(a.l), bh = f2_unpack(b.h), bl = f2_unpack(b.l);
+    ff2_mac(c.h, c.l, f2_bcast(-ah.x), f2_bcast(-al.x), b.h, b.l);
+    ff2_mac(c.h, c.l, f2_pack(ah.y, -ah.y), f2_pack(al.y, -al.y), f2_pack(bh.y, bh.x), f2_pack(bl.y, bl.x));
+    return c;
+}
+__device__ __forceinline__ Sc p_shfl(Sc a, int r)
+{
+    return Sc{__shfl_sync(0xffffffffu, a.h, r), __shfl_sync(0xffffffffu, a.l, r)};
+}
+__device__ __forceinline__ Pc p_shfl(Pc a, int r)
+{
+    return Pc{__shfl_sync(0xffffffffu, a.h, r), __shfl_sync(0xffffffffu, a.l, r)};
+}
+
+// 1 / sqrt(d), Re d > 0, for values that have been scaled to about 1: an FP32
+// seed and two Newton steps in FP64
 __device__ __forceinline__ double nr_rsqrt(double d)
 {
     double x = 1.f / sqrtf((float)d);
@@ -223,76 +262,131 @@ __device__ __forceinline__ cd nr_rsqrt(cd d)
     return x;
 }
 
-// G of the approximate inverse: a warp per row.  The row's pattern S (m
-// entries, ascending, the row itself last) is in the slice layout; the warp
-// gathers A(S, S) into shared memory, factors it L D L^T in place (lane =
-// row), and back-substitutes L^T y = e_m; the row is y / sqrt(d_m), formed in
-// FP64 from the FP64 matrix (scaled by a power of four of its diagonal) and
-// cast, as the IC(0) factor is.  A row whose
-// pivots are not positive, or whose entries are no FP32 numbers, keeps its
-// scaled diagonal alone.
+// G of the approximate inverse: GL lanes per row.  The row's pattern S (m
+// entries, ascending, the row itself last) is in the slice layout; the lanes
+// gather A(S, S) into shared memory, factor it L D L^T in place (lane = row),
+// and back-substitute L^T y = e_m; the row is y / sqrt(d_m), from the FP64
+// matrix (scaled by a power of four of its diagonal), and cast, as the IC(0)
+// factor is.  A row whose pivots are not positive, or whose entries are no FP32
+// numbers, keeps its scaled diagonal alone.
+// Values are pairs of floats: on disc and cylinder matrices the rows differ from
+// an FP64 elimination's by at most 4e-14, and after the cast in no entry.  FP64
+// instructions hold a warp's pipe for 16 clocks, and a row's pivots are a chain:
+// a warp per row in FP64 was 10 % of a request on 3D meshes of 2k to 4k nodes.
+// Rows of at most 8 entries (2D) go four to a warp and rows of at most 16 two to
+// a warp, each size in CTAs of its own.
 // ---------------------------------------------------------------------------
-template <class V64, class V>
-__global__ void __launch_bounds__(32 * FSAI_WARPS) fsai_kernel(int n, const int* __restrict__ rowptr,
-                                                              const int* __restrict__ colidx,
-                                                              const int* __restrict__ diagpos,
-                                                              const V64* __restrict__ A, const int* __restrict__ gptr,
-                                                              const int* __restrict__ gcol,
-                                                              const int* __restrict__ gcnt, V* __restrict__ gval)
+template <class V64, class V, int GL, class P>
+__device__ __forceinline__ void fsai_rows_of(P (*sm)[GL][GL + 1], int (*ss)[GL], int block, int n,
+                                             const int* __restrict__ rowptr, const int* __restrict__ colidx,
+                                             const int* __restrict__ diagpos, const V64* __restrict__ A,
+                                             const int* __restrict__ gptr, const int* __restrict__ gcol,
+                                             const int* __restrict__ gcnt, V* __restrict__ gval)
 {
-    __shared__ V64 sm[FSAI_WARPS][FSAI_MAXM][FSAI_MAXM + 1];
-    __shared__ int ss[FSAI_WARPS][FSAI_MAXM];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * FSAI_WARPS + w;
-    if (i >= n) return;
-    V64(*M)[FSAI_MAXM + 1] = sm[w];
-    int* S = ss[w];
-    const int m = gcnt[i], base = gptr[i >> 5] + (i & 31);
-    const double dg = re(A[diagpos[i]]);
-    bool ok = isfinite(dg) && dg > 0.0;  // the same value in every lane, here and below
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, q = threadIdx.x / GL, gl = lane % GL, g0 = lane - gl;
+    if (q >= fsai_rows(GL)) return;
+    const int i = block * fsai_rows(GL) + q;
+    P(*M)[GL + 1] = sm[q];
+    int* S = ss[q];
+    int m = i < n ? gcnt[i] : 0;
+    if (m > GL || (GL > 8 && m <= GL / 2)) m = 0;  // other CTAs' row
+    const int mm = (int)__reduce_max_sync(ALL, (unsigned)m);  // the warp's rows step together
+    if (mm == 0) return;
+    const int base = m ? gptr[i >> 5] + (i & 31) : 0;
+    const double dg = m ? re(A[diagpos[i]]) : 1.0;
+    bool ok = m && isfinite(dg) && dg > 0.0;  // the same value in a row's lanes, here and below
     const int ex = ok ? ilogb(dg) >> 1 : 0;
     const double sc = ldexp(1.0, -2 * ex);
-    if (lane < m) S[lane] = gcol[base + 32 * lane];
+    if (gl < m) S[gl] = gcol[base + 32 * gl];
     for (int a = 0; a < m; a++)
-        if (lane < m) M[a][lane] = vzero<V64>();
+        if (gl < m) p_set(M[a][gl], vzero<V64>());
     __syncwarp();
-    for (int a = 0; a < m; a++) {
-        const int ra = S[a];
-        for (int p = rowptr[ra] + lane; p < rowptr[ra + 1]; p += 32) {
-            const int c = colidx[p];
-            for (int b = 0; b <= a; b++)
-                if (S[b] == c) M[a][b] = vscale(A[p], sc);
+    // each lane its row of A, four entries in flight
+    if (gl < m) {
+        const int ra = S[gl], p1 = rowptr[ra + 1];
+        for (int p = rowptr[ra]; p < p1; p += 4) {
+            int c[4];
+            V64 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                c[u] = p + u < p1 ? colidx[p + u] : ra + 1;
+                v[u] = A[min(p + u, p1 - 1)];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                // (the lanes split their entries together, wherever these belong)
+                P e;
+                p_set(e, vscale(v[u], sc));
+                int at = -1;
+                for (int b = 0; b < mm; b++)
+                    if (b <= gl && S[b] == c[u]) at = b;
+                if (at >= 0) M[gl][at] = e;
+            }
         }
     }
     __syncwarp();
-    for (int j = 0; j < m; j++) {
-        const V64 d = M[j][j];
-        ok &= sfinite(d) && re(d) > 0.0;
-        if (!ok) break;
-        V64 l = vzero<V64>();
-        if (lane > j && lane < m) {
-            l = vmul(M[lane][j], nr_recip(d));
-            for (int c = j + 1; c <= lane; c++) M[lane][c] = vfms(M[lane][c], l, M[c][j]);
+    for (int j = 0; j < mm; j++) {
+        const P d = M[j < m ? j : 0][j < m ? j : 0];
+        ok &= j >= m || (p_finite(d) && p_re(d) > 0.f);
+        const bool on = ok && gl > j && gl < m;
+        P l = d;
+        if (on) {
+            l = p_div(M[gl][j], d);
+            for (int c = j + 1; c <= gl; c += 4) {
+                P v[4], w[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) { v[u] = M[gl][min(c + u, gl)]; w[u] = M[min(c + u, gl)][j]; }
+#pragma unroll
+                for (int u = 0; u < 4; u++) v[u] = p_nms(v[u], l, w[u]);
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (c + u <= gl) M[gl][c + u] = v[u];
+            }
         }
         __syncwarp();
-        if (lane > j && lane < m) M[lane][j] = l;
+        if (on) M[gl][j] = l;
         __syncwarp();
+    }
+    // lane j of the row holds y_j
+    P t;
+    p_set(t, vmake<V64>(gl == m - 1 ? 1.0 : 0.0, 0.0));
+    for (int r = mm - 1; r > 0; r--) {
+        const P tr = p_shfl(t, g0 + r);
+        if (ok && r < m && gl < r) t = p_nms(t, M[r][gl], tr);
     }
     V y = vzero<V>();
-    if (ok) {
-        // lane j holds y_j
-        V64 t = lane == m - 1 ? vmake<V64>(1.0, 0.0) : vzero<V64>();
-        for (int r = m - 1; r > 0; r--) {
-            const V64 tr = shfl(t, r);
-            if (lane < r) t = vfms(t, M[r][lane], tr);
-        }
-        y = vcast<V, V64>(vscale(vmul(t, nr_rsqrt(M[m - 1][m - 1])), ldexp(1.0, -ex)));
-        ok = __all_sync(0xffffffffu, lane >= m || sfinite(y));
-    }
-    if (!ok) y = lane == m - 1 ? vcast<V, V64>(vrecip(ssqrt(A[diagpos[i]]))) : vzero<V>();
-    if (lane < m) gval[base + 32 * lane] = y;
+    if (ok) y = vcast<V, V64>(vscale(vmul(p_get(t), nr_rsqrt(p_get(M[m - 1][m - 1]))), ldexp(1.0, -ex)));
+    constexpr unsigned ROW = GL == 32 ? ALL : (1u << (GL & 31)) - 1u;
+    ok &= ((__ballot_sync(ALL, gl >= m || sfinite(y)) >> g0) & ROW) == ROW;
+    if (m == 0) return;
+    if (!ok) y = gl == m - 1 ? vcast<V, V64>(vrecip(ssqrt(A[diagpos[i]]))) : vzero<V>();
+    if (gl < m) gval[base + 32 * gl] = y;
     // padding entries of the slice
     const int wd = (gptr[(i >> 5) + 1] - gptr[i >> 5]) >> 5;
-    for (int e = m + lane; e < wd; e += 32) gval[base + 32 * e] = vzero<V>();
+    for (int e = m + gl; e < wd; e += GL) gval[base + 32 * e] = vzero<V>();
+}
+
+template <class V64, class V>
+__global__ void __launch_bounds__(FSAI_NT) fsai_kernel(int n, int n32, int n16, const int* __restrict__ rowptr,
+                                                      const int* __restrict__ colidx, const int* __restrict__ diagpos,
+                                                      const V64* __restrict__ A, const int* __restrict__ gptr,
+                                                      const int* __restrict__ gcol, const int* __restrict__ gcnt,
+                                                      V* __restrict__ gval)
+{
+    using P = typename PairOf<V>::T;
+    __shared__ union Sm {
+        P m8[fsai_rows(8)][8][9], m16[fsai_rows(16)][16][17], m32[fsai_rows(32)][32][33];
+        __device__ Sm() {}
+    } sm;
+    __shared__ int ss[FSAI_NT];
+    const int b = blockIdx.x;
+    if (b < n32)
+        fsai_rows_of<V64, V, 32, P>(sm.m32, (int(*)[32])ss, b, n, rowptr, colidx, diagpos, A, gptr, gcol, gcnt, gval);
+    else if (b < n32 + n16)
+        fsai_rows_of<V64, V, 16, P>(sm.m16, (int(*)[16])ss, b - n32, n, rowptr, colidx, diagpos, A, gptr, gcol, gcnt, gval);
+    else
+        fsai_rows_of<V64, V, 8, P>(sm.m8, (int(*)[8])ss, b - n32 - n16, n, rowptr, colidx, diagpos, A, gptr, gcol, gcnt, gval);
 }
 
 // ---------------------------------------------------------------------------
@@ -994,13 +1088,14 @@ template void (*resident_kernel<double, float>(int))(ResArgs<double, float>);
 template void (*resident_kernel<cd, cf>(int))(ResArgs<cd, cf>);
 
 template <class V64, class V>
-void (*fsai_kernel_of())(int, const int*, const int*, const int*, const V64*, const int*, const int*, const int*, V*)
+void (*fsai_kernel_of())(int, int, int, const int*, const int*, const int*, const V64*, const int*, const int*, const int*,
+                         V*)
 {
     return fsai_kernel<V64, V>;
 }
-template void (*fsai_kernel_of<double, float>())(int, const int*, const int*, const int*, const double*, const int*,
-                                                 const int*, const int*, float*);
-template void (*fsai_kernel_of<cd, cf>())(int, const int*, const int*, const int*, const cd*, const int*, const int*,
-                                          const int*, cf*);
+template void (*fsai_kernel_of<double, float>())(int, int, int, const int*, const int*, const int*, const double*,
+                                                 const int*, const int*, const int*, float*);
+template void (*fsai_kernel_of<cd, cf>())(int, int, int, const int*, const int*, const int*, const cd*, const int*,
+                                          const int*, const int*, cf*);
 
 }  // namespace tg

@@ -2158,8 +2158,10 @@ static void build_resident(tg_solver s)
     V32* sg = (V32*)s->sg32.ensure((size_t)m.sg.len * sizeof(V32));
     V32* st = (V32*)s->st32.ensure((size_t)m.st.len * sizeof(V32));
     launch(ell_gather_kernel<V32>, cdiv_u(m.sa.len, 256), 256, 0, s->stream, m.sa.len, m.sa.src, A32, sa);
-    launch(fsai_kernel_of<V64, V32>(), cdiv_u(m.n, FSAI_WARPS), 32 * FSAI_WARPS, 0, s->stream, m.n, m.rowptr, m.colidx,
-           m.diagpos, (const V64*)s->val64.as<V64>(), m.sg.ptr, m.sg.col, m.gcnt, sg);
+    const unsigned n32 = s->mesh->h.gmax > 16 ? cdiv_u(m.n, fsai_rows(32)) : 0;
+    const unsigned n16 = s->mesh->h.gmax > 8 ? cdiv_u(m.n, fsai_rows(16)) : 0;
+    launch(fsai_kernel_of<V64, V32>(), n32 + n16 + cdiv_u(m.n, fsai_rows(8)), FSAI_NT, 0, s->stream, m.n, (int)n32,
+           (int)n16, m.rowptr, m.colidx, m.diagpos, (const V64*)s->val64.as<V64>(), m.sg.ptr, m.sg.col, m.gcnt, sg);
     launch(ell_gather_kernel<V32>, cdiv_u(m.st.len, 256), 256, 0, s->stream, m.st.len, m.st.src, sg, st);
     s->res_ready = true;
 }
