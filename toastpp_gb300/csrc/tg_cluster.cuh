@@ -66,13 +66,13 @@ constexpr int IC_NT = 256;      // threads of a CTA
 template <class V>
 void (*ic_cluster_kernel_of(int lv))(IcClArgs<V>);
 
-// G of the approximate inverse from A's values in CSR order; the first n32 CTAs
+// G of the approximate inverse from A's float-float values in CSR order; the first n32 CTAs
 // take the rows of 17 to 32 entries, the next n16 those of 9 to 16, the others
 // those of at most 8
 constexpr int FSAI_NT = 128;
 constexpr int fsai_rows(int gl) { return gl == 32 ? 2 : FSAI_NT / gl; }  // rows of such a CTA (35 KB of complex matrices)
 template <class V64, class V>
-void (*fsai_kernel_of())(int n, int n32, int n16, const int* rowptr, const int* colidx, const int* diagpos, const V64* A,
+void (*fsai_kernel_of())(int n, int n32, int n16, const int* rowptr, const int* colidx, const int* diagpos, const void* A,
                          const int* gptr, const int* gcol, const int* gcnt, V* gval);
 
 }  // namespace tg

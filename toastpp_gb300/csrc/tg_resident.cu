@@ -201,16 +201,19 @@ __device__ __forceinline__ Scc p_sc(Pc a)
     return Scc{sc_norm(h.x, l.x), sc_norm(h.y, l.y)};
 }
 __device__ __forceinline__ Pc p_sc(Scc a) { return Pc{f2_pack(a.x.h, a.y.h), f2_pack(a.x.l, a.y.l)}; }
-__device__ __forceinline__ void p_set(Sc& p, double x)
+// entry e of the float-float matrix (re_hi, re_lo, im_hi, im_lo), times f
+__device__ __forceinline__ void p_load(Sc& p, const void* A, int e, float f)
 {
-    const float2 f = ff_split(x);
-    p = Sc{f.x, f.y};
+    const float2 v = ((const float2*)A)[e];
+    p = Sc{v.x * f, v.y * f};
 }
-__device__ __forceinline__ void p_set(Pc& p, cd x)
+__device__ __forceinline__ void p_load(Pc& p, const void* A, int e, float f)
 {
-    const float2 a = ff_split(x.x), b = ff_split(x.y);
-    p = Pc{f2_pack(a.x, b.x), f2_pack(a.y, b.y)};
+    const float4 v = ((const float4*)A)[e];
+    p = Pc{f2_pack(v.x * f, v.z * f), f2_pack(v.y * f, v.w * f)};
 }
+__device__ __forceinline__ void p_set(Sc& p, float x) { p = Sc{x, 0.f}; }
+__device__ __forceinline__ void p_set(Pc& p, float x) { p = Pc{f2_pack(x, 0.f), 0ull}; }
 __device__ __forceinline__ double p_get(Sc a) { return (double)a.h + (double)a.l; }
 __device__ __forceinline__ cd p_get(Pc a)
 {
@@ -265,21 +268,21 @@ __device__ __forceinline__ cd nr_rsqrt(cd d)
 // G of the approximate inverse: GL lanes per row.  The row's pattern S (m
 // entries, ascending, the row itself last) is in the slice layout; the lanes
 // gather A(S, S) into shared memory, factor it L D L^T in place (lane = row),
-// and back-substitute L^T y = e_m; the row is y / sqrt(d_m), from the FP64
-// matrix (scaled by a power of four of its diagonal), and cast, as the IC(0)
-// factor is.  A row whose pivots are not positive, or whose entries are no FP32
+// and back-substitute L^T y = e_m; the row is y / sqrt(d_m), from the
+// float-float matrix (scaled by a power of four of its diagonal), and cast.  A row whose pivots are not positive, or whose entries are no FP32
 // numbers, keeps its scaled diagonal alone.
 // Values are pairs of floats: on disc and cylinder matrices the rows differ from
-// an FP64 elimination's by at most 4e-14, and after the cast in no entry.  FP64
-// instructions hold a warp's pipe for 16 clocks, and a row's pivots are a chain:
-// a warp per row in FP64 was 10 % of a request on 3D meshes of 2k to 4k nodes.
+// an FP64 elimination's (which the IC(0) factor is formed by) by at most 4e-14,
+// and after the cast in no entry.  FP64 instructions hold a warp's pipe for 16
+// clocks, and a row's pivots are a chain: a warp per row in FP64 was 10 % of a
+// request on 3D meshes of 2k to 4k nodes.
 // Rows of at most 8 entries (2D) go four to a warp and rows of at most 16 two to
 // a warp, each size in CTAs of its own.
 // ---------------------------------------------------------------------------
 template <class V64, class V, int GL, class P>
 __device__ __forceinline__ void fsai_rows_of(P (*sm)[GL][GL + 1], int (*ss)[GL], int block, int n,
                                              const int* __restrict__ rowptr, const int* __restrict__ colidx,
-                                             const int* __restrict__ diagpos, const V64* __restrict__ A,
+                                             const int* __restrict__ diagpos, const void* __restrict__ A,
                                              const int* __restrict__ gptr, const int* __restrict__ gcol,
                                              const int* __restrict__ gcnt, V* __restrict__ gval)
 {
@@ -294,34 +297,33 @@ __device__ __forceinline__ void fsai_rows_of(P (*sm)[GL][GL + 1], int (*ss)[GL],
     const int mm = (int)__reduce_max_sync(ALL, (unsigned)m);  // the warp's rows step together
     if (mm == 0) return;
     const int base = m ? gptr[i >> 5] + (i & 31) : 0;
-    const double dg = m ? re(A[diagpos[i]]) : 1.0;
-    bool ok = m && isfinite(dg) && dg > 0.0;  // the same value in a row's lanes, here and below
-    const int ex = ok ? ilogb(dg) >> 1 : 0;
-    const double sc = ldexp(1.0, -2 * ex);
+    P dg;
+    p_set(dg, 1.f);
+    if (m) p_load(dg, A, diagpos[i], 1.f);
+    bool ok = m && p_finite(dg) && p_re(dg) > 0.f;  // the same value in a row's lanes, here and below
+    const int ex = ok ? ilogbf(p_re(dg)) >> 1 : 0;
+    const float sc = ldexpf(1.f, -2 * ex);
     if (gl < m) S[gl] = gcol[base + 32 * gl];
     for (int a = 0; a < m; a++)
-        if (gl < m) p_set(M[a][gl], vzero<V64>());
+        if (gl < m) p_set(M[a][gl], 0.f);
     __syncwarp();
     // each lane its row of A, four entries in flight
     if (gl < m) {
         const int ra = S[gl], p1 = rowptr[ra + 1];
         for (int p = rowptr[ra]; p < p1; p += 4) {
             int c[4];
-            V64 v[4];
+            P v[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 c[u] = p + u < p1 ? colidx[p + u] : ra + 1;
-                v[u] = A[min(p + u, p1 - 1)];
+                p_load(v[u], A, min(p + u, p1 - 1), sc);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                // (the lanes split their entries together, wherever these belong)
-                P e;
-                p_set(e, vscale(v[u], sc));
                 int at = -1;
                 for (int b = 0; b < mm; b++)
                     if (b <= gl && S[b] == c[u]) at = b;
-                if (at >= 0) M[gl][at] = e;
+                if (at >= 0) M[gl][at] = v[u];
             }
         }
     }
@@ -350,7 +352,7 @@ __device__ __forceinline__ void fsai_rows_of(P (*sm)[GL][GL + 1], int (*ss)[GL],
     }
     // lane j of the row holds y_j
     P t;
-    p_set(t, vmake<V64>(gl == m - 1 ? 1.0 : 0.0, 0.0));
+    p_set(t, gl == m - 1 ? 1.f : 0.f);
     for (int r = mm - 1; r > 0; r--) {
         const P tr = p_shfl(t, g0 + r);
         if (ok && r < m && gl < r) t = p_nms(t, M[r][gl], tr);
@@ -360,7 +362,7 @@ __device__ __forceinline__ void fsai_rows_of(P (*sm)[GL][GL + 1], int (*ss)[GL],
     constexpr unsigned ROW = GL == 32 ? ALL : (1u << (GL & 31)) - 1u;
     ok &= ((__ballot_sync(ALL, gl >= m || sfinite(y)) >> g0) & ROW) == ROW;
     if (m == 0) return;
-    if (!ok) y = gl == m - 1 ? vcast<V, V64>(vrecip(ssqrt(A[diagpos[i]]))) : vzero<V>();
+    if (!ok) y = gl == m - 1 ? vcast<V, V64>(vrecip(ssqrt(p_get(dg)))) : vzero<V>();
     if (gl < m) gval[base + 32 * gl] = y;
     // padding entries of the slice
     const int wd = (gptr[(i >> 5) + 1] - gptr[i >> 5]) >> 5;
@@ -370,7 +372,7 @@ __device__ __forceinline__ void fsai_rows_of(P (*sm)[GL][GL + 1], int (*ss)[GL],
 template <class V64, class V>
 __global__ void __launch_bounds__(FSAI_NT) fsai_kernel(int n, int n32, int n16, const int* __restrict__ rowptr,
                                                       const int* __restrict__ colidx, const int* __restrict__ diagpos,
-                                                      const V64* __restrict__ A, const int* __restrict__ gptr,
+                                                      const void* __restrict__ A, const int* __restrict__ gptr,
                                                       const int* __restrict__ gcol, const int* __restrict__ gcnt,
                                                       V* __restrict__ gval)
 {
@@ -1088,14 +1090,14 @@ template void (*resident_kernel<double, float>(int))(ResArgs<double, float>);
 template void (*resident_kernel<cd, cf>(int))(ResArgs<cd, cf>);
 
 template <class V64, class V>
-void (*fsai_kernel_of())(int, int, int, const int*, const int*, const int*, const V64*, const int*, const int*, const int*,
+void (*fsai_kernel_of())(int, int, int, const int*, const int*, const int*, const void*, const int*, const int*, const int*,
                          V*)
 {
     return fsai_kernel<V64, V>;
 }
-template void (*fsai_kernel_of<double, float>())(int, int, int, const int*, const int*, const int*, const double*,
+template void (*fsai_kernel_of<double, float>())(int, int, int, const int*, const int*, const int*, const void*,
                                                  const int*, const int*, const int*, float*);
-template void (*fsai_kernel_of<cd, cf>())(int, int, int, const int*, const int*, const int*, const cd*, const int*,
+template void (*fsai_kernel_of<cd, cf>())(int, int, int, const int*, const int*, const int*, const void*, const int*,
                                           const int*, const int*, cf*);
 
 }  // namespace tg

@@ -2161,7 +2161,7 @@ static void build_resident(tg_solver s)
     const unsigned n32 = s->mesh->h.gmax > 16 ? cdiv_u(m.n, fsai_rows(32)) : 0;
     const unsigned n16 = s->mesh->h.gmax > 8 ? cdiv_u(m.n, fsai_rows(16)) : 0;
     launch(fsai_kernel_of<V64, V32>(), n32 + n16 + cdiv_u(m.n, fsai_rows(8)), FSAI_NT, 0, s->stream, m.n, (int)n32,
-           (int)n16, m.rowptr, m.colidx, m.diagpos, (const V64*)s->val64.as<V64>(), m.sg.ptr, m.sg.col, m.gcnt, sg);
+           (int)n16, m.rowptr, m.colidx, m.diagpos, (const void*)s->valff.p, m.sg.ptr, m.sg.col, m.gcnt, sg);
     launch(ell_gather_kernel<V32>, cdiv_u(m.st.len, 256), 256, 0, s->stream, m.st.len, m.st.src, sg, st);
     s->res_ready = true;
 }
