@@ -161,17 +161,25 @@ int tg_solver_set_refinement(tg_solver s, double inner_tol, int max_outer, int i
 /* mixed precision with BiCGSTAB requested: how the FP32 inner work runs.
    0: restarted refinement (a new FP32 BiCGSTAB solve per FP64 step);
    1: ONE FP32 BiCGSTAB process per right-hand side whose residual is replaced
-      by the FP64 residual b - A x whenever it has fallen by inner_tol
-      (reliable updates);
+      by the true residual b - A x of the FP64 solution whenever it has fallen
+      by inner_tol (reliable updates).  The product A x is formed in float-float
+      arithmetic (about 2^-46 of |A||x|), and in FP64 for tolerances below 1e-13
+      and where the float-float one is too noisy for the residual expected;
    2 (default): as 1 with an FP32 COCG process for complex systems (the
       conjugate-orthogonal CG of the complex symmetric F).  While the vectors
       fit on the chip, an ICH-preconditioned solve in the default ordering runs
       as one kernel on thread-block clusters, with CG for real systems and a
       factorised sparse approximate inverse on F's own pattern in place of the
-      IC(0) sweeps; CG requests run the same way.  Larger blocks take one SpMM
-      and one IC(0) apply per COCG iteration, real systems as 1.
+      IC(0) sweeps; CG requests run the same way, with every A x in FP64.  Its
+      sums are compensated FP32 pairs (about 2^-46).  Larger blocks, and columns
+      that this kernel does not bring to their bounds (breakdowns, systems that
+      are not positive definite, too many replacements), take one SpMM and one
+      IC(0) apply per COCG iteration, real systems as 1.
    The FP64 result meets tol in every mode.  At most 4 * max_outer residual
-   replacements per right-hand side. */
+   replacements per right-hand side.  maxit bounds the iterations of the process
+   that runs; for real systems on the cluster kernel an iteration of a BiCGSTAB
+   request counts two products, as BiCGSTAB's, and a CG request's limit bounds each
+   inner solve (max_outer of them), as restarted refinement does. */
 /* mixed precision only: the componentwise backward-error bound of every
    solution (default 1e-10; 0 turns the test off).  Besides |b - A x| <= tol |b|
    the FP64 refinement then continues until

@@ -13,8 +13,8 @@
 // Why not the level-scheduled sparse kernels of the IC(0) sweeps: a complete
 // factor has a level per column of the root path, 196 on the 3.2k-node disc,
 // each a launch of a few rows with up to 150 serial merge steps (367 us a
-// level).  The dense fronts turn that into about 50 launches bound by the FP64
-// rate (2 multiply-adds a clock on an SM): reset and 32 solves 60.0 -> 1.3 ms
+// level).  The dense fronts turn that into about 70 launches (43 at the reset
+// and 29 at the solve, with what surrounds them) bound by the FP64 rate (2 multiply-adds a clock on an SM): reset and 32 solves 60.0 -> 1.3 ms
 // (3.2k nodes, 100 MHz), 337 -> 3.0 ms (12.5k nodes), 5.6 s -> 12.5 ms (7.5k-node
 // cylinder).
 //

@@ -34,10 +34,17 @@
 // 12.5k-node disc with 64 columns, 35 with them on chip, and 22 against 11 on
 // the 3.2k-node disc with 32.
 //
-// Measured, whole requests before and after: 217 nodes, 8 columns 2.88 -> 0.38
-// ms; 3.2k nodes CW, 32 columns 8.41 -> 1.00 ms; data gradient on 12.5k nodes
-// (two solves of 32 columns) 157 -> 8.2 ms, of which most was columns whose
+// Measured, whole requests before and after: 217 nodes, 8 columns 2.88 -> 0.40
+// ms; 3.2k nodes CW, 32 columns 8.41 -> 1.06 ms; data gradient on 12.5k nodes
+// (two solves of 32 columns) 157 -> 8.6 ms, of which most was columns whose
 // residuals the float-float product could not resolve (below).
+//
+// Precision.  Vectors, the matrices and G are FP32, as in the batched FP32
+// processes; sums are compensated FP32 pairs (TwoSum, about 2^-46) of FP32
+// products, where those add four rows in FP32 and then in FP64; the recursion's
+// scalars and G's rows are formed in pairs.  The solution and its true residual
+// are FP64: the product in float-float, a row in FP64 where that is too noisy for
+// it, and for CG requests and tolerances below 1e-13 always in FP64.
 //
 // Thread mapping: a thread per row, with the cluster's LV columns as one word
 // of 4 to 16 bytes.  (Sharing a row between lanes, for more columns a cluster,

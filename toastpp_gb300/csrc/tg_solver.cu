@@ -2693,8 +2693,10 @@ static void solve_mixed(tg_solver s, int k, const V64* B, V64* X, ColState* co, 
     if (s->method == TG_SOLVER_BICGSTAB && s->reliable) {
         // complex systems: COCG inner process (one SpMM and one IC(0) apply
         // per iteration) unless BiCGSTAB was asked for (reliable mode 1)
-        // (CG requests keep restarted refinement: the reliable-update CG
-        // process measured slower on the 3.2k-node CW disc, 9.6 against 8.4 ms)
+        // (CG requests whose blocks come here take restarted refinement below: the
+        // reliable-update process on this path, one launch per step, measured
+        // slower on the 3.2k-node CW disc, 9.6 against 8.4 ms, before such meshes
+        // went to the resident kernel)
         const bool cocg = vt<V32>::cplx && s->reliable == 2;
         solve_reliable<V64, V32>(s, k, B, X, co, R, R32, E32, ci, e64, e32, maxit, cocg);
         return;
