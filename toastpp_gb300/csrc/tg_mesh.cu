@@ -706,6 +706,8 @@ PartSize Mesh::part_size(int cs)
 {
     TG_CHECK(cs == 1 || cs == 2 || cs == 4 || cs == 8 || cs == 16, TG_ERR_ARG, "cluster size");
     std::lock_guard<std::mutex> lk(part_mu);
+    auto it = part_sizes.find(cs);
+    if (it != part_sizes.end()) return it->second;
     const int n = h.n, ns = (n + 31) / 32;
     auto first = [&](int r, int c) { return std::min(n, (int)((long long)ns * r / c) * 32); };
     if (reach.empty()) {
@@ -732,7 +734,7 @@ PartSize Mesh::part_size(int cs)
         S.len = std::max(S.len, h.sa.ptr[s1] - h.sa.ptr[s0] + h.sg.ptr[s1] - h.sg.ptr[s0] + h.st.ptr[s1] - h.st.ptr[s0]);
     }
     for (int r = 0; r < cs; r++) S.slots = std::max(S.slots, first(r + 1, cs) - first(r, cs) + halo[r]);
-    return S;
+    return part_sizes[cs] = S;
 }
 
 const PartDev* Mesh::part(int cs)

@@ -176,6 +176,7 @@ struct Mesh {
     // the sizes of the split for clusters of cs (1, 2, 4, 8, 16) CTAs, from one
     // pass over the pattern for all of them: what a choice of cs needs
     PartSize part_size(int cs);
+    std::map<int, PartSize> part_sizes;
     std::vector<unsigned short> reach;
     // the split itself, built at its first use; null when a CTA's slots pass 16 bits
     const PartDev* part(int cs);

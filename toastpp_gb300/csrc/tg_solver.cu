@@ -599,15 +599,6 @@ struct Engine {
         return ic_shapes[{k, ico}] = best;
     }
 
-    // sizes of the split of the last shape, kept: part_size counts them anew
-    PartSize ic_size(int cs)
-    {
-        if (psz_cs != cs) { psz = mesh->part_size(cs); psz_cs = cs; }
-        return psz;
-    }
-    PartSize psz{};
-    int psz_cs = 0;
-
     // shared memory of a CTA: the vector, then levels and rows of both sweeps
     size_t ic_vec_bytes(const PartSize& P, int lv) const { return ((size_t)P.slots * lv * sizeof(V) + 15) / 16 * 16; }
     size_t ic_smem(const PartSize& P, int lv)
@@ -673,7 +664,7 @@ struct Engine {
     {
         const auto sh = ic_shape(k);
         const IcPartDev* I = mesh->ic_part(sh.cs, ico);
-        const PartSize P = ic_size(sh.cs);
+        const PartSize P = mesh->part_size(sh.cs);
         IcClArgs<V> a;
         a.mofs = (int)ic_vec_bytes(P, sh.lv);
         a.f = I->f; a.b = I->b;
