@@ -149,7 +149,7 @@ TGHD cd csqrt_d(cd z)
 
 TGHD cd cdiv(cd a, cd b)
 {
-    // Smith's algorithm: scaled to avoid overflow
+    // Smith (1962): scaled to avoid overflow
     if (fabs(b.x) >= fabs(b.y)) {
         double r = b.y / b.x, den = b.x + b.y * r;
         return cd{(a.x + a.y * r) / den, (a.y - a.x * r) / den};

@@ -219,17 +219,6 @@ __global__ void __launch_bounds__(256) grid_planes_cm_kernel(GridDev G, int k, i
     }
 }
 
-// Smith's complex division (Smith 1962)
-__device__ __forceinline__ cd cdiv_smith(cd a, cd b)
-{
-    if (fabs(b.x) >= fabs(b.y)) {
-        const double r = b.y / b.x, den = b.x + b.y * r;
-        return cd{(a.x + a.y * r) / den, (a.y - a.x * r) / den};
-    }
-    const double r = b.x / b.y, den = b.x * r + b.y;
-    return cd{(a.x * r + a.y) / den, (a.y * r - a.x) / den};
-}
-
 // One launch before the grid and element kernels: the factor of each link's
 // row, sc / y for log data (Smith's division for complex y), sc for linear
 // data (y null), formed in FP64 and cast to the Jacobian's arithmetic type;
@@ -243,7 +232,7 @@ __global__ void grid_prep_kernel(size_t cnt0, const V64* __restrict__ x0, size_t
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i < (size_t)nqm) {
         if constexpr (vt<V64>::cplx) {
-            const cd r = y ? cdiv_smith(cd{1.0, 0.0}, y[i]) : cd{1.0, 0.0};
+            const cd r = y ? cdiv(cd{1.0, 0.0}, y[i]) : cd{1.0, 0.0};
             ysc[i] = vcast<C, cd>(cd{r.x * sc, r.y * sc});
         } else {
             ysc[i] = vcast<C, double>(y ? sc / y[i] : sc);
